@@ -126,8 +126,6 @@ const DevRef& dev_ref(int dim, int order) {
     d->tc64.upload(t64.data(), t64.size() * sizeof(double));
     d->tc32 = DevBuf(t32.size() * sizeof(float));
     d->tc32.upload(t32.data(), t32.size() * sizeof(float));
-    d->tc_ok64 = tc_warps_for<double>(dim, order) >= 2;
-    d->tc_ok32 = tc_warps_for<float>(dim, order) >= 2;
   }
   auto* raw = d.get();
   slot[0] = std::move(d);
@@ -238,8 +236,9 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
   a.beta = beta;
   a.c = c ? c : y;
   a.tcg = f64 ? (const T*)mesh->tcg64.p : (const T*)mesh->tcg32.p;
+  a.fgeo = f64 ? (const T*)fgeo64.p : (const T*)fgeo32.p;
   a.tcgen05 = kernel == 3;
-  const bool tc_ok = (kernel == 0 || kernel >= 2) && (f64 ? dref->tc_ok64 : dref->tc_ok32);
+  const bool tc_ok = kernel == 0 || kernel >= 2;
   if (tc_ok && ncomp > 1 && pin_elem < 0) {
     // vector operator: one tensor-core scalar apply per component (its own boundary
     // types; slip faces get no face terms there), then the slip faces' coupling terms
@@ -281,6 +280,10 @@ void sipg_op::refresh_tau(cudaStream_t s) {
   SIPG_CUDA(launch_tau<float>(mesh->dim, order, dref->itab.as<int8_t>(), mesh->geof32.as<float>(),
                               mesh->nbr.as<int>(), mesh->fcode.as<uint32_t>(), f32, mesh->K,
                               tau32.as<float>(), s));
+  SIPG_CUDA(launch_face_geo<double>(mesh->dim, mesh->tcg64.as<double>(), tau64.as<double>(), mesh->K,
+                                    fgeo64.as<double>(), s));
+  SIPG_CUDA(launch_face_geo<float>(mesh->dim, mesh->tcg32.as<float>(), tau32.as<float>(), mesh->K,
+                                   fgeo32.as<float>(), s));
 }
 
 BlockArgs sipg_op::block_args(int mode, int ref_volume, double* out, bool with_pin) const {
@@ -336,6 +339,8 @@ std::unique_ptr<sipg_op> create_op(sipg_mesh* m, int order, int ncomp) {
   const int Nf = m->dim + 1;
   op->tau64 = DevBuf((size_t)m->K * Nf * sizeof(double));
   op->tau32 = DevBuf((size_t)m->K * Nf * sizeof(float));
+  op->fgeo64 = DevBuf((size_t)m->K * Nf * 4 * sizeof(double));
+  op->fgeo32 = DevBuf((size_t)m->K * Nf * 4 * sizeof(float));
   op->bct_host.assign((size_t)ncomp * m->Kb, SIPG_BC_DIRICHLET);
   op->bct = DevBuf(std::max<size_t>(1, op->bct_host.size()));
   std::vector<uint8_t> b(op->bct_host.size(), 0);

@@ -53,8 +53,7 @@ inline void ensure(DevBuf& b, size_t n) {
 struct DevRef {
   RefElement ref;
   DevBuf c64, c32, itab, mf;
-  DevBuf tc64, tc32;   // tensor-core constant blobs (A1 | A2)
-  bool tc_ok64 = false, tc_ok32 = false;
+  DevBuf tc64, tc32;   // tensor-core constant blobs (pass 1 | pass 2)
   int Np = 0, Nfp = 0;
 };
 const DevRef& dev_ref(int dim, int order);  // cached per device
@@ -95,6 +94,7 @@ struct sipg_op {
   const sipg::DevRef* dref = nullptr;
   bool has_factor = false;
   sipg::DevBuf factor64, factor32, tau64, tau32;
+  sipg::DevBuf fgeo64, fgeo32;  // face coefficients of the tensor-core apply (launch_face_geo), kept with tau
   int mm_mode = 0;
   double mm_scalar = 0.0;
   sipg::DevBuf mm64, mm32;

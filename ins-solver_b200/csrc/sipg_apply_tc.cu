@@ -13,20 +13,35 @@
 // out exactly like an A block once the dummy summation index k is permuted
 // (slot t <-> logical column 2t, slot t+4 <-> 2t+1, folded into the packing of
 // B), so a product's result feeds the next product from registers and the
-// elementwise steps (metric terms, fluxes) run on fragment registers.
+// elementwise steps (metric terms, fluxes) run on fragment registers. In FP64 a
+// last block of nodes that is at most half full binds slot t to its node t alone,
+// and the second of its two k = 4 steps (all padding) is not issued.
 //
-//   pass 1 (traces): per face node k = (f, j) with volume node m = fmask(f, j):
-//           g = f(m) sum_r c_r(f) (D_r x)(m), c_r = n_f . grad r, computed as
-//           x (TE x Np) . BF_r (Np x Nf*Nfp), BF_r[n][k] = D_r[m(k)][n];
-//           trace[e][f] = (x(m(f, j)) for j < Nfp, g(f, j) for j < Nfp).
-//   pass 2 (apply): gr_r = x . B1_r (gradient in the reference directions),
-//           w_r = J f sum_s K_rs gr_s (K = G G^T, the metric of the element),
-//           fluxes from the own and the neighbour's traces
-//             [u] = u- - u+, n.{q} = (g- - g+)/2 (n+ = -n-), boundary faces as
-//             vmf_3d_mult_avg_jump.h:43-80,
+//   pass 1 (volume): gr_r = x . B1_r (gradient in the reference directions),
+//           h_r = f gr_r, w_r = J sum_s K_rs h_s (K = G G^T, the metric),
+//           y = alpha (sum_r w_r . (M D_r) + (J mm x) . M) + beta c,
+//           trace[e][f] = (x(m), (sJ / 2) sum_r c_r(f) h_r(m)) for the face nodes
+//           m = fmask(f, j), c_r = n_f . grad r: the value and half the scaled
+//           normal flux q = (sJ / 2) n . f grad x.
+//   pass 2 (faces): [u] = u- - u+, n.{q} = (q- - q+) / sJ (n+ = -n-; both sides
+//           share sJ), boundary faces as vmf_3d_mult_avg_jump.h:43-80
+//           (Dirichlet: u+ = -u-, q+ = -q-; Neumann: u+ = u-, q+ = q-),
 //             Fu = sJ (tau [u]/2 - n.{q}), S = -sJ f [u]/2 (fvmf_3d_mult_flux.h:13-22),
-//           Z_r = w_r . M^T + (c_r S) . EMAT^T,
-//           y = sum_r Z_r . D_r + Fu . EMAT^T + (J mm x) . M^T.
+//           y += alpha (Fu . EMAT^T + sum_r (c_r S) . (D_r^T EMAT)^T).
+//
+// The products with M and EMAT are folded into the derivative's (M D_r and
+// D_r^T EMAT are single 8 x 8-blocked operands) and the gradient is computed once,
+// in the pass that also needs it for the traces: at p = 3 in 3D 210 FP64 MMAs
+// (m8n8k4) per 8 elements and 114 TF32 ones per 16, against 372 and 186 when
+// pass 1 evaluated the derivatives at the face nodes and pass 2 the gradient
+// again, M and D one after the other. Element rows, traces and geometry are read
+// from global memory straight into fragment registers (a quad of lanes reads a
+// contiguous piece of a row), so shared memory holds only the operands and, in
+// pass 1, the rearrangement of node values into trace records: more warps per SM
+// and fewer instructions than with every input staged. Measured per apply, before
+// and after that rearrangement: FP64 p = 4 Helmholtz at 48^3 x 6 tets 2.24 -> 1.22 ms
+// (DMMA-bound: 24 of the 37 TFLOP/s the FP64 pipe has), FP32 p = 3 two-phase at
+// 24^3 x 6 42.8 -> 37.5 us (latency-bound).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -56,10 +71,8 @@ struct Frag<float> {
   using V2 = float2;
   // FP32 values go to the TF32 MMA as they are: the tensor core uses the sign,
   // exponent and top 10 mantissa bits (truncation, relative error below 2^-10
-  // per operand instead of 2^-11 after a round-to-nearest conversion). Dropping
-  // the conversion instruction (about 160 per warp tile and lane at p = 3) left
-  // the iteration counts of the mixed-precision solves unchanged.
-  __device__ static __forceinline__ float op(float x) { return x; }
+  // per operand instead of 2^-11 after a round-to-nearest conversion); the
+  // iteration counts of the mixed-precision solves are the same with either.
   // m16n8k8: a0 (g, t) a1 (g+8, t) a2 (g, t+4) a3 (g+8, t+4); b0 (t, g) b1 (t+4, g);
   // c0 (g, 2t) c1 (g, 2t+1) c2 (g+8, 2t) c3 (g+8, 2t+1).
   __device__ static __forceinline__ void mma(float (&c)[2][2], const float (&a)[2][2], V2 b) {
@@ -70,29 +83,28 @@ struct Frag<float> {
         : "r"(__float_as_uint(a[0][0])), "r"(__float_as_uint(a[1][0])), "r"(__float_as_uint(a[0][1])),
           "r"(__float_as_uint(a[1][1])), "r"(__float_as_uint(b.x)), "r"(__float_as_uint(b.y)));
   }
+  // a block whose second logical columns are all padding: no shorter form
+  __device__ static __forceinline__ void mma_half(float (&c)[2][2], const float (&a)[2][2], V2 b) { mma(c, a, b); }
 };
 
 template <>
 struct Frag<double> {
   static constexpr int R = 1;
   using V2 = double2;
-  __device__ static __forceinline__ double op(double x) { return x; }
   // two m8n8k4 steps: a0 (g, t), b0 (t, g), c0 (g, 2t) c1 (g, 2t+1); the first
   // binds slot t to logical column 2t, the second to 2t+1.
   __device__ static __forceinline__ void mma(double (&c)[1][2], const double (&a)[1][2], V2 b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(c[0][0]), "+d"(c[0][1])
-                 : "d"(a[0][0]), "d"(b.x));
+    mma_half(c, a, b);
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(c[0][0]), "+d"(c[0][1])
                  : "d"(a[0][1]), "d"(b.y));
   }
+  __device__ static __forceinline__ void mma_half(double (&c)[1][2], const double (&a)[1][2], V2 b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(c[0][0]), "+d"(c[0][1])
+                 : "d"(a[0][0]), "d"(b.x));
+  }
 };
-
-// Smallest m >= n with m = 8 (mod 16): row stride of staged element data for
-// which the pair loads of a fragment (two adjacent columns per lane, element
-// rows g) fall in distinct banks.
-__host__ __device__ constexpr int pad816(int n) { return n <= 8 ? 8 : rup(n - 8, 16) + 8; }
 
 template <typename T, int DIM, int P>
 struct Tc {
@@ -100,47 +112,30 @@ struct Tc {
   static constexpr int NP = C::NP, NFP = C::NFP, NF = C::NF;
   static constexpr int R = Frag<T>::R, TE = 8 * R;   // elements per warp tile
   static constexpr int NT = rup(NP, 8) / 8;          // node blocks
-  static constexpr int KF = NF * NFP;                // face nodes of an element
+  // FP64: the last node block holds at most 4 nodes, one per lane of a quad
+  static constexpr bool HALF = R == 1 && NP % 8 >= 1 && NP % 8 <= 4;
+  static constexpr int TRP = rup(NFP, 2);            // face nodes of a record, padded to pairs (padding: zeros)
+  static constexpr int TR = 2 * TRP;                 // record: (u, q) per face node
+  static constexpr int KF = NF * TRP;                // face nodes of an element with their padding
   static constexpr int FT = rup(KF, 8) / 8;          // face-node blocks
-  static constexpr int TRP = rup(NFP, 2);            // g part of a trace record starts here
-  static constexpr int TR = rup(2 * TRP, 4);         // record length: a 16-byte multiple
   static constexpr int BLK = 64;                     // values per packed 8 x 8 block
-  // pass-2 blob: B1_r (NT x NT blocks), BM, BE (FT x NT), B3_r; then the pass-1 blob BF_r (NT x FT)
+  // pass-1 blob: B1_r, BS_r = M D_r, BM (NT x NT blocks each); pass-2 blob: BE (FT x NT), BQ_r = (D_r^T EMAT)^T
   static constexpr int B1 = 0;
-  static constexpr int BM = B1 + DIM * NT * NT * BLK;
-  static constexpr int BE = BM + NT * NT * BLK;
-  static constexpr int B3 = BE + FT * NT * BLK;
-  static constexpr int N2 = B3 + DIM * NT * NT * BLK;
-  static constexpr int BF = N2;
-  static constexpr int N1 = DIM * NT * FT * BLK;
-  static constexpr int NALL = N2 + N1;
-  static constexpr int XS = pad816(NP);              // staged row stride of x and factor
-  static constexpr int TS = pad816(NF * TR);         // staged row stride of an element's trace records
-  // copy piece of an x / factor row (rows start on multiples of Np values)
-  static constexpr int XCB = (NP * (int)sizeof(T)) % 16 == 0 ? 16 : (NP * (int)sizeof(T)) % 8 == 0 ? 8 : 4;
+  static constexpr int BS = B1 + DIM * NT * NT * BLK;
+  static constexpr int BM = BS + DIM * NT * NT * BLK;
+  static constexpr int N1 = BM + NT * NT * BLK;
+  static constexpr int BE = 0;                       // within the pass-2 blob
+  static constexpr int BQ = BE + FT * NT * BLK;
+  static constexpr int N2 = BQ + DIM * FT * NT * BLK;
+  static constexpr int NALL = N1 + N2;
   // geometry block of a warp tile (launch_tc_geom), rows of TE values: NV volume
   // rows (J, then the metric K = G G^T by rows of its upper triangle, zero rows),
   // then NFG x NF face rows [q][f] (q: sJ, c_0, c_1, c_2)
   static constexpr int NV = 8, NFG = 4, GROWS = NV + NFG * NF;
-  static constexpr int SFG = NFG * NF * TE;
-  // element stage (T units, every part a multiple of 64 bytes): x, factor, then
-  // the face rows of the geometry block (pass 1) or the whole block and tau (pass 2)
-  static constexpr int SX = 0, SF = TE * XS, SG = 2 * TE * XS;
-  static constexpr int ST1 = SG + SFG;
-  static constexpr int STAU = SG + GROWS * TE, ST2 = STAU + TE * NF;
-  static constexpr int SI = TE * NF + TE;            // int slot: nbr, face codes
-  // pass 1 warp: 2 stages, output records
-  static constexpr int W1_T = 2 * ST1 + TE * TS;
-  static constexpr int W2_I = 3 * SI;
-  static constexpr int CH = TR * (int)sizeof(T) / 16;  // 16-byte chunks per trace record
-};
-
-// Pass-2 warp area: NS element stages, own and neighbour trace records (one
-// buffer each).
-template <typename T, int DIM, int P, int NS>
-struct W2 {
-  using X = Tc<T, DIM, P>;
-  static constexpr int STR = NS * X::ST2, SNB = STR + X::TE * X::TS, T_ = SNB + X::TE * X::TS;
+  // pass 1 warp area: (x, h_0, h_1, h_2) per node, odd node stride, then reused for the tile's records
+  static constexpr int HS = NP | 1;
+  static constexpr int W1 = TE * HS * 4 > TE * NF * TR ? TE * HS * 4 : TE * NF * TR;
+  static constexpr int LPE = 32 / TE, FPL = (NF + LPE - 1) / LPE;  // record gather: lanes per element, faces per lane
 };
 
 // Row of the metric entry K_rs (r <= s) in the geometry block.
@@ -154,117 +149,42 @@ template <typename T>
 __device__ __forceinline__ typename Frag<T>::V2 ld2(const T* p) {
   return *reinterpret_cast<const typename Frag<T>::V2*>(p);
 }
+// four consecutive values, 16-byte aligned
+__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
+  const double2 q = reinterpret_cast<const double2*>(p)[0], r = reinterpret_cast<const double2*>(p)[1];
+  v[0] = q.x; v[1] = q.y; v[2] = r.x; v[3] = r.y;
+}
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
+  reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
+  reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
+}
 
-// CB-byte asynchronous copy (4, 8 or 16), zero-filled past `bytes`.
-template <int CB>
-__device__ __forceinline__ void cp_async_n(void* sdst, const void* gsrc, int bytes) {
+__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  if (CB == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gsrc), "r"(bytes));
-  else if (CB == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gsrc), "r"(bytes));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gsrc), "r"(bytes));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::); }
-__device__ __forceinline__ void cp_wait_but_one() { asm volatile("cp.async.wait_group 1;\n" ::); }
 
-// Copy `total` bytes (a multiple of 16) to shared memory: the first `valid`
-// come from base + off (16-byte aligned), the rest is zero.
-__device__ __forceinline__ void copy_block(void* s, const void* base, size_t off, int total, int valid, int lane) {
-  const char* b = static_cast<const char*>(base);
-  for (int c = lane * 16; c < total; c += 32 * 16) {
-    const int n = min(16, max(0, valid - c));
-    cp_async_n<16>(static_cast<char*>(s) + c, n > 0 ? b + off + c : b, n);
-  }
+// `bytes` (a multiple of 16) of a 16-byte aligned blob to shared memory by the whole CTA.
+__device__ __forceinline__ void copy_blob(void* s, const void* g, int bytes) {
+#pragma unroll 4
+  for (int c = threadIdx.x * 16; c < bytes; c += blockDim.x * 16)
+    cp_async16(static_cast<char*>(s) + c, static_cast<const char*>(g) + c);
+  cp_commit();
 }
 
-// NR rows of LEN values (global rows contiguous from row0) into shared rows of
-// stride DS; rows at or past nvalid are zero-filled (zero) or skipped. Lane
-// handles row lane % NR and every (32 / NR)-th piece of it, so the row address is
-// computed once.
-template <typename T, int CB, int LEN, int DS, int NR>
-__device__ __forceinline__ void copy_rows(T* dst, const T* base, size_t row0, int nvalid, int lane, bool zero) {
-  constexpr int V = CB / (int)sizeof(T), CPR = LEN / V, LPR = 32 / NR;
-  static_assert(LEN % V == 0, "row length must be a multiple of the copy piece");
-  static_assert(32 % NR == 0, "rows must divide the warp");
-  const int r = lane % NR, q = lane / NR;
-  const bool v = r < nvalid;
-  if (!v && !zero) return;
-  T* d = dst + r * DS;
-  const T* src = v ? base + (row0 + r) * LEN : base;
-#pragma unroll
-  for (int c0 = 0; c0 < CPR; c0 += LPR) {
-    const int c = c0 + q;
-    if (c < CPR) cp_async_n<CB>(d + c * V, v ? src + c * V : base, v ? CB : 0);
-  }
-}
-
-template <typename T, int DIM, int P>
-__device__ __forceinline__ void issue_elem(const ApplyArgs<T>& a, T* st, int tile, int lane, bool pass2) {
-  using X = Tc<T, DIM, P>;
-  constexpr int NP = X::NP, NF = X::NF, TE = X::TE, S = sizeof(T);
-  const int e0 = tile * TE;
-  const int ne = max(0, min(TE, a.K - e0));
-  copy_rows<T, X::XCB, NP, X::XS, TE>(st + X::SX, a.x, (size_t)e0, ne, lane, true);
-  if (a.factor) copy_rows<T, X::XCB, NP, X::XS, TE>(st + X::SF, a.factor, (size_t)e0, ne, lane, true);
-  // the geometry block is zero past K, so a started tile copies it whole
-  const size_t gb = (size_t)tile * X::GROWS * TE * S;
-  if (pass2) {
-    copy_block(st + X::SG, a.tcg, gb, X::GROWS * TE * S, ne > 0 ? X::GROWS * TE * S : 0, lane);
-    copy_block(st + X::STAU, a.tau, (size_t)e0 * NF * S, TE * NF * S, ne * NF * S, lane);
-  } else {
-    copy_block(st + X::SG, a.tcg, gb + (size_t)X::NV * TE * S, X::SFG * S, ne > 0 ? X::SFG * S : 0, lane);
-  }
-}
-
-template <typename T, int DIM, int P>
-__device__ __forceinline__ void issue_ints(const ApplyArgs<T>& a, int* slot, int tile, int lane) {
-  using X = Tc<T, DIM, P>;
-  constexpr int NF = X::NF, TE = X::TE;
-  const int e0 = tile * TE;
-  const int ne = max(0, min(TE, a.K - e0));
-  copy_block(slot, a.nbr, (size_t)e0 * NF * 4, TE * NF * 4, ne * NF * 4, lane);
-  copy_block(slot + TE * NF, a.fcode, (size_t)e0 * 4, TE * 4, ne * 4, lane);
-}
-
-// Own and neighbour trace records of a tile whose connectivity has arrived
-// (records that are never read are not copied).
-template <typename T, int DIM, int P, int NS>
-__device__ __forceinline__ void issue_traces(const ApplyArgs<T>& a, const T* trace, T* w, const int* slot, int tile,
-                                             int lane) {
-  using X = Tc<T, DIM, P>;
-  using L = W2<T, DIM, P, NS>;
-  constexpr int NF = X::NF, TE = X::TE, CH = X::CH, TR = X::TR, TS = X::TS, VPC = 16 / sizeof(T);
-  const int e0 = tile * TE;
-  const int ne = max(0, min(TE, a.K - e0));
-  copy_rows<T, 16, NF * TR, TS, TE>(w + L::STR, trace, (size_t)e0, ne, lane, false);
-  const int* nbr = slot;
-  const int* code = slot + TE * NF;
-  // one neighbour record (CH pieces) per lane and round
-#pragma unroll
-  for (int lf0 = 0; lf0 < TE * NF; lf0 += 32) {
-    const int lf = lf0 + lane;
-    if (lf < TE * NF) {
-      const int el = lf / NF, f = lf % NF;
-      const int nb = nbr[lf];
-      if (el < ne && nb >= 0) {
-        const int fr = (code[el] >> (8 * f)) & 3;
-        T* d = w + L::SNB + el * TS + f * TR;
-        const T* src = trace + ((size_t)nb * NF + fr) * TR;
-#pragma unroll
-        for (int c = 0; c < CH; ++c) cp_async_n<16>(d + c * VPC, src + c * VPC, 16);
-      }
-    }
-  }
-}
-
-// 1/sqrt: the hardware approximation in FP32 (the TF32 path tolerates its ulps), exact in FP64.
+// sJ and c_r = n . grad r of face f (n the outward unit normal) from the geometric factors g.
 __device__ __forceinline__ float inv_sqrt(float v) { return rsqrtf(v); }
 __device__ __forceinline__ double inv_sqrt(double v) { return 1.0 / sqrt(v); }
 
-// sJ and c_r = n . grad r of face f (n the outward unit normal) from the geometric factors g.
 template <typename T, int DIM>
 __device__ __forceinline__ void face_geom(const T* g, int f, T& sJ, T (&c)[3]) {
   T n[3];
@@ -307,510 +227,426 @@ __device__ __forceinline__ void face_geom(const T* g, int f, T& sJ, T (&c)[3]) {
   }
 }
 
+// Node values of the lane's elements in fragment order: v[nt][ri][ci] = row e0 + g + 8 ri,
+// node 8 nt + 2t + ci (HALF's last block: node 8 nt + t, then padding); zero past Np and
+// past the tile's ne elements.
 template <typename T, int DIM, int P>
-__device__ __forceinline__ T fgeo(const T* sfg, int q, int f, int el) {
+__device__ __forceinline__ void load_nodes(const T* __restrict__ base, int e0, int ne,
+                                           T (&v)[Tc<T, DIM, P>::NT][Frag<T>::R][2], int g, int t) {
   using X = Tc<T, DIM, P>;
-  return sfg[(q * X::NF + f) * X::TE + el];
-}
-
-// Zero the padding columns (Np .. XS-1) of the x and factor rows of `nst` element
-// stages `stride` values apart: the fragment loads read them and the copies never
-// write them. Nothing else in a warp area is read before it is written.
-template <typename T, int DIM, int P>
-__device__ __forceinline__ void zero_row_padding(T* W, int nst, int stride, int lane) {
-  using X = Tc<T, DIM, P>;
-  constexpr int PAD = X::XS - X::NP, TE = X::TE;
-  if (PAD == 0) return;
-  for (int i = lane; i < nst * 2 * TE * PAD; i += 32) {
-    const int row = i / PAD, c = i % PAD;  // row over (stage, x rows then factor rows)
-    W[(row / (2 * TE)) * stride + (row % (2 * TE)) * X::XS + X::NP + c] = T(0);
+#pragma unroll
+  for (int ri = 0; ri < X::R; ++ri) {
+    const bool in = g + 8 * ri < ne;
+    const T* row = base + (size_t)(e0 + (in ? g + 8 * ri : 0)) * X::NP;
+#pragma unroll
+    for (int nt = 0; nt < X::NT; ++nt) {
+      const int n0 = 8 * nt + 2 * t;
+      if (X::HALF && nt == X::NT - 1) {
+        v[nt][ri][0] = in && 8 * nt + t < X::NP ? row[8 * nt + t] : T(0);
+        v[nt][ri][1] = T(0);
+      } else if (X::NP % 2 == 0) {  // pairs of nodes are aligned
+        typename Frag<T>::V2 q{T(0), T(0)};
+        if (in && n0 < X::NP) q = ld2(row + n0);
+        v[nt][ri][0] = q.x;
+        v[nt][ri][1] = q.y;
+      } else {
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) v[nt][ri][ci] = in && n0 + ci < X::NP ? row[n0 + ci] : T(0);
+      }
+    }
   }
 }
 
-// A blocks of x: u[kb][ri][ci] = x[g + 8 ri][8 kb + 2t + ci]
-// (staged rows are zero past Np).
 template <typename T, int DIM, int P>
-__device__ __forceinline__ void load_x_frags(const T* sx, T (&u)[Tc<T, DIM, P>::NT][Frag<T>::R][2], int g, int t) {
+__device__ __forceinline__ void store_nodes(T* base, int e0, int ne, const T (&v)[Tc<T, DIM, P>::NT][Frag<T>::R][2],
+                                            int g, int t) {
   using X = Tc<T, DIM, P>;
 #pragma unroll
-  for (int kb = 0; kb < X::NT; ++kb)
+  for (int ri = 0; ri < X::R; ++ri) {
+    if (g + 8 * ri >= ne) continue;
+    T* row = base + (size_t)(e0 + g + 8 * ri) * X::NP;
 #pragma unroll
-    for (int ri = 0; ri < X::R; ++ri) {
-      const auto v = ld2(sx + (g + 8 * ri) * X::XS + 8 * kb + 2 * t);
-      u[kb][ri][0] = Frag<T>::op(v.x);
-      u[kb][ri][1] = Frag<T>::op(v.y);
+    for (int nt = 0; nt < X::NT; ++nt) {
+      const int n0 = 8 * nt + 2 * t;
+      if (X::HALF && nt == X::NT - 1) {
+        if (8 * nt + t < X::NP) row[8 * nt + t] = v[nt][ri][0];
+      } else if (X::NP % 2 == 0) {
+        if (n0 < X::NP) *reinterpret_cast<typename Frag<T>::V2*>(row + n0) = typename Frag<T>::V2{v[nt][ri][0], v[nt][ri][1]};
+      } else {
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci)
+          if (n0 + ci < X::NP) row[n0 + ci] = v[nt][ri][ci];
+      }
     }
+  }
+}
+
+// Node of fragment entry (nt, ci) on lane t (at or past Np: padding).
+template <typename T, int DIM, int P>
+__device__ __forceinline__ int frag_node(int nt, int ci, int t) {
+  using X = Tc<T, DIM, P>;
+  if (X::HALF && nt == X::NT - 1) return ci == 0 ? 8 * nt + t : X::NP;
+  return 8 * nt + 2 * t + ci;
+}
+
+// c += a . b over one node block kb
+template <typename T, int DIM, int P>
+__device__ __forceinline__ void mma_nodes(T (&c)[Frag<T>::R][2], const T (&a)[Frag<T>::R][2],
+                                          typename Frag<T>::V2 b, int kb) {
+  if (Tc<T, DIM, P>::HALF && kb == Tc<T, DIM, P>::NT - 1) Frag<T>::mma_half(c, a, b);
+  else Frag<T>::mma(c, a, b);
 }
 
 // ---------------------------------------------------------------- pass 1
-template <typename T, int DIM, int P, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 1) sipg_trace_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
-                                                                 T* __restrict__ trace) {
+template <typename T, int DIM, int P, int WARPS, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
+                                                                       T* __restrict__ trace) {
   using X = Tc<T, DIM, P>;
   using F = Frag<T>;
-  using V2 = typename F::V2;
-  constexpr int NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT, R = X::R, TE = X::TE, TR = X::TR, KF = X::KF,
-                XS = X::XS, TS = X::TS, TRP = X::TRP;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* BFs = reinterpret_cast<T*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  T* W = BFs + X::N1 + warp * X::W1_T;
-  int8_t* fmask = reinterpret_cast<int8_t*>(BFs + X::N1 + WARPS * X::W1_T);
-  T* sout = W + 2 * X::ST1;
-  const int ntiles = (a.K + TE - 1) / TE;
-  const int stride = gridDim.x * WARPS;
-  // warp-major tile order: the last, partial round of tiles is spread over all
-  // CTAs (SMs) instead of filling the first ones
-  int tile = warp * gridDim.x + blockIdx.x;
-  pdl_trigger();
-  zero_row_padding<T, DIM, P>(W, 2, X::ST1, lane);
-  for (int i = threadIdx.x; i < X::N1; i += blockDim.x) BFs[i] = blob[X::BF + i];
-  for (int i = threadIdx.x; i < NF * NFP; i += blockDim.x) fmask[i] = a.itab[i];
-  pdl_wait();  // x, factor and the trace buffer belong to the preceding kernels
-  __syncwarp();
-  issue_elem<T, DIM, P>(a, W, tile, lane, false);
-  cp_commit();
-  __syncthreads();
-  for (int it = 0; tile < ntiles; ++it, tile += stride) {
-    T* st = W + (it & 1) * X::ST1;
-    cp_wait_all();
-    __syncwarp();
-    issue_elem<T, DIM, P>(a, W + ((it & 1) ^ 1) * X::ST1, tile + stride, lane, false);
-    cp_commit();
-    const int e0 = tile * TE;
-    const int ne = min(TE, a.K - e0);
-    T* sx = st + X::SX;
-    const T* sf = st + X::SF;
-    const T* sfg = st + X::SG;  // face rows of the geometry block
-    if (lane == 0 && a.pin_elem >= e0 && a.pin_elem < e0 + ne) sx[(a.pin_elem - e0) * XS + a.pin_node] = T(0);
-    __syncwarp();
-    T u[NT][R][2];
-    load_x_frags<T, DIM, P>(sx, u, g, t);
-#pragma unroll
-    for (int fb = 0; fb < FT; ++fb) {
-      T acc[DIM][R][2];
-#pragma unroll
-      for (int r = 0; r < DIM; ++r)
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri) acc[r][ri][0] = acc[r][ri][1] = T(0);
-#pragma unroll
-      for (int kb = 0; kb < NT; ++kb)
-#pragma unroll
-        for (int r = 0; r < DIM; ++r) F::mma(acc[r], u[kb], ldb(BFs, (r * NT + kb) * FT + fb, lane));
-      if constexpr (NFP % 2 == 0) {
-        // the two columns of a lane lie on one face
-        const int k0 = 8 * fb + 2 * t;
-        if (k0 < KF) {
-          const int f = k0 / NFP, j0 = k0 % NFP;
-          const int m0 = fmask[k0], m1 = fmask[k0 + 1];
-#pragma unroll
-          for (int ri = 0; ri < R; ++ri) {
-            const int el = g + 8 * ri;
-            T s0 = T(0), s1 = T(0);
-#pragma unroll
-            for (int r = 0; r < DIM; ++r) {
-              const T c = fgeo<T, DIM, P>(sfg, 1 + r, f, el);
-              s0 += c * acc[r][ri][0];
-              s1 += c * acc[r][ri][1];
-            }
-            const T* xr = sx + el * XS;
-            const T fm0 = a.factor ? sf[el * XS + m0] : T(1), fm1 = a.factor ? sf[el * XS + m1] : T(1);
-            T* rec = sout + el * TS + f * TR;
-            *reinterpret_cast<V2*>(rec + j0) = V2{xr[m0], xr[m1]};
-            *reinterpret_cast<V2*>(rec + TRP + j0) = V2{fm0 * s0, fm1 * s1};
-          }
-        }
-      } else {
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri)
-#pragma unroll
-          for (int ci = 0; ci < 2; ++ci) {
-            const int k = 8 * fb + 2 * t + ci;
-            if (k < KF) {
-              const int el = g + 8 * ri;
-              const int f = k / NFP, j = k % NFP;
-              const int m = fmask[k];
-              T s = T(0);
-#pragma unroll
-              for (int r = 0; r < DIM; ++r) s += fgeo<T, DIM, P>(sfg, 1 + r, f, el) * acc[r][ri][ci];
-              const T fm = a.factor ? sf[el * XS + m] : T(1);
-              T* rec = sout + el * TS + f * TR;
-              rec[j] = sx[el * XS + m];
-              rec[TRP + j] = fm * s;
-            }
-          }
-      }
-    }
-    __syncwarp();
-    // coalesced write-out of the tile's records
-    {
-      using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-      constexpr int VPC = 16 / sizeof(T), CPE = NF * X::CH;
-      const int n = ne * CPE;
-      for (int i = lane; i < n; i += 32) {
-        const int el = i / CPE, c = i % CPE;
-        *reinterpret_cast<V4*>(trace + (size_t)(e0 + el) * NF * TR + c * VPC) =
-            *reinterpret_cast<const V4*>(sout + el * TS + c * VPC);
-      }
-    }
-    __syncwarp();
-  }
-  cp_wait_all();
-}
-
-// ---------------------------------------------------------------- pass 2
-// NS = 2: the next tile's element data is fetched during the whole current tile
-// (double-buffered stage); NS = 1: after the current tile's fluxes, which frees
-// shared memory for more warps per SM.
-template <typename T, int DIM, int P, int WARPS, int NS>
-__global__ void __launch_bounds__(WARPS * 32, 1) sipg_apply_tc_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
-                                                                    const T* __restrict__ trace) {
-  using X = Tc<T, DIM, P>;
-  using L = W2<T, DIM, P, NS>;
-  using F = Frag<T>;
-  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT, R = X::R, TE = X::TE, TR = X::TR,
-                KF = X::KF, TRP = X::TRP, XS = X::XS, TS = X::TS;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, R = X::R, TE = X::TE, TR = X::TR, TRP = X::TRP,
+                HS = X::HS, LPE = X::LPE, FPL = X::FPL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* B = reinterpret_cast<T*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  T* W = B + X::N2 + warp * L::T_;
-  int* ibase = reinterpret_cast<int*>(B + X::N2 + WARPS * L::T_);
-  int* I = ibase + warp * X::W2_I;
-  int8_t* itab = reinterpret_cast<int8_t*>(ibase + WARPS * X::W2_I);
-  const int8_t* fmask = itab;
-  const int8_t* perm = itab + NF * NFP;
-  const T* str = W + L::STR;
-  const T* snb = W + L::SNB;
+  const bool has_mm = a.mm_mode != MM_NONE;
+  T* W = B + X::N1 + warp * X::W1;
   const int ntiles = (a.K + TE - 1) / TE;
   const int stride = gridDim.x * WARPS;
   // warp-major tile order: the last, partial round of tiles is spread over all
   // CTAs (SMs) instead of filling the first ones
   int tile = warp * gridDim.x + blockIdx.x;
   pdl_trigger();
-  zero_row_padding<T, DIM, P>(W, NS, X::ST2, lane);
-  __syncwarp();
-  // prologue: constants and the connectivity of the first two tiles (set-up data),
-  // then, once the preceding kernels are done, the first tile's element data
-  issue_ints<T, DIM, P>(a, I, tile, lane);
-  issue_ints<T, DIM, P>(a, I + X::SI, tile + stride, lane);
-  for (int i = threadIdx.x; i < X::N2; i += blockDim.x) B[i] = blob[i];
-  for (int i = threadIdx.x; i < Cfg<DIM, P>::ITAB; i += blockDim.x) itab[i] = a.itab[i];
-  pdl_wait();
-  issue_elem<T, DIM, P>(a, W, tile, lane, true);
-  cp_commit();
-  __syncthreads();
-  cp_wait_all();
-  __syncwarp();
-  issue_traces<T, DIM, P, NS>(a, trace, W, I, tile, lane);
-  cp_commit();
-  // this lane's face-node columns per block: face | node in face << 4 | volume nodes << 10, << 18
-  int fbi[FT];
+  copy_blob(B, blob, (has_mm ? X::N1 : X::BM) * (int)sizeof(T));
+  // record gather: this lane's element of the tile and the volume nodes of its faces, 4 per word
+  constexpr int NW = (TRP + 3) / 4;
+  const int gel = lane / LPE, gf0 = (lane % LPE) * FPL;
+  unsigned fm[FPL][NW];
 #pragma unroll
-  for (int fb = 0; fb < FT; ++fb) {
-    const int k0 = 8 * fb + 2 * t;
-    fbi[fb] = -1;
-    if (NFP % 2 == 0 && k0 < KF) fbi[fb] = (k0 / NFP) | ((k0 % NFP) << 4) | (fmask[k0] << 10) | (fmask[k0 + 1] << 18);
-  }
-  for (int it = 0; tile < ntiles; ++it, tile += stride) {
-    const int sb = NS == 2 ? (it & 1) : 0, slot = it % 3;
-    T* st = W + sb * X::ST2;
-    const int* ints = I + slot * X::SI;
-    // element data of this tile and connectivity of the next one have arrived (the
-    // tile's trace records, issued after the previous tile's fluxes, may still be in flight)
-    cp_wait_but_one();
-    __syncwarp();
-    if (NS == 2) {
-      issue_ints<T, DIM, P>(a, I + ((it + 2) % 3) * X::SI, tile + 2 * stride, lane);
-      issue_elem<T, DIM, P>(a, W + (sb ^ 1) * X::ST2, tile + stride, lane, true);
-      cp_commit();
+  for (int i = 0; i < FPL; ++i)
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      unsigned v = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        if (4 * w + b < NFP && gf0 + i < NF) v |= (unsigned)(uint8_t)a.itab[(gf0 + i) * NFP + 4 * w + b] << (8 * b);
+      fm[i][w] = v;
     }
-
+  pdl_wait();  // x, factor, c, y and the trace buffer belong to the preceding kernels
+  T u[NT][R][2];
+  if (tile < ntiles) load_nodes<T, DIM, P>(a.x, tile * TE, min(TE, a.K - tile * TE), u, g, t);
+  cp_wait_all();
+  __syncthreads();
+  for (; tile < ntiles; tile += stride) {
     const int e0 = tile * TE;
     const int ne = min(TE, a.K - e0);
-    T* sx = st + X::SX;
-    const T* sf = st + X::SF;
-    const T* sg = st + X::SG;
-    const T* stau = st + X::STAU;
-    const int* snbr = ints;
-    const int* scode = ints + TE * NF;
-    if (lane == 0 && a.pin_elem >= e0 && a.pin_elem < e0 + ne) sx[(a.pin_elem - e0) * XS + a.pin_node] = T(0);
-    // c values read by the epilogue (beta != 0), loaded now so that their latency
-    // hides behind the tile's products
-    T yold[NT][R][2];
-    if (a.beta != T(0)) {
+    const bool pin_here = a.pin_elem >= e0 && a.pin_elem < e0 + ne;
+    T upin = T(0);
+    if (pin_here) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int ri = 0; ri < R; ++ri) {
-          const int el = g + 8 * ri, n0 = 8 * nt + 2 * t;
-          const T* crow = a.c + (size_t)(e0 + el) * NP;
-          if (NP % 2 == 0) {  // node pairs (n0, n0 + 1) are aligned
-            typename F::V2 v{T(0), T(0)};
-            if (el < ne && n0 < NP) v = ld2(crow + n0);
-            yold[nt][ri][0] = v.x;
-            yold[nt][ri][1] = v.y;
-          } else {
+        for (int ri = 0; ri < R; ++ri)
 #pragma unroll
-            for (int ci = 0; ci < 2; ++ci) yold[nt][ri][ci] = (el < ne && n0 + ci < NP) ? crow[n0 + ci] : T(0);
-          }
-        }
+          for (int ci = 0; ci < 2; ++ci)
+            if (e0 + g + 8 * ri == a.pin_elem && frag_node<T, DIM, P>(nt, ci, t) == a.pin_node) {
+              upin = u[nt][ri][ci];
+              u[nt][ri][ci] = T(0);
+            }
     }
-    const T* sfg = sg + X::NV * TE;  // face rows of the geometry block
-    __syncwarp();
-
-    // metric of the lane's elements: J and K = G G^T
-    T Jm[R], Km[R][DIM][DIM];
-#pragma unroll
-    for (int ri = 0; ri < R; ++ri) {
-      const int el = g + 8 * ri;
-      Jm[ri] = sg[el];
-#pragma unroll
-      for (int r = 0; r < DIM; ++r)
-#pragma unroll
-        for (int s = r; s < DIM; ++s) {
-          const T v = sg[kidx(DIM, r, s) * TE + el];
-          Km[ri][r][s] = v;
-          Km[ri][s][r] = v;
-        }
-    }
-
+    T fac[NT][R][2];
+    if (a.factor) load_nodes<T, DIM, P>(a.factor, e0, ne, fac, g, t);
+    const T* gb = a.tcg + (size_t)tile * X::GROWS * TE;
     // gr_r = x . B1_r
     T w[DIM][NT][R][2];
-    {
-      T u[NT][R][2];
-      load_x_frags<T, DIM, P>(sx, u, g, t);
+#pragma unroll
+    for (int r = 0; r < DIM; ++r)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri) w[r][nt][ri][0] = w[r][nt][ri][1] = T(0);
+#pragma unroll
+    for (int kb = 0; kb < NT; ++kb)
 #pragma unroll
       for (int r = 0; r < DIM; ++r)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
+          mma_nodes<T, DIM, P>(w[r][nt], u[kb], ldb(B + X::B1, (r * NT + kb) * NT + nt, lane), kb);
+    // h_r = f gr_r, kept per node for the traces; w_r = J sum_s K_rs h_s
+    __syncwarp();  // the previous tile's records have left the warp area
 #pragma unroll
-          for (int ri = 0; ri < R; ++ri) w[r][nt][ri][0] = w[r][nt][ri][1] = T(0);
+    for (int ri = 0; ri < R; ++ri) {
+      const int el = g + 8 * ri;
+      const T Jm = gb[el];
+      T Km[DIM][DIM];
 #pragma unroll
-      for (int kb = 0; kb < NT; ++kb)
+      for (int r = 0; r < DIM; ++r)
 #pragma unroll
-        for (int r = 0; r < DIM; ++r)
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) F::mma(w[r][nt], u[kb], ldb(B + X::B1, (r * NT + kb) * NT + nt, lane));
-    }
-    // w_r = J f sum_s K_rs gr_s (A blocks of the next product)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int ri = 0; ri < R; ++ri) {
-        const int el = g + 8 * ri;
-        T fJ[2] = {Jm[ri], Jm[ri]};
-        if (a.factor) {
-          const auto fv = ld2(sf + el * XS + 8 * nt + 2 * t);
-          fJ[0] *= fv.x;
-          fJ[1] *= fv.y;
+        for (int s = r; s < DIM; ++s) {
+          const T v = Jm * gb[kidx(DIM, r, s) * TE + el];
+          Km[r][s] = v;
+          Km[s][r] = v;
         }
 #pragma unroll
-        for (int ci = 0; ci < 2; ++ci) {
-          T gr[DIM];
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-          for (int s = 0; s < DIM; ++s) gr[s] = w[s][nt][ri][ci];
+        for (int ci = 0; ci < 2; ++ci) {
+          if (X::HALF && nt == NT - 1 && ci == 1) continue;
+          T h[3] = {T(0), T(0), T(0)};
+#pragma unroll
+          for (int s = 0; s < DIM; ++s) h[s] = a.factor ? fac[nt][ri][ci] * w[s][nt][ri][ci] : w[s][nt][ri][ci];
+          const int m = frag_node<T, DIM, P>(nt, ci, t);
+          if (8 * nt + 8 <= NP || m < NP) st4(W + (el * HS + m) * 4, u[nt][ri][ci], h[0], h[1], h[2]);
 #pragma unroll
           for (int r = 0; r < DIM; ++r) {
             T v = T(0);
 #pragma unroll
-            for (int s = 0; s < DIM; ++s) v += Km[ri][r][s] * gr[s];
-            w[r][nt][ri][ci] = F::op(fJ[ci] * v);
+            for (int s = 0; s < DIM; ++s) v += Km[r][s] * h[s];
+            w[r][nt][ri][ci] = v;
           }
         }
-      }
-    // Z_r = w_r . M^T ; y = (J mm x) . M^T
-    T z[DIM][NT][R][2], y[NT][R][2];
+    }
+    // y = sum_r w_r . BS_r + (J mm x) . BM
+    T y[NT][R][2];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int ri = 0; ri < R; ++ri) {
-        y[nt][ri][0] = y[nt][ri][1] = T(0);
+      for (int ri = 0; ri < R; ++ri) y[nt][ri][0] = y[nt][ri][1] = T(0);
+    if (has_mm) {
+      T mm[NT][R][2];
+      if (a.mm_mode == MM_NODAL) load_nodes<T, DIM, P>(a.mm, e0, ne, mm, g, t);
 #pragma unroll
-        for (int r = 0; r < DIM; ++r) z[r][nt][ri][0] = z[r][nt][ri][1] = T(0);
-      }
-    const bool has_mm = a.mm_mode != MM_NONE;
-#pragma unroll
-    for (int kb = 0; kb < NT; ++kb) {
-      T mx[R][2];
-      if (has_mm) {
+      for (int kb = 0; kb < NT; ++kb) {
+        T mx[R][2];
 #pragma unroll
         for (int ri = 0; ri < R; ++ri)
 #pragma unroll
-          for (int ci = 0; ci < 2; ++ci) {
-            const int el = g + 8 * ri, m = 8 * kb + 2 * t + ci;
-            T v = T(0);
-            if (m < NP && el < ne) {
-              const T mmv = a.mm_mode == MM_SCALAR ? a.mm_scalar : a.mm[(size_t)(e0 + el) * NP + m];
-              v = Jm[ri] * mmv * sx[el * XS + m];
-            }
-            mx[ri][ci] = F::op(v);
-          }
-      }
+          for (int ci = 0; ci < 2; ++ci)
+            mx[ri][ci] = gb[g + 8 * ri] * (a.mm_mode == MM_NODAL ? mm[kb][ri][ci] : a.mm_scalar) * u[kb][ri][ci];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const auto b = ldb(B + X::BM, kb * NT + nt, lane);
-#pragma unroll
-        for (int r = 0; r < DIM; ++r) F::mma(z[r][nt], w[r][kb], b);
-        if (has_mm) F::mma(y[nt], mx, b);
+        for (int nt = 0; nt < NT; ++nt) mma_nodes<T, DIM, P>(y[nt], mx, ldb(B + X::BM, kb * NT + nt, lane), kb);
       }
     }
-    // the tile's trace records have arrived
-    if (NS == 2) cp_wait_but_one();
-    else cp_wait_all();
-    __syncwarp();
-    // face fluxes: y += Fu . EMAT^T ; Z_r += (c_r S) . EMAT^T
-#pragma unroll
-    for (int fb = 0; fb < FT; ++fb) {
-      T fu[R][2], sv[DIM][R][2];
-      if constexpr (NFP % 2 == 0) {
-        // the two columns of a lane lie on one face
-        const int fi = fbi[fb];
-        const int f = fi & 15, j0 = (fi >> 4) & 63, m0 = (fi >> 10) & 255, m1 = (fi >> 18) & 255;
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri) {
-          const int el = g + 8 * ri;
-          T vfu[2] = {T(0), T(0)}, vs[2] = {T(0), T(0)}, cr[DIM];
-#pragma unroll
-          for (int r = 0; r < DIM; ++r) cr[r] = T(0);
-          if (fi >= 0 && el < ne) {
-            const int lf = el * NF + f;
-            const T* own = str + el * TS + f * TR;
-            const auto um = ld2(own + j0);
-            const auto gm = ld2(own + TRP + j0);
-            const int nb = snbr[lf];
-            T jump[2] = {T(0), T(0)}, navg[2] = {T(0), T(0)};
-            if (nb >= 0) {
-              const int8_t* pr = perm + ((scode[el] >> (8 * f + 2)) & 7) * NFP + j0;
-              const T* rec = snb + el * TS + f * TR;
-              const int kk0 = pr[0], kk1 = pr[1];
-              jump[0] = um.x - rec[kk0];
-              jump[1] = um.y - rec[kk1];
-              navg[0] = T(0.5) * (gm.x - rec[TRP + kk0]);
-              navg[1] = T(0.5) * (gm.y - rec[TRP + kk1]);
-            } else if (a.bct[-nb - 1] == BC_DIRICHLET) {
-              jump[0] = T(2) * um.x;
-              jump[1] = T(2) * um.y;
-              navg[0] = gm.x;
-              navg[1] = gm.y;
-            }
-            const T sJ = fgeo<T, DIM, P>(sfg, 0, f, el);
-#pragma unroll
-            for (int r = 0; r < DIM; ++r) cr[r] = fgeo<T, DIM, P>(sfg, 1 + r, f, el);
-            const T tau = stau[lf];
-            const T fm0 = a.factor ? sf[el * XS + m0] : T(1);
-            const T fm1 = a.factor ? sf[el * XS + m1] : T(1);
-            const T h0 = T(0.5) * jump[0], h1 = T(0.5) * jump[1];
-            vfu[0] = sJ * (tau * h0 - navg[0]);
-            vfu[1] = sJ * (tau * h1 - navg[1]);
-            vs[0] = -sJ * fm0 * h0;
-            vs[1] = -sJ * fm1 * h1;
-          }
-#pragma unroll
-          for (int ci = 0; ci < 2; ++ci) {
-            fu[ri][ci] = F::op(vfu[ci]);
-#pragma unroll
-            for (int r = 0; r < DIM; ++r) sv[r][ri][ci] = F::op(cr[r] * vs[ci]);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int ri = 0; ri < R; ++ri)
-#pragma unroll
-          for (int ci = 0; ci < 2; ++ci) {
-            const int el = g + 8 * ri, k = 8 * fb + 2 * t + ci;
-            T vfu = T(0), vs = T(0), cr[DIM];
-#pragma unroll
-            for (int r = 0; r < DIM; ++r) cr[r] = T(0);
-            if (k < KF && el < ne) {
-              const int f = k / NFP, j = k % NFP;
-              const int lf = el * NF + f;
-              const T* own = str + el * TS + f * TR;
-              const T um = own[j], gm = own[TRP + j];
-              const int nb = snbr[lf];
-              T jump = T(0), navg = T(0);
-              if (nb >= 0) {
-                const int kk = perm[((scode[el] >> (8 * f + 2)) & 7) * NFP + j];
-                const T* rec = snb + el * TS + f * TR;
-                jump = um - rec[kk];
-                navg = T(0.5) * (gm - rec[TRP + kk]);
-              } else if (a.bct[-nb - 1] == BC_DIRICHLET) {
-                jump = T(2) * um;
-                navg = gm;
-              }
-              const T hj = T(0.5) * jump;
-              const T sJ = fgeo<T, DIM, P>(sfg, 0, f, el);
-              const T fm = a.factor ? sf[el * XS + fmask[k]] : T(1);
-              vfu = sJ * (stau[lf] * hj - navg);
-              vs = -sJ * fm * hj;
-#pragma unroll
-              for (int r = 0; r < DIM; ++r) cr[r] = fgeo<T, DIM, P>(sfg, 1 + r, f, el);
-            }
-            fu[ri][ci] = F::op(vfu);
-#pragma unroll
-            for (int r = 0; r < DIM; ++r) sv[r][ri][ci] = F::op(cr[r] * vs);
-          }
-      }
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const auto b = ldb(B + X::BE, fb * NT + nt, lane);
-        F::mma(y[nt], fu, b);
-#pragma unroll
-        for (int r = 0; r < DIM; ++r) F::mma(z[r][nt], sv[r], b);
-      }
-    }
-    // the trace buffer (and with NS = 1 the element stage) is free: the next tile's
-    // data lands during the rest of this tile and the next tile's volume products
-    __syncwarp();
-    if (NS == 1) {
-      issue_ints<T, DIM, P>(a, I + ((it + 2) % 3) * X::SI, tile + 2 * stride, lane);
-      issue_elem<T, DIM, P>(a, W, tile + stride, lane, true);
-      cp_commit();
-    }
-    issue_traces<T, DIM, P, NS>(a, trace, W, I + ((it + 1) % 3) * X::SI, tile + stride, lane);
-    cp_commit();
-    // y += sum_r Z_r . D_r
+    // the next tile's x lands during the products
+    const int next = tile + stride;
+    if (next < ntiles) load_nodes<T, DIM, P>(a.x, next * TE, min(TE, a.K - next * TE), u, g, t);
 #pragma unroll
     for (int r = 0; r < DIM; ++r)
 #pragma unroll
-      for (int kb = 0; kb < NT; ++kb) {
-        T zr[R][2];
+      for (int kb = 0; kb < NT; ++kb)
 #pragma unroll
-        for (int ri = 0; ri < R; ++ri) {
-          zr[ri][0] = F::op(z[r][kb][ri][0]);
-          zr[ri][1] = F::op(z[r][kb][ri][1]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) F::mma(y[nt], zr, ldb(B + X::B3, (r * NT + kb) * NT + nt, lane));
-      }
-    // epilogue: pinned row, alpha / beta, store (pairs of nodes when Np is even)
-    const bool pin_here = a.pin_elem >= e0 && a.pin_elem < e0 + ne;
+        for (int nt = 0; nt < NT; ++nt)
+          mma_nodes<T, DIM, P>(y[nt], w[r][kb], ldb(B + X::BS, (r * NT + kb) * NT + nt, lane), kb);
+    // pinned row, alpha / beta, store
+    T yold[NT][R][2];
+    if (a.beta != T(0)) load_nodes<T, DIM, P>(a.c, e0, ne, yold, g, t);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-      for (int ri = 0; ri < R; ++ri) {
-        const int el = g + 8 * ri;
-        if (el >= ne) continue;
-        const size_t row = (size_t)(e0 + el) * NP;
-        T acc[2];
+      for (int ri = 0; ri < R; ++ri)
 #pragma unroll
         for (int ci = 0; ci < 2; ++ci) {
-          const int n = 8 * nt + 2 * t + ci;
-          acc[ci] = y[nt][ri][ci];
-          if (pin_here && e0 + el == a.pin_elem && n == a.pin_node) acc[ci] = a.pin_scale * a.x[row + n];
-          acc[ci] *= a.alpha;
-          if (a.beta != T(0)) acc[ci] += a.beta * yold[nt][ri][ci];
+          T v = y[nt][ri][ci];
+          if (pin_here && e0 + g + 8 * ri == a.pin_elem && frag_node<T, DIM, P>(nt, ci, t) == a.pin_node)
+            v = a.pin_scale * upin;
+          v *= a.alpha;
+          if (a.beta != T(0)) v += a.beta * yold[nt][ri][ci];
+          y[nt][ri][ci] = v;
         }
-        const int n0 = 8 * nt + 2 * t;
-        if (NP % 2 == 0) {
-          if (n0 < NP) *reinterpret_cast<typename F::V2*>(a.y + row + n0) = typename F::V2{acc[0], acc[1]};
-        } else {
-          if (n0 < NP) a.y[row + n0] = acc[0];
-          if (n0 + 1 < NP) a.y[row + n0 + 1] = acc[1];
+    store_nodes<T, DIM, P>(a.y, e0, ne, y, g, t);
+    // trace records: gathered by (element, face), then written out as one contiguous piece
+    __syncwarp();
+    T ru[FPL][TRP], rq[FPL][TRP];
+#pragma unroll
+    for (int i = 0; i < FPL; ++i) {
+      T fg[4] = {T(0), T(0), T(0), T(0)};
+      const bool in = gf0 + i < NF && gel < ne;
+      if (in) ld4(a.fgeo + ((size_t)(e0 + gel) * NF + gf0 + i) * 4, fg);
+#pragma unroll
+      for (int j = 0; j < TRP; ++j) {
+        ru[i][j] = rq[i][j] = T(0);
+        if (j < NFP) {
+          T h[4];
+          ld4(W + (gel * HS + ((fm[i][j / 4] >> (8 * (j % 4))) & 255u)) * 4, h);
+          ru[i][j] = h[0];
+          T q = fg[1] * h[1];
+#pragma unroll
+          for (int r = 1; r < DIM; ++r) q += fg[1 + r] * h[1 + r];
+          rq[i][j] = -q;  // fgeo holds -sJ c_r / 2
         }
       }
+    }
     __syncwarp();
+#pragma unroll
+    for (int i = 0; i < FPL; ++i)
+      if (gf0 + i < NF)
+#pragma unroll
+        for (int j = 0; j < TRP; j += 2)
+          st4(W + (gel * NF + gf0 + i) * TR + 2 * j, ru[i][j], rq[i][j], ru[i][j + 1], rq[i][j + 1]);
+    __syncwarp();
+    {
+      using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+      constexpr int VPC = 16 / sizeof(T), FULL = TE * NF * TR / VPC;
+      const int n = ne * (NF * TR / VPC);
+      V4* dst = reinterpret_cast<V4*>(trace + (size_t)e0 * NF * TR);
+#pragma unroll
+      for (int i0 = 0; i0 < FULL; i0 += 32)
+        if (i0 + lane < n) dst[i0 + lane] = reinterpret_cast<const V4*>(W)[i0 + lane];
+    }
   }
+}
+
+// ---------------------------------------------------------------- pass 2
+// This lane's face-node pair of block fb: its face f and first node j0 (f = NF past the last).
+template <typename T, int DIM, int P>
+__device__ __forceinline__ void fb_pair(int fb, int t, int& f, int& j0) {
+  using X = Tc<T, DIM, P>;
+  const int k0 = 8 * fb + 2 * t;
+  f = k0 / X::TRP;
+  j0 = k0 % X::TRP;
+}
+
+template <typename T, int DIM, int P, int WARPS, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
+                                                                     const T* __restrict__ trace) {
+  using X = Tc<T, DIM, P>;
+  using C = Cfg<DIM, P>;
+  using F = Frag<T>;
+  using V2 = typename F::V2;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT, R = X::R, TE = X::TE, TR = X::TR,
+                TRP = X::TRP, HP = TRP / 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* B = reinterpret_cast<T*>(smem_raw);
+  uint16_t* ptab = reinterpret_cast<uint16_t*>(B + X::N2);  // [orientation][pair]: neighbour positions of a node pair
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int ntiles = (a.K + TE - 1) / TE;
+  const int stride = gridDim.x * WARPS;
+  int tile = warp * gridDim.x + blockIdx.x;  // warp-major, as in pass 1
+  pdl_trigger();
+  copy_blob(B, blob, X::N2 * (int)sizeof(T));
+  for (int i = threadIdx.x; i < C::NPERM * HP; i += blockDim.x) {
+    const int sg = i / HP, j = 2 * (i % HP);
+    const int8_t* pp = a.itab + NF * NFP + sg * NFP;
+    ptab[i] = (uint16_t)(pp[j] | ((j + 1 < NFP ? pp[j + 1] : j + 1) << 8));  // a padding node maps to itself
+  }
+  // this lane's node pair per block: volume nodes
+  unsigned fmn[FT];
+#pragma unroll
+  for (int fb = 0; fb < FT; ++fb) {
+    int f, j0;
+    fb_pair<T, DIM, P>(fb, t, f, j0);
+    fmn[fb] = 0;
+    if (f < NF) {
+      const unsigned m0 = (uint8_t)a.itab[f * NFP + j0];
+      fmn[fb] = m0 | ((j0 + 1 < NFP ? (unsigned)(uint8_t)a.itab[f * NFP + j0 + 1] : m0) << 8);
+    }
+  }
+  // connectivity of the lane's elements (set-up data)
+  int nb[R][NF];
+  uint32_t code[R];
+  auto load_conn = [&](int tl) {
+#pragma unroll
+    for (int ri = 0; ri < R; ++ri) {
+      const int e = tl * TE + g + 8 * ri;
+      if (tl < ntiles && e < a.K) {
+        if (NF == 4) {
+          const int4 q = *reinterpret_cast<const int4*>(a.nbr + (size_t)e * NF);
+          nb[ri][0] = q.x; nb[ri][1] = q.y; nb[ri][2] = q.z; nb[ri][NF - 1] = q.w;
+        } else {
+#pragma unroll
+          for (int f = 0; f < NF; ++f) nb[ri][f] = a.nbr[(size_t)e * NF + f];
+        }
+        code[ri] = a.fcode[e];
+      }
+    }
+  };
+  load_conn(tile);
+  pdl_wait();
   cp_wait_all();
+  __syncthreads();
+  for (; tile < ntiles; tile += stride) {
+    const int e0 = tile * TE;
+    const int ne = min(TE, a.K - e0);
+    T yold[NT][R][2];
+    load_nodes<T, DIM, P>(a.y, e0, ne, yold, g, t);
+    T y[NT][R][2];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri) y[nt][ri][0] = y[nt][ri][1] = T(0);
+#pragma unroll
+    for (int fb = 0; fb < FT; ++fb) {
+      int f, j0;
+      fb_pair<T, DIM, P>(fb, t, f, j0);
+      T fu[R][2], sv[DIM][R][2];
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri) {
+        fu[ri][0] = fu[ri][1] = T(0);
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) sv[r][ri][0] = sv[r][ri][1] = T(0);
+        const int e = e0 + g + 8 * ri;
+        if (g + 8 * ri < ne && f < NF) {
+          int n = nb[ri][0];
+#pragma unroll
+          for (int k = 1; k < NF; ++k) n = f == k ? nb[ri][k] : n;
+          const unsigned cf = (code[ri] >> (8 * f)) & 255u;
+          const T* own = trace + ((size_t)e * NF + f) * TR;
+          T um[4], fg[4];
+          ld4(own + 2 * j0, um);  // u, q of the pair's nodes
+          ld4(a.fgeo + ((size_t)e * NF + f) * 4, fg);
+          // exterior: the neighbour's record, or the own one (with a sign) on a boundary face
+          const unsigned kk = n >= 0 ? ptab[(cf >> 2) * HP + (j0 >> 1)] : (unsigned)(j0 | ((j0 + 1) << 8));
+          const T* rec = n >= 0 ? trace + ((size_t)n * NF + (cf & 3u)) * TR : own;
+          V2 p0 = ld2(rec + 2 * (kk & 255u)), p1 = ld2(rec + 2 * (kk >> 8));
+          if (n < 0 && a.bct[-n - 1] == BC_DIRICHLET) {
+            p0.x = -p0.x; p0.y = -p0.y;
+            p1.x = -p1.x; p1.y = -p1.y;
+          }
+          T s0 = um[0] - p0.x, s1 = um[2] - p1.x;
+          fu[ri][0] = fg[0] * s0 - (um[1] - p0.y);
+          fu[ri][1] = fg[0] * s1 - (um[3] - p1.y);
+          if (a.factor) {
+            s0 *= a.factor[(size_t)e * NP + (fmn[fb] & 255u)];
+            s1 *= a.factor[(size_t)e * NP + (fmn[fb] >> 8)];
+          }
+#pragma unroll
+          for (int r = 0; r < DIM; ++r) {
+            sv[r][ri][0] = fg[1 + r] * s0;
+            sv[r][ri][1] = fg[1 + r] * s1;
+          }
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        F::mma(y[nt], fu, ldb(B + X::BE, fb * NT + nt, lane));
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) F::mma(y[nt], sv[r], ldb(B + X::BQ, (r * FT + fb) * NT + nt, lane));
+      }
+    }
+    load_conn(tile + stride);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int ri = 0; ri < R; ++ri)
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          const bool pinned = e0 + g + 8 * ri == a.pin_elem && frag_node<T, DIM, P>(nt, ci, t) == a.pin_node;
+          y[nt][ri][ci] = yold[nt][ri][ci] + (pinned ? T(0) : a.alpha * y[nt][ri][ci]);
+        }
+    store_nodes<T, DIM, P>(a.y, e0, ne, y, g, t);
+  }
+}
+
+// Face coefficients of an operator, one thread per element face: (sJ tau / 2, -sJ c_r / 2).
+template <typename T, int DIM, int TE>
+__global__ void k_face_geo(const T* __restrict__ tcg, const T* __restrict__ tau, int K, T* __restrict__ out) {
+  constexpr int NF = DIM + 1, NV = 8, NFG = 4, GROWS = NV + NFG * NF;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * NF; i += gridDim.x * blockDim.x) {
+    const int e = i / NF, f = i % NF;
+    const T* g = tcg + (size_t)(e / TE) * GROWS * TE + e % TE;
+    const T hs = T(0.5) * g[(NV + f) * TE];
+    st4(out + (size_t)i * 4, hs * tau[i], -hs * g[(NV + NF + f) * TE], -hs * g[(NV + 2 * NF + f) * TE],
+        -hs * g[(NV + 3 * NF + f) * TE]);
+  }
 }
 
 // Geometry blocks of the tensor-core apply, one thread per element slot of a
@@ -856,97 +692,61 @@ constexpr int kSmemBudget = 227 * 1024;
 template <typename T, int DIM, int P>
 constexpr size_t smem1(int w) {
   using X = Tc<T, DIM, P>;
-  return (size_t)(X::N1 + w * X::W1_T) * sizeof(T) + X::NF * X::NFP;
-}
-template <typename T, int DIM, int P, int NS>
-constexpr size_t smem2(int w) {
-  using X = Tc<T, DIM, P>;
-  return (size_t)(X::N2 + w * W2<T, DIM, P, NS>::T_) * sizeof(T) + (size_t)w * X::W2_I * 4 + Cfg<DIM, P>::ITAB;
+  return (size_t)(X::N1 + w * X::W1) * sizeof(T);
 }
 template <typename T, int DIM, int P>
-constexpr int warps1() {
-  int w = 16;
-  while (w > 1 && smem1<T, DIM, P>(w) > (size_t)kSmemBudget) --w;
-  return w;
-}
-// 0 when not even one warp tile fits next to the constants
-template <typename T, int DIM, int P, int NS>
-constexpr int warps2() {
-  int w = 16;
-  while (w > 0 && smem2<T, DIM, P, NS>(w) > (size_t)kSmemBudget) --w;
-  return w;
+constexpr size_t smem2() {
+  using X = Tc<T, DIM, P>;
+  return (size_t)X::N2 * sizeof(T) + Cfg<DIM, P>::NPERM * (X::TRP / 2) * sizeof(uint16_t);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <typename T, int DIM, int P, int WARPS>
-cudaError_t launch_pass1(const ApplyArgs<T>& a, const T* blob, T* trace, int ntiles, int num_sms, cudaStream_t s) {
-  static_assert(WARPS >= 1 && smem1<T, DIM, P>(WARPS) <= (size_t)kSmemBudget, "pass-1 warps do not fit");
-  auto k = sipg_trace_kernel<T, DIM, P, WARPS>;
-  const size_t bytes = smem1<T, DIM, P>(WARPS);
+template <typename Kern, typename T, typename TT>
+cudaError_t launch_pass(Kern k, const ApplyArgs<T>& a, const T* blob, TT* trace, int warps, size_t bytes, int ntiles,
+                        int num_sms, cudaStream_t s) {
   cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (err != cudaSuccess) return err;
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, WARPS * 32, bytes);
-  const int grid = std::min((ntiles + WARPS - 1) / WARPS, num_sms * std::max(per_sm, 1));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, warps * 32, bytes);
+  const int grid = std::min(ntiles, num_sms * std::max(per_sm, 1));
   if (grid > 0) {
-    pdl_launch(k, dim3(grid), dim3(WARPS * 32), bytes, s, a, blob, trace);
+    err = pdl_launch(k, dim3(grid), dim3(warps * 32), bytes, s, a, blob, trace);
+    if (err != cudaSuccess) return err;
     note_launch();
   }
   return cudaSuccess;
 }
 
-template <typename T, int DIM, int P, int NS, int WARPS>
-cudaError_t launch_pass2(const ApplyArgs<T>& a, const T* blob, const T* trace, int ntiles, int num_sms,
-                         cudaStream_t s) {
-  static_assert(WARPS >= 1 && smem2<T, DIM, P, NS>(WARPS) <= (size_t)kSmemBudget, "pass-2 warps do not fit");
-  auto k = sipg_apply_tc_kernel<T, DIM, P, WARPS, NS>;
-  const size_t bytes = smem2<T, DIM, P, NS>(WARPS);
-  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+template <typename T, int DIM, int P, int WARPS, int MINB>
+cudaError_t launch_passes(const ApplyArgs<T>& a, const T* blob, T* trace, int ntiles, int num_sms, cudaStream_t s) {
+  static_assert(smem1<T, DIM, P>(WARPS) <= (size_t)kSmemBudget && smem2<T, DIM, P>() <= (size_t)kSmemBudget,
+                "the operands do not fit");
+  cudaError_t err = launch_pass(sipg_volume_kernel<T, DIM, P, WARPS, MINB>, a, blob, trace, WARPS,
+                                smem1<T, DIM, P>(WARPS), ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, WARPS * 32, bytes);
-  const int grid = std::min((ntiles + WARPS - 1) / WARPS, num_sms * std::max(per_sm, 1));
-  if (grid > 0) {
-    pdl_launch(k, dim3(grid), dim3(WARPS * 32), bytes, s, a, blob, trace);
-    note_launch();
-  }
-  return cudaSuccess;
+  return launch_pass(sipg_face_kernel<T, DIM, P, WARPS, MINB>, a, blob + Tc<T, DIM, P>::N1, (const T*)trace, WARPS,
+                     smem2<T, DIM, P>(), ntiles, num_sms, s);
 }
 
-constexpr int cmin(int a, int b) { return a < b ? a : b; }
-
-// Launch shapes by the number of warp tiles: large meshes run as many warps per SM
-// as shared memory allows (pass 2 single-buffered once every warp has at least two
-// tiles); meshes with fewer tiles than a full-width wave over the SMs use narrow
-// CTAs (4 or 2 warps), so that every SM gets work.
+// Launch shape: two CTAs of 8 warps per SM where their shared memory fits (128 registers
+// per thread), else (FP64 p = 4 in 3D) one of 12. A grid of min(tiles, resident CTAs) with
+// warp-major tiles spreads any number of tiles over all SMs: on a small mesh a CTA has one
+// tile and its other warps only help to copy the operands.
 template <typename T, int DIM, int P>
 cudaError_t launch_tc_t(const ApplyArgs<T>& a, const T* blob, T* trace, int num_sms, cudaStream_t s) {
-  constexpr int WA = warps1<T, DIM, P>(), W2D = warps2<T, DIM, P, 2>(), W2S = warps2<T, DIM, P, 1>();
-  if (W2D < 1) return cudaErrorInvalidConfiguration;
   using X = Tc<T, DIM, P>;
   if constexpr (std::is_same<T, float>::value) {
     // FP32: the tcgen05 kernels (their constants follow the mma.sync blob)
     if (a.tcgen05 && tc5_supported(DIM, P)) return launch_apply_tc5(DIM, P, a, blob + X::NALL, trace, num_sms, s);
   }
-  // the kernels copy caller vectors in 16-byte pieces: other alignments take the CUDA-core kernel
+  // the kernels read caller vectors in 16-byte pieces: other alignments take the CUDA-core kernel
   if (!aligned16(a.x) || !aligned16(a.y) || !aligned16(trace) || (a.factor && !aligned16(a.factor)) ||
       (a.beta != T(0) && !aligned16(a.c)))
     return launch_apply<T>(DIM, P, a, num_sms, s);
   const int ntiles = (a.K + X::TE - 1) / X::TE;
-  const long long wave = (long long)num_sms;
-  cudaError_t err;
-  // pass 1 on large meshes: at most 12 warps per SM. It is latency-bound, so the
-  // time goes with the number of tile rounds; at 24^3 x 6 tets (35 tiles per SM in
-  // FP32, 70 in FP64) 12 warps give full rounds where 15 or 16 leave a partial one
-  if (ntiles >= wave * WA) err = launch_pass1<T, DIM, P, cmin(12, WA)>(a, blob, trace, ntiles, num_sms, s);
-  else if (ntiles >= wave * 4) err = launch_pass1<T, DIM, P, cmin(4, WA)>(a, blob, trace, ntiles, num_sms, s);
-  else err = launch_pass1<T, DIM, P, cmin(2, WA)>(a, blob, trace, ntiles, num_sms, s);
-  if (err != cudaSuccess) return err;
-  if (W2S > W2D && ntiles >= 2 * wave * W2S) err = launch_pass2<T, DIM, P, 1, (W2S > W2D ? W2S : W2D)>(a, blob, trace, ntiles, num_sms, s);
-  else if (ntiles >= wave * W2D) err = launch_pass2<T, DIM, P, 2, W2D>(a, blob, trace, ntiles, num_sms, s);
-  else if (ntiles >= wave * 4) err = launch_pass2<T, DIM, P, 2, cmin(4, W2D)>(a, blob, trace, ntiles, num_sms, s);
-  else err = launch_pass2<T, DIM, P, 2, cmin(2, W2D)>(a, blob, trace, ntiles, num_sms, s);
+  constexpr bool two = 2 * (smem1<T, DIM, P>(8) + 1024) <= (size_t)kSmemBudget + 1024;
+  const cudaError_t err = launch_passes<T, DIM, P, two ? 8 : 12, two ? 2 : 1>(a, blob, trace, ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
   return cudaGetLastError();
 }
@@ -955,7 +755,7 @@ cudaError_t launch_tc_t(const ApplyArgs<T>& a, const T* blob, T* trace, int num_
 template <typename T, int DIM, int P>
 void build_tc_consts_t(const RefElement& r, std::vector<double>& out) {
   using X = Tc<T, DIM, P>;
-  constexpr int NP = X::NP, NT = X::NT, FT = X::FT, KF = X::KF;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT;
   out.assign(X::NALL, 0.0);
   // entry (row, col) of a logical matrix stored as 8 x 8 blocks, nblk_n blocks per block row
   auto put = [&](int base, int nblk_n, int row, int col, double v) {
@@ -963,21 +763,32 @@ void build_tc_consts_t(const RefElement& r, std::vector<double>& out) {
     const int lane = gg * 4 + kr / 2;
     out[(size_t)base + ((size_t)(kb * nblk_n + nt) * 32 + lane) * 2 + (kr % 2)] = v;
   };
+  // logical column of node m: HALF's last block has one node per lane of a quad (columns 0, 2, 4, 6)
+  auto col = [](int m) { return X::HALF && m / 8 == NT - 1 ? m / 8 * 8 + 2 * (m % 8) : m; };
+  // logical column of face node (f, j): faces padded to TRP
+  auto fcol = [](int f, int j) { return f * X::TRP + j; };
   const double* D[3] = {r.Dr.data(), r.Ds.data(), r.Dt.data()};
   for (int rr = 0; rr < DIM; ++rr)
     for (int m = 0; m < NP; ++m)
       for (int n = 0; n < NP; ++n) {
-        put(X::B1 + rr * NT * NT * X::BLK, NT, n, m, D[rr][m * NP + n]);  // B1_r[n][m] = D_r[m][n]
-        put(X::B3 + rr * NT * NT * X::BLK, NT, m, n, D[rr][m * NP + n]);  // B3_r[m][n] = D_r[m][n]
+        put(X::B1 + rr * NT * NT * X::BLK, NT, col(n), col(m), D[rr][m * NP + n]);  // B1_r[n][m] = D_r[m][n]
+        double v = 0.0;
+        for (int k = 0; k < NP; ++k) v += r.M[m * NP + k] * D[rr][k * NP + n];
+        put(X::BS + rr * NT * NT * X::BLK, NT, col(m), col(n), v);                  // BS_r = M D_r
       }
   for (int m = 0; m < NP; ++m)
-    for (int n = 0; n < NP; ++n) put(X::BM, NT, m, n, r.M[n * NP + m]);     // BM[m][n] = M[n][m]
-  for (int k = 0; k < KF; ++k)
-    for (int n = 0; n < NP; ++n) put(X::BE, NT, k, n, r.EMAT[n * KF + k]);  // BE[k][n] = EMAT[n][k]
-  for (int rr = 0; rr < DIM; ++rr)
-    for (int n = 0; n < NP; ++n)
-      for (int k = 0; k < KF; ++k)
-        put(X::BF + rr * NT * FT * X::BLK, FT, n, k, D[rr][r.fmask[k] * NP + n]);  // BF_r[n][k] = D_r[m(k)][n]
+    for (int n = 0; n < NP; ++n) put(X::BM, NT, col(m), col(n), r.M[n * NP + m]);   // BM[m][n] = M[n][m]
+  for (int f = 0; f < NF; ++f)
+    for (int j = 0; j < NFP; ++j)
+      for (int n = 0; n < NP; ++n) {
+        const int k = f * NFP + j;
+        put(X::N1 + X::BE, NT, fcol(f, j), col(n), r.EMAT[n * NF * NFP + k]);       // BE[k][n] = EMAT[n][k]
+        for (int rr = 0; rr < DIM; ++rr) {
+          double v = 0.0;
+          for (int m = 0; m < NP; ++m) v += D[rr][m * NP + n] * r.EMAT[m * NF * NFP + k];
+          put(X::N1 + X::BQ + rr * FT * NT * X::BLK, NT, fcol(f, j), col(n), v);    // BQ_r[k][n] = (D_r^T EMAT)[n][k]
+        }
+      }
   if (std::is_same<T, float>::value) {
     std::vector<double> t5;  // empty where the order has no tcgen05 kernels
     build_tc5_consts(DIM, P, r, t5);
@@ -1013,12 +824,6 @@ void build_tc_consts(int dim, int order, const RefElement& r, std::vector<double
 }
 
 template <typename T>
-int tc_warps_for(int dim, int order) {
-  SIPG_DISPATCH_TC(dim, order, return warps2<T, D, P, 2>());
-  return 0;
-}
-
-template <typename T>
 size_t tc_geom_values(int dim, int K) {
   constexpr int TE = 8 * Frag<T>::R;
   const size_t ntiles = ((size_t)K + TE - 1) / TE;
@@ -1038,6 +843,19 @@ cudaError_t launch_tc_geom(int dim, const T* geof, int K, T* out, cudaStream_t s
   return cudaGetLastError();
 }
 
+template <typename T>
+cudaError_t launch_face_geo(int dim, const T* tcg, const T* tau, int K, T* out, cudaStream_t s) {
+  constexpr int TE = 8 * Frag<T>::R;
+  const size_t n = (size_t)K * (dim + 1);
+  const int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+  if (grid == 0) return cudaSuccess;
+  if (dim == 3) k_face_geo<T, 3, TE><<<grid, 256, 0, s>>>(tcg, tau, K, out);
+  else if (dim == 2) k_face_geo<T, 2, TE><<<grid, 256, 0, s>>>(tcg, tau, K, out);
+  else return cudaErrorInvalidValue;
+  note_launch();
+  return cudaGetLastError();
+}
+
 size_t tc_trace_values(int dim, int order, int K) {
   const int trp = rup(nfp_of(dim, order), 2);
   return (size_t)K * (dim + 1) * rup(2 * trp, 4);
@@ -1049,8 +867,8 @@ template cudaError_t launch_apply_tc<double>(int, int, const ApplyArgs<double>&,
                                              cudaStream_t);
 template void build_tc_consts<float>(int, int, const RefElement&, std::vector<double>&);
 template void build_tc_consts<double>(int, int, const RefElement&, std::vector<double>&);
-template int tc_warps_for<float>(int, int);
-template int tc_warps_for<double>(int, int);
+template cudaError_t launch_face_geo<float>(int, const float*, const float*, int, float*, cudaStream_t);
+template cudaError_t launch_face_geo<double>(int, const double*, const double*, int, double*, cudaStream_t);
 template size_t tc_geom_values<float>(int, int);
 template size_t tc_geom_values<double>(int, int);
 template cudaError_t launch_tc_geom<float>(int, const float*, int, float*, cudaStream_t);

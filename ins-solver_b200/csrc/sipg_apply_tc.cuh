@@ -20,9 +20,10 @@ cudaError_t launch_apply_tc(int dim, int order, const ApplyArgs<T>& a, const T* 
 size_t tc_trace_values(int dim, int order, int K);
 template <typename T>
 void build_tc_consts(int dim, int order, const RefElement& r, std::vector<double>& out);
-// Warps per CTA of the apply pass (below 2: use the CUDA-core kernel).
+// Face coefficients of an operator (ApplyArgs::fgeo), K x NF x 4 values: sJ tau / 2 and
+// -sJ c_r / 2, from the mesh's geometry blocks and the operator's penalty.
 template <typename T>
-int tc_warps_for(int dim, int order);
+cudaError_t launch_face_geo(int dim, const T* tcg, const T* tau, int K, T* out, cudaStream_t s);
 // Element and face geometry of the tensor-core apply (ApplyArgs::tcg), computed
 // once per mesh from the K x NG geometric factors: tc_geom_values<T>(dim, K)
 // values, one block per warp tile of elements (zero past K).

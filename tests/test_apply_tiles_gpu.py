@@ -1,0 +1,31 @@
+"""Edges of the tensor-core apply's warp tiles (8 elements FP64, 16 FP32): meshes below one
+tile, exactly some tiles and with a remainder, a pinned DOF in the last tile, and the
+in-place apply (y over x), at every order in 2D and 3D."""
+import numpy as np
+import pytest
+
+import oracle_py as O
+import sipg
+from helpers import TOL_FP64, TOL_TF32, DevArray, make_op, random_case, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("dim,n", [(2, 1), (2, 4), (2, 5), (3, 1), (3, 2), (3, 3)])
+def test_tile_edges_pin_and_in_place(dim, n, order):
+    mesh, t, e, om, x, f, m, bct = random_case(dim, n, order, 1, seed=7 * order + dim)
+    op = make_op(mesh, order, 1, f, bct=bct)
+    K, Np = mesh.K, x.shape[2]
+    op.set_pin(K - 1, Np - 1)
+    xs = x.copy()
+    xs[0, K - 1, Np - 1] = 0.0
+    ref = O.mult(om, xs, bct, f)
+    ref[0, K - 1, Np - 1] = O.diag(om, 1, bct, f)[0, K - 1, Np - 1] * x[0, K - 1, Np - 1]
+    for prec, dtype, tol in ((sipg.FP64, np.float64, TOL_FP64), (sipg.FP32, np.float32, TOL_TF32)):
+        xd, yd = DevArray(x.astype(dtype)), DevArray(np.full(x.shape, 7.0, dtype))
+        op.apply_device(prec, xd.p, yd.p)
+        y = yd.get()
+        assert rel_err(y.astype(np.float64), ref) < tol
+        op.apply_device(prec, xd.p, xd.p)  # every tile reads its own rows before it writes them
+        assert np.array_equal(xd.get(), y)
