@@ -236,9 +236,10 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
   a.beta = beta;
   a.c = c ? c : y;
   a.tcg = f64 ? (const T*)mesh->tcg64.p : (const T*)mesh->tcg32.p;
+  a.nrec = nrec.as<uint32_t>();
   a.fgeo = f64 ? (const T*)fgeo64.p : (const T*)fgeo32.p;
   a.tcgen05 = kernel == 3;
-  const bool tc_ok = kernel == 0 || kernel >= 2;
+  const bool tc_ok = (kernel == 0 || kernel >= 2) && nrec.p;
   if (tc_ok && ncomp > 1 && pin_elem < 0) {
     // vector operator: one tensor-core scalar apply per component (its own boundary
     // types; slip faces get no face terms there), then the slip faces' coupling terms
@@ -252,7 +253,7 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
       ac.x = x + comp * per;
       ac.y = y + comp * per;
       ac.c = a.c + comp * per;
-      ac.bct = bct.as<uint8_t>() + (size_t)comp * mesh->Kb;
+      ac.nrec = nrec.as<uint32_t>() + (size_t)comp * mesh->K * (mesh->dim + 1);
       SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, ac, tcc, tr.as<T>(), num_sms(), s));
     }
     SIPG_CUDA(launch_slip<T>(mesh->dim, order, a, mesh->belems.as<int>(), mesh->n_belem, s));
@@ -280,10 +281,17 @@ void sipg_op::refresh_tau(cudaStream_t s) {
   SIPG_CUDA(launch_tau<float>(mesh->dim, order, dref->itab.as<int8_t>(), mesh->geof32.as<float>(),
                               mesh->nbr.as<int>(), mesh->fcode.as<uint32_t>(), f32, mesh->K,
                               tau32.as<float>(), s));
-  SIPG_CUDA(launch_face_geo<double>(mesh->dim, mesh->tcg64.as<double>(), tau64.as<double>(), mesh->K,
-                                    fgeo64.as<double>(), s));
-  SIPG_CUDA(launch_face_geo<float>(mesh->dim, mesh->tcg32.as<float>(), tau32.as<float>(), mesh->K,
-                                   fgeo32.as<float>(), s));
+  SIPG_CUDA(launch_face_geo(mesh->dim, mesh->tcg64.as<double>(), tau64.as<double>(), fgeo64.as<double>(),
+                            mesh->tcg32.as<float>(), tau32.as<float>(), fgeo32.as<float>(), mesh->K, s));
+}
+
+void sipg_op::refresh_bc() {
+  if (!nrec.p) return;
+  for (int c = 0; c < ncomp; ++c)
+    SIPG_CUDA(launch_neighbour_records(mesh->dim, mesh->nbr.as<int>(), mesh->fcode.as<uint32_t>(),
+                                       bct.as<uint8_t>() + (size_t)c * mesh->Kb, mesh->K,
+                                       nrec.as<uint32_t>() + (size_t)c * mesh->K * (mesh->dim + 1), 0));
+  SIPG_CUDA(cudaStreamSynchronize(0));
 }
 
 BlockArgs sipg_op::block_args(int mode, int ref_volume, double* out, bool with_pin) const {
@@ -345,6 +353,8 @@ std::unique_ptr<sipg_op> create_op(sipg_mesh* m, int order, int ncomp) {
   op->bct = DevBuf(std::max<size_t>(1, op->bct_host.size()));
   std::vector<uint8_t> b(op->bct_host.size(), 0);
   if (!b.empty()) op->bct.upload(b.data(), b.size());
+  if (neighbour_records_fit(m->dim, m->K)) op->nrec = DevBuf((size_t)ncomp * m->K * Nf * sizeof(uint32_t));
+  op->refresh_bc();
   op->eb64 = apply_pick_eb(m->dim, order, ncomp, true);
   op->eb32 = apply_pick_eb(m->dim, order, ncomp, false);
   op->refresh_tau(0);
@@ -387,6 +397,7 @@ void set_bc_types_host(sipg_op* op, const std::vector<int>& types) {
     op->bct_host[i] = types[i];
   }
   if (n) op->bct.upload(b.data(), n);
+  op->refresh_bc();
 }
 }  // namespace sipg
 
@@ -597,6 +608,7 @@ int sipg_op_set_bc_types(sipg_op* op, const int* types) {
       op->bct_host[i] = types[i];
     }
     if (n) op->bct.upload(b.data(), n);
+    op->refresh_bc();
     op->refresh_pin(0);
     if (op->oi) {
       oi_assemble(op, 0);

@@ -100,6 +100,7 @@ struct sipg_op {
   sipg::DevBuf mm64, mm32;
   sipg::DevBuf bct;           // ncomp x Kb uint8
   std::vector<int> bct_host;  // ncomp x Kb
+  sipg::DevBuf nrec;          // neighbour records of the tensor-core apply, ncomp x K x Nf (ApplyArgs::nrec)
   int pin_elem = -1, pin_node = -1;
   double pin_scale = 1.0;
   int eb64 = 0, eb32 = 0;
@@ -117,6 +118,7 @@ struct sipg_op {
   // y = alpha A x + beta c, c = y when null (beta == 0: c is not read)
   void apply(const T* x, T* y, cudaStream_t s, T alpha = T(1), T beta = T(0), const T* c = nullptr) const;
   void refresh_tau(cudaStream_t s);
+  void refresh_bc();  // neighbour records after bct changed (synchronous)
   sipg::BlockArgs block_args(int mode, int ref_volume, double* out, bool with_pin) const;
   void apply_bc_device(const double* bc, double* rhs, cudaStream_t s) const;
   void refresh_pin(cudaStream_t s);

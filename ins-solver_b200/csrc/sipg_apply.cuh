@@ -78,6 +78,10 @@ __device__ __forceinline__ void simplex_face_normal(const double* g, int f, doub
 // Boundary condition types (problem_specific_3d.h: 0 Dirichlet, 1 Neumann; slip 2).
 enum : int { BC_DIRICHLET = 0, BC_NEUMANN = 1, BC_SLIP = 2 };
 
+// Codes of boundary faces in ApplyArgs::nrec, after the orientations (6 in 3D, 2 in 2D);
+// natural: Neumann, and slip faces, whose terms launch_slip adds
+enum : int { NREC_NATURAL = 6, NREC_DIRICHLET = 7 };
+
 // mm modes
 enum : int { MM_NONE = 0, MM_SCALAR = 1, MM_NODAL = 2 };
 
@@ -105,6 +109,8 @@ struct ApplyArgs {
   T alpha, beta;          // y = alpha * A x + beta * c (beta == 0: c is not read)
   const T* c;             // ncomp x K x NP; y unless the caller gives another vector
   const T* tcg;           // tensor-core path: tile-major element and face geometry (launch_tc_geom)
+  const uint32_t* nrec;   // tensor-core path: K x NF, neighbour record (nb NF + its face) << 3 | orientation;
+                          // a boundary face's own record with NREC_DIRICHLET or NREC_NATURAL
   const T* fgeo;          // tensor-core path: face coefficients K x NF x 4 (launch_face_geo)
   int tcgen05 = 0;        // tensor-core path, FP32: tcgen05 kernels where the order has them (else mma.sync)
 };

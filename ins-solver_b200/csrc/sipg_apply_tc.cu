@@ -38,10 +38,12 @@
 // from global memory straight into fragment registers (a quad of lanes reads a
 // contiguous piece of a row), so shared memory holds only the operands and, in
 // pass 1, the rearrangement of node values into trace records: more warps per SM
-// and fewer instructions than with every input staged. Measured per apply, before
-// and after that rearrangement: FP64 p = 4 Helmholtz at 48^3 x 6 tets 2.24 -> 1.22 ms
-// (DMMA-bound: 24 of the 37 TFLOP/s the FP64 pipe has), FP32 p = 3 two-phase at
-// 24^3 x 6 42.8 -> 37.5 us (latency-bound).
+// and fewer instructions than with every input staged. A boundary face is a code in its
+// neighbour record, so pass 2 has no branch between a tile's loads.
+// Measured per apply, with the earlier form (derivatives at the face nodes in pass 1, all
+// inputs staged) and now: FP64 p = 4 Helmholtz at 48^3 x 6 tets 2.24 -> 0.99 ms (30 of the
+// 37 TFLOP/s the FP64 pipe has, counting issued MMAs), FP64 p = 3 two-phase at 24^3 x 6
+// 97 -> 65 us, FP32 there 42.8 -> 32.4 us (L1 transactions of the gathers and latency).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -76,7 +78,7 @@ struct Frag<float> {
   // m16n8k8: a0 (g, t) a1 (g+8, t) a2 (g, t+4) a3 (g+8, t+4); b0 (t, g) b1 (t+4, g);
   // c0 (g, 2t) c1 (g, 2t+1) c2 (g+8, 2t) c3 (g+8, 2t+1).
   __device__ static __forceinline__ void mma(float (&c)[2][2], const float (&a)[2][2], V2 b) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%0,%1,%2,%3};\n"
         : "+f"(c[0][0]), "+f"(c[0][1]), "+f"(c[1][0]), "+f"(c[1][1])
@@ -95,12 +97,12 @@ struct Frag<double> {
   // binds slot t to logical column 2t, the second to 2t+1.
   __device__ static __forceinline__ void mma(double (&c)[1][2], const double (&a)[1][2], V2 b) {
     mma_half(c, a, b);
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(c[0][0]), "+d"(c[0][1])
                  : "d"(a[0][1]), "d"(b.y));
   }
   __device__ static __forceinline__ void mma_half(double (&c)[1][2], const double (&a)[1][2], V2 b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(c[0][0]), "+d"(c[0][1])
                  : "d"(a[0][0]), "d"(b.x));
   }
@@ -132,10 +134,17 @@ struct Tc {
   // rows (J, then the metric K = G G^T by rows of its upper triangle, zero rows),
   // then NFG x NF face rows [q][f] (q: sJ, c_0, c_1, c_2)
   static constexpr int NV = 8, NFG = 4, GROWS = NV + NFG * NF;
-  // pass 1 warp area: (x, h_0, h_1, h_2) per node, odd node stride, then reused for the tile's records
-  static constexpr int HS = NP | 1;
-  static constexpr int W1 = TE * HS * 4 > TE * NF * TR ? TE * HS * 4 : TE * NF * TR;
+  // pass 1 warp area: (x, h_0, h_1, h_2) per node in planes of 16 bytes (FP32 one, FP64 two),
+  // then reused for the tile's records; both element strides are odd numbers of 16-byte
+  // pieces, so lanes on consecutive elements hit distinct banks
+  static constexpr int VPC = 16 / (int)sizeof(T);    // values per 16-byte piece
+  static constexpr int HS = NP | 1;                  // pieces per element of a plane
+  static constexpr int RS = (NF * TR / VPC) | 1;     // pieces per element of the records
+  static constexpr int HW = TE * HS * 4, RW = TE * RS * VPC;
+  static constexpr int W1 = HW > RW ? HW : RW;
   static constexpr int LPE = 32 / TE, FPL = (NF + LPE - 1) / LPE;  // record gather: lanes per element, faces per lane
+  // the next tile's x is fetched during the products where registers allow
+  static constexpr bool PREFETCH = NT * R * 2 * (int)sizeof(T) <= 48;
 };
 
 // Row of the metric entry K_rs (r <= s) in the geometry block.
@@ -164,6 +173,27 @@ __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d
 __device__ __forceinline__ void st4(double* p, double a, double b, double c, double d) {
   reinterpret_cast<double2*>(p)[0] = make_double2(a, b);
   reinterpret_cast<double2*>(p)[1] = make_double2(c, d);
+}
+
+// (x, h_0, h_1, h_2) of a node in pass 1's planes: piece `at` of each
+template <int PLANE>
+__device__ __forceinline__ void st_node(float* w, int at, float x, float a, float b, float c) {
+  reinterpret_cast<float4*>(w)[at] = make_float4(x, a, b, c);
+}
+template <int PLANE>
+__device__ __forceinline__ void st_node(double* w, int at, double x, double a, double b, double c) {
+  reinterpret_cast<double2*>(w)[at] = make_double2(x, a);
+  reinterpret_cast<double2*>(w)[PLANE + at] = make_double2(b, c);
+}
+template <int PLANE>
+__device__ __forceinline__ void ld_node(const float* w, int at, float (&v)[4]) {
+  const float4 q = reinterpret_cast<const float4*>(w)[at];
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+template <int PLANE>
+__device__ __forceinline__ void ld_node(const double* w, int at, double (&v)[4]) {
+  const double2 q = reinterpret_cast<const double2*>(w)[at], r = reinterpret_cast<const double2*>(w)[PLANE + at];
+  v[0] = q.x; v[1] = q.y; v[2] = r.x; v[3] = r.y;
 }
 
 __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
@@ -304,7 +334,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
   using X = Tc<T, DIM, P>;
   using F = Frag<T>;
   constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, R = X::R, TE = X::TE, TR = X::TR, TRP = X::TRP,
-                HS = X::HS, LPE = X::LPE, FPL = X::FPL;
+                HS = X::HS, FPL = X::FPL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* B = reinterpret_cast<T*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -319,7 +349,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
   copy_blob(B, blob, (has_mm ? X::N1 : X::BM) * (int)sizeof(T));
   // record gather: this lane's element of the tile and the volume nodes of its faces, 4 per word
   constexpr int NW = (TRP + 3) / 4;
-  const int gel = lane / LPE, gf0 = (lane % LPE) * FPL;
+  const int gel = lane % TE, gf0 = (lane / TE) * FPL;
   unsigned fm[FPL][NW];
 #pragma unroll
   for (int i = 0; i < FPL; ++i)
@@ -356,6 +386,18 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
     T fac[NT][R][2];
     if (a.factor) load_nodes<T, DIM, P>(a.factor, e0, ne, fac, g, t);
     const T* gb = a.tcg + (size_t)tile * X::GROWS * TE;
+    T Jm[R], Km[R][DIM][DIM], fg[FPL][4];
+#pragma unroll
+    for (int ri = 0; ri < R; ++ri) {
+      Jm[ri] = gb[g + 8 * ri];
+#pragma unroll
+      for (int r = 0; r < DIM; ++r)
+#pragma unroll
+        for (int s = r; s < DIM; ++s) Km[ri][r][s] = gb[kidx(DIM, r, s) * TE + g + 8 * ri];
+    }
+#pragma unroll
+    for (int i = 0; i < FPL; ++i)  // the record gather's face coefficients
+      ld4(a.fgeo + ((size_t)min(e0 + gel, a.K - 1) * NF + min(gf0 + i, NF - 1)) * 4, fg[i]);
     // gr_r = x . B1_r
     T w[DIM][NT][R][2];
 #pragma unroll
@@ -376,15 +418,12 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
 #pragma unroll
     for (int ri = 0; ri < R; ++ri) {
       const int el = g + 8 * ri;
-      const T Jm = gb[el];
-      T Km[DIM][DIM];
 #pragma unroll
       for (int r = 0; r < DIM; ++r)
 #pragma unroll
         for (int s = r; s < DIM; ++s) {
-          const T v = Jm * gb[kidx(DIM, r, s) * TE + el];
-          Km[r][s] = v;
-          Km[s][r] = v;
+          Km[ri][r][s] *= Jm[ri];
+          Km[ri][s][r] = Km[ri][r][s];
         }
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
@@ -395,12 +434,12 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
 #pragma unroll
           for (int s = 0; s < DIM; ++s) h[s] = a.factor ? fac[nt][ri][ci] * w[s][nt][ri][ci] : w[s][nt][ri][ci];
           const int m = frag_node<T, DIM, P>(nt, ci, t);
-          if (8 * nt + 8 <= NP || m < NP) st4(W + (el * HS + m) * 4, u[nt][ri][ci], h[0], h[1], h[2]);
+          if (8 * nt + 8 <= NP || m < NP) st_node<TE * HS>(W, el * HS + m, u[nt][ri][ci], h[0], h[1], h[2]);
 #pragma unroll
           for (int r = 0; r < DIM; ++r) {
             T v = T(0);
 #pragma unroll
-            for (int s = 0; s < DIM; ++s) v += Km[r][s] * h[s];
+            for (int s = 0; s < DIM; ++s) v += Km[ri][r][s] * h[s];
             w[r][nt][ri][ci] = v;
           }
         }
@@ -421,14 +460,13 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
         for (int ri = 0; ri < R; ++ri)
 #pragma unroll
           for (int ci = 0; ci < 2; ++ci)
-            mx[ri][ci] = gb[g + 8 * ri] * (a.mm_mode == MM_NODAL ? mm[kb][ri][ci] : a.mm_scalar) * u[kb][ri][ci];
+            mx[ri][ci] = Jm[ri] * (a.mm_mode == MM_NODAL ? mm[kb][ri][ci] : a.mm_scalar) * u[kb][ri][ci];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) mma_nodes<T, DIM, P>(y[nt], mx, ldb(B + X::BM, kb * NT + nt, lane), kb);
       }
     }
-    // the next tile's x lands during the products
     const int next = tile + stride;
-    if (next < ntiles) load_nodes<T, DIM, P>(a.x, next * TE, min(TE, a.K - next * TE), u, g, t);
+    if (X::PREFETCH && next < ntiles) load_nodes<T, DIM, P>(a.x, next * TE, min(TE, a.K - next * TE), u, g, t);
 #pragma unroll
     for (int r = 0; r < DIM; ++r)
 #pragma unroll
@@ -458,19 +496,16 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
     T ru[FPL][TRP], rq[FPL][TRP];
 #pragma unroll
     for (int i = 0; i < FPL; ++i) {
-      T fg[4] = {T(0), T(0), T(0), T(0)};
-      const bool in = gf0 + i < NF && gel < ne;
-      if (in) ld4(a.fgeo + ((size_t)(e0 + gel) * NF + gf0 + i) * 4, fg);
 #pragma unroll
       for (int j = 0; j < TRP; ++j) {
         ru[i][j] = rq[i][j] = T(0);
         if (j < NFP) {
           T h[4];
-          ld4(W + (gel * HS + ((fm[i][j / 4] >> (8 * (j % 4))) & 255u)) * 4, h);
+          ld_node<TE * HS>(W, gel * HS + (int)((fm[i][j / 4] >> (8 * (j % 4))) & 255u), h);
           ru[i][j] = h[0];
-          T q = fg[1] * h[1];
+          T q = fg[i][1] * h[1];
 #pragma unroll
-          for (int r = 1; r < DIM; ++r) q += fg[1 + r] * h[1 + r];
+          for (int r = 1; r < DIM; ++r) q += fg[i][1 + r] * h[1 + r];
           rq[i][j] = -q;  // fgeo holds -sJ c_r / 2
         }
       }
@@ -481,30 +516,24 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
       if (gf0 + i < NF)
 #pragma unroll
         for (int j = 0; j < TRP; j += 2)
-          st4(W + (gel * NF + gf0 + i) * TR + 2 * j, ru[i][j], rq[i][j], ru[i][j + 1], rq[i][j + 1]);
+          st4(W + gel * X::RS * X::VPC + (gf0 + i) * TR + 2 * j, ru[i][j], rq[i][j], ru[i][j + 1], rq[i][j + 1]);
     __syncwarp();
     {
       using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-      constexpr int VPC = 16 / sizeof(T), FULL = TE * NF * TR / VPC;
-      const int n = ne * (NF * TR / VPC);
+      constexpr int PPE = NF * TR / X::VPC, FULL = TE * PPE;  // pieces per element, per tile
+      const int n = ne * PPE;
       V4* dst = reinterpret_cast<V4*>(trace + (size_t)e0 * NF * TR);
 #pragma unroll
-      for (int i0 = 0; i0 < FULL; i0 += 32)
-        if (i0 + lane < n) dst[i0 + lane] = reinterpret_cast<const V4*>(W)[i0 + lane];
+      for (int i0 = 0; i0 < FULL; i0 += 32) {
+        const int i = i0 + lane;
+        if (i < n) dst[i] = reinterpret_cast<const V4*>(W)[i + (X::RS - PPE) * (i / PPE)];
+      }
     }
+    if (!X::PREFETCH && next < ntiles) load_nodes<T, DIM, P>(a.x, next * TE, min(TE, a.K - next * TE), u, g, t);
   }
 }
 
 // ---------------------------------------------------------------- pass 2
-// This lane's face-node pair of block fb: its face f and first node j0 (f = NF past the last).
-template <typename T, int DIM, int P>
-__device__ __forceinline__ void fb_pair(int fb, int t, int& f, int& j0) {
-  using X = Tc<T, DIM, P>;
-  const int k0 = 8 * fb + 2 * t;
-  f = k0 / X::TRP;
-  j0 = k0 % X::TRP;
-}
-
 template <typename T, int DIM, int P, int WARPS, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
                                                                      const T* __restrict__ trace) {
@@ -513,59 +542,67 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
   using F = Frag<T>;
   using V2 = typename F::V2;
   constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT, R = X::R, TE = X::TE, TR = X::TR,
-                TRP = X::TRP, HP = TRP / 2;
+                TRP = X::TRP, HP = TRP / 2, NPERM = C::NPERM;
+  static_assert(NPERM <= NREC_NATURAL, "orientation codes");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* B = reinterpret_cast<T*>(smem_raw);
-  uint16_t* ptab = reinterpret_cast<uint16_t*>(B + X::N2);  // [orientation][pair]: neighbour positions of a node pair
+  uint16_t* ptab = reinterpret_cast<uint16_t*>(B + X::N2);  // [orientation][pair]: record positions of a pair's nodes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int ntiles = (a.K + TE - 1) / TE;
   const int stride = gridDim.x * WARPS;
   int tile = warp * gridDim.x + blockIdx.x;  // warp-major, as in pass 1
   pdl_trigger();
   copy_blob(B, blob, X::N2 * (int)sizeof(T));
-  for (int i = threadIdx.x; i < C::NPERM * HP; i += blockDim.x) {
+  for (int i = threadIdx.x; i < 8 * HP; i += blockDim.x) {
     const int sg = i / HP, j = 2 * (i % HP);
     const int8_t* pp = a.itab + NF * NFP + sg * NFP;
-    ptab[i] = (uint16_t)(pp[j] | ((j + 1 < NFP ? pp[j + 1] : j + 1) << 8));  // a padding node maps to itself
+    // a padding node and the nodes of a boundary face map to themselves
+    const int k0 = sg < NPERM ? pp[j] : j, k1 = sg < NPERM && j + 1 < NFP ? pp[j + 1] : j + 1;
+    ptab[i] = (uint16_t)(2 * k0 | (2 * k1) << 8);
   }
-  // this lane's node pair per block: volume nodes
-  unsigned fmn[FT];
+  // this lane's node pair per block: its face and volume nodes (KF padding: face NF)
+  int fb_f[FT], fb_m0[FT], fb_m1[FT];
 #pragma unroll
   for (int fb = 0; fb < FT; ++fb) {
-    int f, j0;
-    fb_pair<T, DIM, P>(fb, t, f, j0);
-    fmn[fb] = 0;
+    const int k0 = 8 * fb + 2 * t, f = k0 / TRP, j0 = k0 % TRP;
+    fb_f[fb] = f;
+    fb_m0[fb] = fb_m1[fb] = 0;
     if (f < NF) {
-      const unsigned m0 = (uint8_t)a.itab[f * NFP + j0];
-      fmn[fb] = m0 | ((j0 + 1 < NFP ? (unsigned)(uint8_t)a.itab[f * NFP + j0 + 1] : m0) << 8);
+      fb_m0[fb] = (uint8_t)a.itab[f * NFP + j0];
+      fb_m1[fb] = j0 + 1 < NFP ? (uint8_t)a.itab[f * NFP + j0 + 1] : fb_m0[fb];
     }
   }
-  // connectivity of the lane's elements (set-up data)
-  int nb[R][NF];
-  uint32_t code[R];
+  // connectivity of the lane's elements (set-up data): neighbour record << 3 | code.
+  // Rows past the tile's end repeat the mesh's last element: they are computed and not stored.
+  uint32_t nb[R][NF];
   auto load_conn = [&](int tl) {
 #pragma unroll
     for (int ri = 0; ri < R; ++ri) {
-      const int e = tl * TE + g + 8 * ri;
-      if (tl < ntiles && e < a.K) {
-        if (NF == 4) {
-          const int4 q = *reinterpret_cast<const int4*>(a.nbr + (size_t)e * NF);
-          nb[ri][0] = q.x; nb[ri][1] = q.y; nb[ri][2] = q.z; nb[ri][NF - 1] = q.w;
-        } else {
+      const int e = min(tl * TE + g + 8 * ri, a.K - 1);
+      if (NF == 4) {
+        const uint4 q = *reinterpret_cast<const uint4*>(a.nrec + (size_t)e * NF);
+        nb[ri][0] = q.x; nb[ri][1] = q.y; nb[ri][2] = q.z; nb[ri][NF - 1] = q.w;
+      } else {
 #pragma unroll
-          for (int f = 0; f < NF; ++f) nb[ri][f] = a.nbr[(size_t)e * NF + f];
-        }
-        code[ri] = a.fcode[e];
+        for (int f = 0; f < NF; ++f) nb[ri][f] = a.nrec[(size_t)e * NF + f];
       }
     }
   };
-  load_conn(tile);
+  if (tile < ntiles) load_conn(tile);
   pdl_wait();
   cp_wait_all();
   __syncthreads();
   for (; tile < ntiles; tile += stride) {
     const int e0 = tile * TE;
     const int ne = min(TE, a.K - e0);
+    const T *own[R], *fg_row[R], *f_row[R];
+#pragma unroll
+    for (int ri = 0; ri < R; ++ri) {
+      const int e = min(e0 + g + 8 * ri, a.K - 1);
+      own[ri] = trace + (size_t)e * NF * TR + 4 * t;
+      fg_row[ri] = a.fgeo + (size_t)e * NF * 4;
+      f_row[ri] = a.factor + (size_t)e * NP;
+    }
     T yold[NT][R][2];
     load_nodes<T, DIM, P>(a.y, e0, ne, yold, g, t);
     T y[NT][R][2];
@@ -575,44 +612,41 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
       for (int ri = 0; ri < R; ++ri) y[nt][ri][0] = y[nt][ri][1] = T(0);
 #pragma unroll
     for (int fb = 0; fb < FT; ++fb) {
-      int f, j0;
-      fb_pair<T, DIM, P>(fb, t, f, j0);
+      const int flo = 8 * fb / TRP;  // the block's first face; its pairs lie on flo .. fhi
+      const int fhi = (8 * fb + 6) / TRP;
+      const int f = fb_f[fb];
       T fu[R][2], sv[DIM][R][2];
 #pragma unroll
       for (int ri = 0; ri < R; ++ri) {
-        fu[ri][0] = fu[ri][1] = T(0);
+        uint32_t n = nb[ri][flo < NF ? flo : 0];
 #pragma unroll
-        for (int r = 0; r < DIM; ++r) sv[r][ri][0] = sv[r][ri][1] = T(0);
-        const int e = e0 + g + 8 * ri;
-        if (g + 8 * ri < ne && f < NF) {
-          int n = nb[ri][0];
-#pragma unroll
-          for (int k = 1; k < NF; ++k) n = f == k ? nb[ri][k] : n;
-          const unsigned cf = (code[ri] >> (8 * f)) & 255u;
-          const T* own = trace + ((size_t)e * NF + f) * TR;
-          T um[4], fg[4];
-          ld4(own + 2 * j0, um);  // u, q of the pair's nodes
-          ld4(a.fgeo + ((size_t)e * NF + f) * 4, fg);
-          // exterior: the neighbour's record, or the own one (with a sign) on a boundary face
-          const unsigned kk = n >= 0 ? ptab[(cf >> 2) * HP + (j0 >> 1)] : (unsigned)(j0 | ((j0 + 1) << 8));
-          const T* rec = n >= 0 ? trace + ((size_t)n * NF + (cf & 3u)) * TR : own;
-          V2 p0 = ld2(rec + 2 * (kk & 255u)), p1 = ld2(rec + 2 * (kk >> 8));
-          if (n < 0 && a.bct[-n - 1] == BC_DIRICHLET) {
-            p0.x = -p0.x; p0.y = -p0.y;
-            p1.x = -p1.x; p1.y = -p1.y;
-          }
-          T s0 = um[0] - p0.x, s1 = um[2] - p1.x;
-          fu[ri][0] = fg[0] * s0 - (um[1] - p0.y);
-          fu[ri][1] = fg[0] * s1 - (um[3] - p1.y);
+        for (int k = flo + 1; k <= fhi && k < NF; ++k) n = f == k ? nb[ri][k] : n;
+        const int sg = (int)(n & 7u);
+        const bool pad = X::KF % 8 != 0 && f >= NF;  // no face: its operand rows are zero, its values finite
+        const unsigned kk = ptab[sg * HP + ((8 * fb + 2 * t - TRP * f) >> 1)];
+        const T* rec = trace + (size_t)(n >> 3) * TR;
+        T um[4] = {T(0), T(0), T(0), T(0)}, fg[4] = {T(0), T(0), T(0), T(0)};
+        V2 p0{T(0), T(0)}, p1{T(0), T(0)};
+        T f0 = T(1), f1 = T(1);
+        if (!pad) {
+          ld4(own[ri] + 16 * fb, um);  // (u, q) of the pair's nodes
+          ld4(fg_row[ri] + 4 * f, fg);
+          p0 = ld2(rec + (kk & 255u));
+          p1 = ld2(rec + (kk >> 8));
           if (a.factor) {
-            s0 *= a.factor[(size_t)e * NP + (fmn[fb] & 255u)];
-            s1 *= a.factor[(size_t)e * NP + (fmn[fb] >> 8)];
+            f0 = f_row[ri][fb_m0[fb]];
+            f1 = f_row[ri][fb_m1[fb]];
           }
+        }
+        // exterior values: the neighbour's; a boundary face has its own, negated on Dirichlet faces
+        const T sgn = sg == NREC_DIRICHLET ? T(-1) : T(1);
+        const T s0 = um[0] - sgn * p0.x, s1 = um[2] - sgn * p1.x;
+        fu[ri][0] = fg[0] * s0 - (um[1] - sgn * p0.y);
+        fu[ri][1] = fg[0] * s1 - (um[3] - sgn * p1.y);
 #pragma unroll
-          for (int r = 0; r < DIM; ++r) {
-            sv[r][ri][0] = fg[1 + r] * s0;
-            sv[r][ri][1] = fg[1 + r] * s1;
-          }
+        for (int r = 0; r < DIM; ++r) {
+          sv[r][ri][0] = fg[1 + r] * (f0 * s0);
+          sv[r][ri][1] = fg[1 + r] * (f1 * s1);
         }
       }
 #pragma unroll
@@ -622,7 +656,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
         for (int r = 0; r < DIM; ++r) F::mma(y[nt], sv[r], ldb(B + X::BQ, (r * FT + fb) * NT + nt, lane));
       }
     }
-    load_conn(tile + stride);
+    if (tile + stride < ntiles) load_conn(tile + stride);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -636,16 +670,37 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
   }
 }
 
-// Face coefficients of an operator, one thread per element face: (sJ tau / 2, -sJ c_r / 2).
-template <typename T, int DIM, int TE>
-__global__ void k_face_geo(const T* __restrict__ tcg, const T* __restrict__ tau, int K, T* __restrict__ out) {
-  constexpr int NF = DIM + 1, NV = 8, NFG = 4, GROWS = NV + NFG * NF;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * NF; i += gridDim.x * blockDim.x) {
-    const int e = i / NF, f = i % NF;
-    const T* g = tcg + (size_t)(e / TE) * GROWS * TE + e % TE;
-    const T hs = T(0.5) * g[(NV + f) * TE];
-    st4(out + (size_t)i * 4, hs * tau[i], -hs * g[(NV + NF + f) * TE], -hs * g[(NV + 2 * NF + f) * TE],
-        -hs * g[(NV + 3 * NF + f) * TE]);
+// Neighbour records of one component, one thread per element face (ApplyArgs::nrec).
+__global__ void k_neighbour_records(const int* __restrict__ nbr, const uint32_t* __restrict__ fcode,
+                                    const uint8_t* __restrict__ bct, int K, int NF, uint32_t* __restrict__ out) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)K * NF; i += (size_t)gridDim.x * blockDim.x) {
+    const int n = nbr[i], f = (int)(i % NF);
+    if (n >= 0) {
+      const uint32_t c = (fcode[i / NF] >> (8 * f)) & 255u;  // its face | orientation << 2
+      out[i] = ((uint32_t)n * NF + (c & 3u)) << 3 | c >> 2;
+    } else {
+      out[i] = (uint32_t)i << 3 | (bct[-n - 1] == BC_DIRICHLET ? NREC_DIRICHLET : NREC_NATURAL);
+    }
+  }
+}
+
+// Face coefficients of an operator in both precisions, one thread per element face:
+// (sJ tau / 2, -sJ c_r / 2).
+template <typename T, int DIM>
+__device__ __forceinline__ void face_coeffs(const T* __restrict__ tcg, const T* __restrict__ tau, int i, T* __restrict__ out) {
+  constexpr int NF = DIM + 1, NV = 8, NFG = 4, GROWS = NV + NFG * NF, TE = 8 * Frag<T>::R;
+  const int e = i / NF, f = i % NF;
+  const T* g = tcg + (size_t)(e / TE) * GROWS * TE + e % TE;
+  const T hs = T(0.5) * g[(NV + f) * TE];
+  st4(out + (size_t)i * 4, hs * tau[i], -hs * g[(NV + NF + f) * TE], -hs * g[(NV + 2 * NF + f) * TE],
+      -hs * g[(NV + 3 * NF + f) * TE]);
+}
+template <int DIM>
+__global__ void k_face_geo(const double* tcg64, const double* tau64, double* out64, const float* tcg32,
+                           const float* tau32, float* out32, int K) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * (DIM + 1); i += gridDim.x * blockDim.x) {
+    face_coeffs<double, DIM>(tcg64, tau64, i, out64);
+    face_coeffs<float, DIM>(tcg32, tau32, i, out32);
   }
 }
 
@@ -697,7 +752,7 @@ constexpr size_t smem1(int w) {
 template <typename T, int DIM, int P>
 constexpr size_t smem2() {
   using X = Tc<T, DIM, P>;
-  return (size_t)X::N2 * sizeof(T) + Cfg<DIM, P>::NPERM * (X::TRP / 2) * sizeof(uint16_t);
+  return (size_t)X::N2 * sizeof(T) + 8 * (X::TRP / 2) * sizeof(uint16_t);
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -725,12 +780,12 @@ cudaError_t launch_passes(const ApplyArgs<T>& a, const T* blob, T* trace, int nt
   cudaError_t err = launch_pass(sipg_volume_kernel<T, DIM, P, WARPS, MINB>, a, blob, trace, WARPS,
                                 smem1<T, DIM, P>(WARPS), ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
-  return launch_pass(sipg_face_kernel<T, DIM, P, WARPS, MINB>, a, blob + Tc<T, DIM, P>::N1, (const T*)trace, WARPS,
+  return launch_pass(sipg_face_kernel<T, DIM, P, 8, 2>, a, blob + Tc<T, DIM, P>::N1, (const T*)trace, 8,
                      smem2<T, DIM, P>(), ntiles, num_sms, s);
 }
 
-// Launch shape: two CTAs of 8 warps per SM where their shared memory fits (128 registers
-// per thread), else (FP64 p = 4 in 3D) one of 12. A grid of min(tiles, resident CTAs) with
+// Launch shape: two CTAs of 8 warps per SM (128 registers per thread), for pass 1 one of 12
+// where two do not fit next to the operands (3D p = 4). A grid of min(tiles, resident CTAs) with
 // warp-major tiles spreads any number of tiles over all SMs: on a small mesh a CTA has one
 // tile and its other warps only help to copy the operands.
 template <typename T, int DIM, int P>
@@ -843,14 +898,24 @@ cudaError_t launch_tc_geom(int dim, const T* geof, int K, T* out, cudaStream_t s
   return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_face_geo(int dim, const T* tcg, const T* tau, int K, T* out, cudaStream_t s) {
-  constexpr int TE = 8 * Frag<T>::R;
+bool neighbour_records_fit(int dim, int K) { return (size_t)K * (dim + 1) <= (size_t)1 << 29; }
+
+cudaError_t launch_neighbour_records(int dim, const int* nbr, const uint32_t* fcode, const uint8_t* bct, int K,
+                                     uint32_t* out, cudaStream_t s) {
+  const int grid = (int)std::min<size_t>(((size_t)K * (dim + 1) + 255) / 256, 148 * 16);
+  if (grid == 0) return cudaSuccess;
+  k_neighbour_records<<<grid, 256, 0, s>>>(nbr, fcode, bct, K, dim + 1, out);
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_face_geo(int dim, const double* tcg64, const double* tau64, double* out64, const float* tcg32,
+                            const float* tau32, float* out32, int K, cudaStream_t s) {
   const size_t n = (size_t)K * (dim + 1);
   const int grid = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
   if (grid == 0) return cudaSuccess;
-  if (dim == 3) k_face_geo<T, 3, TE><<<grid, 256, 0, s>>>(tcg, tau, K, out);
-  else if (dim == 2) k_face_geo<T, 2, TE><<<grid, 256, 0, s>>>(tcg, tau, K, out);
+  if (dim == 3) k_face_geo<3><<<grid, 256, 0, s>>>(tcg64, tau64, out64, tcg32, tau32, out32, K);
+  else if (dim == 2) k_face_geo<2><<<grid, 256, 0, s>>>(tcg64, tau64, out64, tcg32, tau32, out32, K);
   else return cudaErrorInvalidValue;
   note_launch();
   return cudaGetLastError();
@@ -867,8 +932,6 @@ template cudaError_t launch_apply_tc<double>(int, int, const ApplyArgs<double>&,
                                              cudaStream_t);
 template void build_tc_consts<float>(int, int, const RefElement&, std::vector<double>&);
 template void build_tc_consts<double>(int, int, const RefElement&, std::vector<double>&);
-template cudaError_t launch_face_geo<float>(int, const float*, const float*, int, float*, cudaStream_t);
-template cudaError_t launch_face_geo<double>(int, const double*, const double*, int, double*, cudaStream_t);
 template size_t tc_geom_values<float>(int, int);
 template size_t tc_geom_values<double>(int, int);
 template cudaError_t launch_tc_geom<float>(int, const float*, int, float*, cudaStream_t);

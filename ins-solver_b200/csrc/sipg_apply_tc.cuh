@@ -20,10 +20,15 @@ cudaError_t launch_apply_tc(int dim, int order, const ApplyArgs<T>& a, const T* 
 size_t tc_trace_values(int dim, int order, int K);
 template <typename T>
 void build_tc_consts(int dim, int order, const RefElement& r, std::vector<double>& out);
-// Face coefficients of an operator (ApplyArgs::fgeo), K x NF x 4 values: sJ tau / 2 and
-// -sJ c_r / 2, from the mesh's geometry blocks and the operator's penalty.
-template <typename T>
-cudaError_t launch_face_geo(int dim, const T* tcg, const T* tau, int K, T* out, cudaStream_t s);
+// Neighbour records of an operator's component (ApplyArgs::nrec): 29 bits of element face,
+// a mesh with more has none and takes the CUDA-core apply.
+bool neighbour_records_fit(int dim, int K);
+cudaError_t launch_neighbour_records(int dim, const int* nbr, const uint32_t* fcode, const uint8_t* bct, int K,
+                                     uint32_t* out, cudaStream_t s);
+// Face coefficients of an operator (ApplyArgs::fgeo) in both precisions, K x NF x 4 values:
+// sJ tau / 2 and -sJ c_r / 2, from the mesh's geometry blocks and the operator's penalty.
+cudaError_t launch_face_geo(int dim, const double* tcg64, const double* tau64, double* out64, const float* tcg32,
+                            const float* tau32, float* out32, int K, cudaStream_t s);
 // Element and face geometry of the tensor-core apply (ApplyArgs::tcg), computed
 // once per mesh from the K x NG geometric factors: tc_geom_values<T>(dim, K)
 // values, one block per warp tile of elements (zero past K).
