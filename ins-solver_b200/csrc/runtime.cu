@@ -241,18 +241,38 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
   a.tcgen05 = kernel == 3;
   const bool tc_ok = (kernel == 0 || kernel >= 2) && nrec.p;
   if (tc_ok && ncomp > 1 && pin_elem < 0) {
-    // vector operator: one tensor-core scalar apply per component (its own boundary
-    // types; slip faces get no face terms there), then the slip faces' coupling terms
     const T* tcc = f64 ? (const T*)dref->tc64.p : (const T*)dref->tc32.p;
     DevBuf& tr = f64 ? trace64 : trace32;
-    if (!tr.p) tr = DevBuf(tc_trace_values(mesh->dim, order, mesh->K) * sizeof(T));
-    const size_t per = (size_t)mesh->K * Np;
+    const size_t one = tc_trace_values(mesh->dim, order, mesh->K) * sizeof(T), per = (size_t)mesh->K * Np;
+    if (!tr.p) {
+      try {
+        tr = DevBuf(one * ncomp);
+      } catch (const Error& e) {  // no room for every component's traces at once
+        if (e.status != SIPG_OUT_OF_MEMORY) throw;
+        cudaGetLastError();
+        tr = DevBuf(one);
+      }
+    }
+    // every component in one pair of launches, slip faces included; needs all components'
+    // traces and every row on a 16-byte boundary (kernel 3 has no such form)
+    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    if (kernel != 3 && tr.bytes >= one * ncomp && per * sizeof(T) % 16 == 0 && aligned(x) && aligned(y) &&
+        (beta == T(0) || aligned(a.c))) {
+      a.ncomp = 1;
+      a.nvec = ncomp;
+      a.slip = slip.as<uint8_t>();
+      SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, a, tcc, tr.as<T>(), num_sms(), s));
+      return;
+    }
+    // else one scalar apply per component (its own boundary types; slip faces get no face
+    // terms there), then the slip faces' coupling terms
     for (int comp = 0; comp < ncomp; ++comp) {
       ApplyArgs<T> ac = a;
       ac.ncomp = 1;
       ac.x = x + comp * per;
       ac.y = y + comp * per;
       ac.c = a.c + comp * per;
+      ac.bct = bct.as<uint8_t>() + (size_t)comp * mesh->Kb;
       ac.nrec = nrec.as<uint32_t>() + (size_t)comp * mesh->K * (mesh->dim + 1);
       SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, ac, tcc, tr.as<T>(), num_sms(), s));
     }
@@ -291,6 +311,9 @@ void sipg_op::refresh_bc() {
     SIPG_CUDA(launch_neighbour_records(mesh->dim, mesh->nbr.as<int>(), mesh->fcode.as<uint32_t>(),
                                        bct.as<uint8_t>() + (size_t)c * mesh->Kb, mesh->K,
                                        nrec.as<uint32_t>() + (size_t)c * mesh->K * (mesh->dim + 1), 0));
+  if (slip.p)
+    SIPG_CUDA(launch_slip_mask(mesh->dim, mesh->nbr.as<int>(), bct.as<uint8_t>(), mesh->K, ncomp, mesh->Kb,
+                               slip.as<uint8_t>(), 0));
   SIPG_CUDA(cudaStreamSynchronize(0));
 }
 
@@ -354,6 +377,7 @@ std::unique_ptr<sipg_op> create_op(sipg_mesh* m, int order, int ncomp) {
   std::vector<uint8_t> b(op->bct_host.size(), 0);
   if (!b.empty()) op->bct.upload(b.data(), b.size());
   if (neighbour_records_fit(m->dim, m->K)) op->nrec = DevBuf((size_t)ncomp * m->K * Nf * sizeof(uint32_t));
+  if (ncomp > 1) op->slip = DevBuf((size_t)m->K);
   op->refresh_bc();
   op->eb64 = apply_pick_eb(m->dim, order, ncomp, true);
   op->eb32 = apply_pick_eb(m->dim, order, ncomp, false);

@@ -101,6 +101,7 @@ struct sipg_op {
   sipg::DevBuf bct;           // ncomp x Kb uint8
   std::vector<int> bct_host;  // ncomp x Kb
   sipg::DevBuf nrec;          // neighbour records of the tensor-core apply, ncomp x K x Nf (ApplyArgs::nrec)
+  sipg::DevBuf slip;          // vector operators: slip faces per element (ApplyArgs::slip)
   int pin_elem = -1, pin_node = -1;
   double pin_scale = 1.0;
   int eb64 = 0, eb32 = 0;

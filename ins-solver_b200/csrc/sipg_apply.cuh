@@ -112,6 +112,8 @@ struct ApplyArgs {
   const uint32_t* nrec;   // tensor-core path: K x NF, neighbour record (nb NF + its face) << 3 | orientation;
                           // a boundary face's own record with NREC_DIRICHLET or NREC_NATURAL
   const T* fgeo;          // tensor-core path: face coefficients K x NF x 4 (launch_face_geo)
+  int nvec = 1;           // tensor-core path: components applied by one launch (x, y, c K x NP apart, nrec K x NF)
+  const uint8_t* slip = nullptr;  // nvec > 1: per element, bit f set where face f is a slip face
   int tcgen05 = 0;        // tensor-core path, FP32: tcgen05 kernels where the order has them (else mma.sync)
 };
 

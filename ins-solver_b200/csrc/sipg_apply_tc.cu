@@ -211,13 +211,12 @@ __device__ __forceinline__ void copy_blob(void* s, const void* g, int bytes) {
   cp_commit();
 }
 
-// sJ and c_r = n . grad r of face f (n the outward unit normal) from the geometric factors g.
+// sJ, c_r = n . grad r and the outward unit normal n of face f from the geometric factors g.
 __device__ __forceinline__ float inv_sqrt(float v) { return rsqrtf(v); }
 __device__ __forceinline__ double inv_sqrt(double v) { return 1.0 / sqrt(v); }
 
 template <typename T, int DIM>
-__device__ __forceinline__ void face_geom(const T* g, int f, T& sJ, T (&c)[3]) {
-  T n[3];
+__device__ __forceinline__ void face_geom(const T* g, int f, T& sJ, T (&c)[3], T (&n)[3]) {
   if (DIM == 3) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -328,7 +327,8 @@ __device__ __forceinline__ void mma_nodes(T (&c)[Frag<T>::R][2], const T (&a)[Fr
 }
 
 // ---------------------------------------------------------------- pass 1
-template <typename T, int DIM, int P, int WARPS, int MINB>
+// VEC: a.nvec components per launch.
+template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
                                                                        T* __restrict__ trace) {
   using X = Tc<T, DIM, P>;
@@ -340,11 +340,12 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const bool has_mm = a.mm_mode != MM_NONE;
   T* W = B + X::N1 + warp * X::W1;
-  const int ntiles = (a.K + TE - 1) / TE;
+  const int ntiles = (a.K + TE - 1) / TE, nvt = VEC ? ntiles * a.nvec : ntiles;  // component-major tiles
   const int stride = gridDim.x * WARPS;
+  const size_t per = (size_t)a.K * NP;  // values per component
   // warp-major tile order: the last, partial round of tiles is spread over all
   // CTAs (SMs) instead of filling the first ones
-  int tile = warp * gridDim.x + blockIdx.x;
+  int vt = warp * gridDim.x + blockIdx.x;
   pdl_trigger();
   copy_blob(B, blob, (has_mm ? X::N1 : X::BM) * (int)sizeof(T));
   // record gather: this lane's element of the tile and the volume nodes of its faces, 4 per word
@@ -363,10 +364,15 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
     }
   pdl_wait();  // x, factor, c, y and the trace buffer belong to the preceding kernels
   T u[NT][R][2];
-  if (tile < ntiles) load_nodes<T, DIM, P>(a.x, tile * TE, min(TE, a.K - tile * TE), u, g, t);
+  auto load_x = [&](int v) {
+    const int comp = VEC ? v / ntiles : 0, e0 = (v - comp * ntiles) * TE;
+    load_nodes<T, DIM, P>(a.x + comp * per, e0, min(TE, a.K - e0), u, g, t);
+  };
+  if (vt < nvt) load_x(vt);
   cp_wait_all();
   __syncthreads();
-  for (; tile < ntiles; tile += stride) {
+  for (; vt < nvt; vt += stride) {
+    const int comp = VEC ? vt / ntiles : 0, tile = vt - comp * ntiles;
     const int e0 = tile * TE;
     const int ne = min(TE, a.K - e0);
     const bool pin_here = a.pin_elem >= e0 && a.pin_elem < e0 + ne;
@@ -465,8 +471,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
         for (int nt = 0; nt < NT; ++nt) mma_nodes<T, DIM, P>(y[nt], mx, ldb(B + X::BM, kb * NT + nt, lane), kb);
       }
     }
-    const int next = tile + stride;
-    if (X::PREFETCH && next < ntiles) load_nodes<T, DIM, P>(a.x, next * TE, min(TE, a.K - next * TE), u, g, t);
+    if (X::PREFETCH && vt + stride < nvt) load_x(vt + stride);
 #pragma unroll
     for (int r = 0; r < DIM; ++r)
 #pragma unroll
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
           mma_nodes<T, DIM, P>(y[nt], w[r][kb], ldb(B + X::BS, (r * NT + kb) * NT + nt, lane), kb);
     // pinned row, alpha / beta, store
     T yold[NT][R][2];
-    if (a.beta != T(0)) load_nodes<T, DIM, P>(a.c, e0, ne, yold, g, t);
+    if (a.beta != T(0)) load_nodes<T, DIM, P>(a.c + comp * per, e0, ne, yold, g, t);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -490,7 +495,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
           if (a.beta != T(0)) v += a.beta * yold[nt][ri][ci];
           y[nt][ri][ci] = v;
         }
-    store_nodes<T, DIM, P>(a.y, e0, ne, y, g, t);
+    store_nodes<T, DIM, P>(a.y + comp * per, e0, ne, y, g, t);
     // trace records: gathered by (element, face), then written out as one contiguous piece
     __syncwarp();
     T ru[FPL][TRP], rq[FPL][TRP];
@@ -522,19 +527,50 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
       using V4 = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
       constexpr int PPE = NF * TR / X::VPC, FULL = TE * PPE;  // pieces per element, per tile
       const int n = ne * PPE;
-      V4* dst = reinterpret_cast<V4*>(trace + (size_t)e0 * NF * TR);
+      V4* dst = reinterpret_cast<V4*>(trace + ((size_t)comp * a.K + e0) * NF * TR);
 #pragma unroll
       for (int i0 = 0; i0 < FULL; i0 += 32) {
         const int i = i0 + lane;
         if (i < n) dst[i] = reinterpret_cast<const V4*>(W)[i + (X::RS - PPE) * (i / PPE)];
       }
     }
-    if (!X::PREFETCH && next < ntiles) load_nodes<T, DIM, P>(a.x, next * TE, min(TE, a.K - next * TE), u, g, t);
+    if (!X::PREFETCH && vt + stride < nvt) load_x(vt + stride);
   }
 }
 
 // ---------------------------------------------------------------- pass 2
-template <typename T, int DIM, int P, int WARPS, int MINB>
+// Slip face of the vector operator, folded in here (3 instead of 7 launches per apply; at
+// p = 3, 16^3 x 6 in FP64 163 -> 58 us per apply with the components batched, where a kernel
+// over the boundary elements alone took 45 us): as vmf_3d_mult_avg_jump.h:9-41, the exterior state mirrors the
+// interior one, u+ = u - 2 n (n . u) and likewise the fluxes q, so that the jump and the average
+// carry the normal components 2 n_c (n . u) and n_c (n . q) alone. `at`: the node pair's place in
+// the element's records; um: component comp's own (u, q) pairs.
+template <typename T, int DIM, int P>
+__device__ __forceinline__ void slip_exterior(const ApplyArgs<T>& a, const T* trace, int e, int f, int at, int comp,
+                                           const T (&um)[4], typename Frag<T>::V2& p0, typename Frag<T>::V2& p1) {
+  using X = Tc<T, DIM, P>;
+  constexpr int NG = Cfg<DIM, P>::NG;
+  T gg[NG], sJ, c[3], n[3];
+#pragma unroll
+  for (int i = 0; i < NG; ++i) gg[i] = a.geof[(size_t)e * NG + i];
+  face_geom<T, DIM>(gg, f, sJ, c, n);
+  T s[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) {
+    T v[4];
+    ld4(trace + ((size_t)k * a.K + e) * X::NF * X::TR + at, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] += n[k] * v[i];
+  }
+  const T n2 = T(2) * (comp == 0 ? n[0] : comp == 1 ? n[1] : n[2]);
+  p0.x = um[0] - n2 * s[0];
+  p0.y = um[1] - n2 * s[1];
+  p1.x = um[2] - n2 * s[2];
+  p1.y = um[3] - n2 * s[3];
+}
+
+// VEC: a.nvec components per launch.
+template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
                                                                      const T* __restrict__ trace) {
   using X = Tc<T, DIM, P>;
@@ -548,9 +584,9 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
   T* B = reinterpret_cast<T*>(smem_raw);
   uint16_t* ptab = reinterpret_cast<uint16_t*>(B + X::N2);  // [orientation][pair]: record positions of a pair's nodes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int ntiles = (a.K + TE - 1) / TE;
+  const int ntiles = (a.K + TE - 1) / TE, nvt = VEC ? ntiles * a.nvec : ntiles;
   const int stride = gridDim.x * WARPS;
-  int tile = warp * gridDim.x + blockIdx.x;  // warp-major, as in pass 1
+  int vt = warp * gridDim.x + blockIdx.x;  // warp-major, as in pass 1
   pdl_trigger();
   copy_blob(B, blob, X::N2 * (int)sizeof(T));
   for (int i = threadIdx.x; i < 8 * HP; i += blockDim.x) {
@@ -575,36 +611,40 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
   // connectivity of the lane's elements (set-up data): neighbour record << 3 | code.
   // Rows past the tile's end repeat the mesh's last element: they are computed and not stored.
   uint32_t nb[R][NF];
-  auto load_conn = [&](int tl) {
+  auto load_conn = [&](int v) {
+    const int comp = VEC ? v / ntiles : 0;
 #pragma unroll
     for (int ri = 0; ri < R; ++ri) {
-      const int e = min(tl * TE + g + 8 * ri, a.K - 1);
+      const size_t e = (size_t)comp * a.K + min((v - comp * ntiles) * TE + g + 8 * ri, a.K - 1);
       if (NF == 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(a.nrec + (size_t)e * NF);
+        const uint4 q = *reinterpret_cast<const uint4*>(a.nrec + e * NF);
         nb[ri][0] = q.x; nb[ri][1] = q.y; nb[ri][2] = q.z; nb[ri][NF - 1] = q.w;
       } else {
 #pragma unroll
-        for (int f = 0; f < NF; ++f) nb[ri][f] = a.nrec[(size_t)e * NF + f];
+        for (int f = 0; f < NF; ++f) nb[ri][f] = a.nrec[e * NF + f];
       }
     }
   };
-  if (tile < ntiles) load_conn(tile);
+  if (vt < nvt) load_conn(vt);
   pdl_wait();
   cp_wait_all();
   __syncthreads();
-  for (; tile < ntiles; tile += stride) {
-    const int e0 = tile * TE;
+  for (; vt < nvt; vt += stride) {
+    const int comp = VEC ? vt / ntiles : 0;
+    const int e0 = (vt - comp * ntiles) * TE;
     const int ne = min(TE, a.K - e0);
+    const T* tr = trace + (size_t)comp * a.K * NF * TR;
+    T* yb = a.y + (size_t)comp * a.K * NP;
     const T *own[R], *fg_row[R], *f_row[R];
 #pragma unroll
     for (int ri = 0; ri < R; ++ri) {
       const int e = min(e0 + g + 8 * ri, a.K - 1);
-      own[ri] = trace + (size_t)e * NF * TR + 4 * t;
+      own[ri] = tr + (size_t)e * NF * TR + 4 * t;
       fg_row[ri] = a.fgeo + (size_t)e * NF * 4;
       f_row[ri] = a.factor + (size_t)e * NP;
     }
     T yold[NT][R][2];
-    load_nodes<T, DIM, P>(a.y, e0, ne, yold, g, t);
+    load_nodes<T, DIM, P>(yb, e0, ne, yold, g, t);
     T y[NT][R][2];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
@@ -624,7 +664,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
         const int sg = (int)(n & 7u);
         const bool pad = X::KF % 8 != 0 && f >= NF;  // no face: its operand rows are zero, its values finite
         const unsigned kk = ptab[sg * HP + ((8 * fb + 2 * t - TRP * f) >> 1)];
-        const T* rec = trace + (size_t)(n >> 3) * TR;
+        const T* rec = tr + (size_t)(n >> 3) * TR;
         T um[4] = {T(0), T(0), T(0), T(0)}, fg[4] = {T(0), T(0), T(0), T(0)};
         V2 p0{T(0), T(0)}, p1{T(0), T(0)};
         T f0 = T(1), f1 = T(1);
@@ -640,6 +680,10 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
         }
         // exterior values: the neighbour's; a boundary face has its own, negated on Dirichlet faces
         const T sgn = sg == NREC_DIRICHLET ? T(-1) : T(1);
+        if (VEC && sg == NREC_NATURAL && !pad) {
+          const int e = min(e0 + g + 8 * ri, a.K - 1);
+          if (a.slip[e] >> f & 1) slip_exterior<T, DIM, P>(a, trace, e, f, 16 * fb + 4 * t, comp, um, p0, p1);
+        }
         const T s0 = um[0] - sgn * p0.x, s1 = um[2] - sgn * p1.x;
         fu[ri][0] = fg[0] * s0 - (um[1] - sgn * p0.y);
         fu[ri][1] = fg[0] * s1 - (um[3] - sgn * p1.y);
@@ -656,7 +700,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
         for (int r = 0; r < DIM; ++r) F::mma(y[nt], sv[r], ldb(B + X::BQ, (r * FT + fb) * NT + nt, lane));
       }
     }
-    if (tile + stride < ntiles) load_conn(tile + stride);
+    if (vt + stride < nvt) load_conn(vt + stride);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -666,7 +710,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
           const bool pinned = e0 + g + 8 * ri == a.pin_elem && frag_node<T, DIM, P>(nt, ci, t) == a.pin_node;
           y[nt][ri][ci] = yold[nt][ri][ci] + (pinned ? T(0) : a.alpha * y[nt][ri][ci]);
         }
-    store_nodes<T, DIM, P>(a.y, e0, ne, y, g, t);
+    store_nodes<T, DIM, P>(yb, e0, ne, y, g, t);
   }
 }
 
@@ -681,6 +725,22 @@ __global__ void k_neighbour_records(const int* __restrict__ nbr, const uint32_t*
     } else {
       out[i] = (uint32_t)i << 3 | (bct[-n - 1] == BC_DIRICHLET ? NREC_DIRICHLET : NREC_NATURAL);
     }
+  }
+}
+
+// Slip faces of a vector operator, one thread per element: bit f set where every component's
+// type of boundary face f is slip.
+__global__ void k_slip_mask(const int* __restrict__ nbr, const uint8_t* __restrict__ bct, int K, int NF, int ncomp,
+                            int Kb, uint8_t* __restrict__ out) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K; e += gridDim.x * blockDim.x) {
+    unsigned m = 0;
+    for (int f = 0; f < NF; ++f) {
+      const int n = nbr[(size_t)e * NF + f];
+      bool s = n < 0;
+      for (int c = 0; s && c < ncomp; ++c) s = bct[(size_t)c * Kb + (-n - 1)] == BC_SLIP;
+      m |= (unsigned)s << f;
+    }
+    out[e] = (uint8_t)m;
   }
 }
 
@@ -729,8 +789,8 @@ __global__ void k_tc_geom(const T* __restrict__ geof, int K, T* __restrict__ out
         }
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        T sJ, c[3];
-        face_geom<T, DIM>(g, f, sJ, c);
+        T sJ, c[3], n[3];
+        face_geom<T, DIM>(g, f, sJ, c, n);
         v[NV + f] = sJ;
 #pragma unroll
         for (int r = 0; r < 3; ++r) v[NV + (1 + r) * NF + f] = c[r];
@@ -773,14 +833,14 @@ cudaError_t launch_pass(Kern k, const ApplyArgs<T>& a, const T* blob, TT* trace,
   return cudaSuccess;
 }
 
-template <typename T, int DIM, int P, int WARPS, int MINB>
+template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC>
 cudaError_t launch_passes(const ApplyArgs<T>& a, const T* blob, T* trace, int ntiles, int num_sms, cudaStream_t s) {
   static_assert(smem1<T, DIM, P>(WARPS) <= (size_t)kSmemBudget && smem2<T, DIM, P>() <= (size_t)kSmemBudget,
                 "the operands do not fit");
-  cudaError_t err = launch_pass(sipg_volume_kernel<T, DIM, P, WARPS, MINB>, a, blob, trace, WARPS,
+  cudaError_t err = launch_pass(sipg_volume_kernel<T, DIM, P, WARPS, MINB, VEC>, a, blob, trace, WARPS,
                                 smem1<T, DIM, P>(WARPS), ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
-  return launch_pass(sipg_face_kernel<T, DIM, P, 8, 2>, a, blob + Tc<T, DIM, P>::N1, (const T*)trace, 8,
+  return launch_pass(sipg_face_kernel<T, DIM, P, 8, 2, VEC>, a, blob + Tc<T, DIM, P>::N1, (const T*)trace, 8,
                      smem2<T, DIM, P>(), ntiles, num_sms, s);
 }
 
@@ -799,9 +859,11 @@ cudaError_t launch_tc_t(const ApplyArgs<T>& a, const T* blob, T* trace, int num_
   if (!aligned16(a.x) || !aligned16(a.y) || !aligned16(trace) || (a.factor && !aligned16(a.factor)) ||
       (a.beta != T(0) && !aligned16(a.c)))
     return launch_apply<T>(DIM, P, a, num_sms, s);
-  const int ntiles = (a.K + X::TE - 1) / X::TE;
+  const int ntiles = (a.K + X::TE - 1) / X::TE * a.nvec;
   constexpr bool two = 2 * (smem1<T, DIM, P>(8) + 1024) <= (size_t)kSmemBudget + 1024;
-  const cudaError_t err = launch_passes<T, DIM, P, two ? 8 : 12, two ? 2 : 1>(a, blob, trace, ntiles, num_sms, s);
+  constexpr int W = two ? 8 : 12, B = two ? 2 : 1;
+  const cudaError_t err = a.nvec > 1 ? launch_passes<T, DIM, P, W, B, true>(a, blob, trace, ntiles, num_sms, s)
+                                     : launch_passes<T, DIM, P, W, B, false>(a, blob, trace, ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
   return cudaGetLastError();
 }
@@ -905,6 +967,15 @@ cudaError_t launch_neighbour_records(int dim, const int* nbr, const uint32_t* fc
   const int grid = (int)std::min<size_t>(((size_t)K * (dim + 1) + 255) / 256, 148 * 16);
   if (grid == 0) return cudaSuccess;
   k_neighbour_records<<<grid, 256, 0, s>>>(nbr, fcode, bct, K, dim + 1, out);
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_slip_mask(int dim, const int* nbr, const uint8_t* bct, int K, int ncomp, int Kb, uint8_t* out,
+                             cudaStream_t s) {
+  const int grid = std::min((K + 255) / 256, 148 * 16);
+  if (grid == 0) return cudaSuccess;
+  k_slip_mask<<<grid, 256, 0, s>>>(nbr, bct, K, dim + 1, ncomp, Kb, out);
   note_launch();
   return cudaGetLastError();
 }

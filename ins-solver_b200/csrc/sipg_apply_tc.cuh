@@ -25,6 +25,9 @@ void build_tc_consts(int dim, int order, const RefElement& r, std::vector<double
 bool neighbour_records_fit(int dim, int K);
 cudaError_t launch_neighbour_records(int dim, const int* nbr, const uint32_t* fcode, const uint8_t* bct, int K,
                                      uint32_t* out, cudaStream_t s);
+// Slip faces of a vector operator (ApplyArgs::slip).
+cudaError_t launch_slip_mask(int dim, const int* nbr, const uint8_t* bct, int K, int ncomp, int Kb, uint8_t* out,
+                             cudaStream_t s);
 // Face coefficients of an operator (ApplyArgs::fgeo) in both precisions, K x NF x 4 values:
 // sJ tau / 2 and -sJ c_r / 2, from the mesh's geometry blocks and the operator's penalty.
 cudaError_t launch_face_geo(int dim, const double* tcg64, const double* tau64, double* out64, const float* tcg32,

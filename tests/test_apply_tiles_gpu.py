@@ -29,3 +29,17 @@ def test_tile_edges_pin_and_in_place(dim, n, order):
         assert rel_err(y.astype(np.float64), ref) < tol
         op.apply_device(prec, xd.p, xd.p)  # every tile reads its own rows before it writes them
         assert np.array_equal(xd.get(), y)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("dim,n", [(2, 5), (2, 7), (3, 1), (3, 3)])
+def test_vector_operator_with_slip_faces(dim, n, order):
+    """All components in one launch, or one after the other where a component's rows do not
+    start on 16 bytes (2D p = 1, n = 5 and 7 in FP32: 150 and 294 values)."""
+    mesh, t, e, om, x, f, m, bct = random_case(dim, n, order, dim, seed=3 * order + dim, slip=True, mm=True)
+    op = make_op(mesh, order, dim, f, m, bct=bct)
+    ref = O.mult(om, x, bct, f, m)
+    for prec, dtype, tol in ((sipg.FP64, np.float64, TOL_FP64), (sipg.FP32, np.float32, TOL_TF32)):
+        xd, yd = DevArray(x.astype(dtype)), DevArray(np.full(x.shape, 7.0, dtype))
+        op.apply_device(prec, xd.p, yd.p)
+        assert rel_err(yd.get().astype(np.float64), ref) < tol
