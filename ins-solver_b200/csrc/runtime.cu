@@ -205,12 +205,8 @@ void sipg_mesh::ensure_device() {
 }
 
 template <typename T>
-void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* c) const {
+ApplyArgs<T> sipg_op::apply_args(const T* x, T* y) const {
   constexpr bool f64 = std::is_same<T, double>::value;
-  if (oi) {  // over-integrated factor: the assembled element blocks
-    bsr_apply<T>(*oi_blocks, x, y, alpha, beta, s, c);
-    return;
-  }
   ApplyArgs<T> a;
   a.consts = f64 ? (const T*)dref->c64.p : (const T*)dref->c32.p;
   a.itab = dref->itab.as<int8_t>();
@@ -232,32 +228,72 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
   a.pin_node = pin_node;
   a.pin_scale = (T)pin_scale;
   a.eb = f64 ? eb64 : eb32;
-  a.alpha = alpha;
-  a.beta = beta;
-  a.c = c ? c : y;
+  a.alpha = T(1);
+  a.beta = T(0);
+  a.c = y;
   a.tcg = f64 ? (const T*)mesh->tcg64.p : (const T*)mesh->tcg32.p;
   a.nrec = nrec.as<uint32_t>();
   a.fgeo = f64 ? (const T*)fgeo64.p : (const T*)fgeo32.p;
   a.tcgen05 = kernel == 3;
+  return a;
+}
+
+template <typename T>
+bool sipg_op::one_launch() const {
+  if (oi || kernel == 1 || !nrec.p || (ncomp > 1 && (pin_elem >= 0 || kernel == 3))) return false;
+  DevBuf& tr = std::is_same<T, double>::value ? trace64 : trace32;
+  const size_t one = tc_trace_values(mesh->dim, order, mesh->K) * sizeof(T);
+  if (!tr.p) {
+    try {
+      tr = DevBuf(one * ncomp);
+    } catch (const Error& e) {  // no room for every component's traces at once
+      if (ncomp == 1 || e.status != SIPG_OUT_OF_MEMORY) throw;
+      cudaGetLastError();
+      tr = DevBuf(one);
+    }
+  }
+  // a vector operator needs all components' traces and every row on a 16-byte boundary
+  return ncomp == 1 || (tr.bytes >= one * ncomp && (size_t)mesh->K * Np * sizeof(T) % 16 == 0);
+}
+
+void sipg_op::apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden,
+                              double* partial, unsigned* counter, double* dot_out, cudaStream_t s) const {
+  ApplyArgs<double> a = apply_args<double>(p, y);
+  if (ncomp > 1) {
+    a.ncomp = 1;
+    a.nvec = ncomp;
+    a.slip = slip.as<uint8_t>();
+  }
+  a.pz = z;
+  a.scal = scal;
+  a.bnum = bnum;
+  a.bden = bden;
+  a.dot_partial = partial;
+  a.dot_counter = counter;
+  a.dot_out = dot_out;
+  SIPG_CUDA(launch_apply_tc<double>(mesh->dim, order, a, dref->tc64.as<double>(), trace64.as<double>(), num_sms(), s));
+}
+
+template <typename T>
+void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* c) const {
+  constexpr bool f64 = std::is_same<T, double>::value;
+  if (oi) {  // over-integrated factor: the assembled element blocks
+    bsr_apply<T>(*oi_blocks, x, y, alpha, beta, s, c);
+    return;
+  }
+  ApplyArgs<T> a = apply_args<T>(x, y);
+  a.alpha = alpha;
+  a.beta = beta;
+  a.c = c ? c : y;
   const bool tc_ok = (kernel == 0 || kernel >= 2) && nrec.p;
   if (tc_ok && ncomp > 1 && pin_elem < 0) {
     const T* tcc = f64 ? (const T*)dref->tc64.p : (const T*)dref->tc32.p;
-    DevBuf& tr = f64 ? trace64 : trace32;
-    const size_t one = tc_trace_values(mesh->dim, order, mesh->K) * sizeof(T), per = (size_t)mesh->K * Np;
-    if (!tr.p) {
-      try {
-        tr = DevBuf(one * ncomp);
-      } catch (const Error& e) {  // no room for every component's traces at once
-        if (e.status != SIPG_OUT_OF_MEMORY) throw;
-        cudaGetLastError();
-        tr = DevBuf(one);
-      }
-    }
-    // every component in one pair of launches, slip faces included; needs all components'
-    // traces and every row on a 16-byte boundary (kernel 3 has no such form)
+    const bool batch = one_launch<T>();
+    const DevBuf& tr = f64 ? trace64 : trace32;
+    const size_t per = (size_t)mesh->K * Np;
+    // every component in one pair of launches, slip faces included
     auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (kernel != 3 && tr.bytes >= one * ncomp && per * sizeof(T) % 16 == 0 && aligned(x) && aligned(y) &&
-        (beta == T(0) || aligned(a.c))) {
+    if (batch && aligned(x) && aligned(y) && (beta == T(0) || aligned(a.c))) {
       a.ncomp = 1;
       a.nvec = ncomp;
       a.slip = slip.as<uint8_t>();
@@ -289,6 +325,8 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
   }
   SIPG_CUDA(launch_apply<T>(mesh->dim, order, a, num_sms(), s));
 }
+template bool sipg_op::one_launch<double>() const;
+template bool sipg_op::one_launch<float>() const;
 template void sipg_op::apply<double>(const double*, double*, cudaStream_t, double, double, const double*) const;
 template void sipg_op::apply<float>(const float*, float*, cudaStream_t, float, float, const float*) const;
 

@@ -118,6 +118,17 @@ struct sipg_op {
   template <typename T>
   // y = alpha A x + beta c, c = y when null (beta == 0: c is not read)
   void apply(const T* x, T* y, cudaStream_t s, T alpha = T(1), T beta = T(0), const T* c = nullptr) const;
+  // Whether a call on 16-byte aligned vectors runs as one pair of tensor-core launches
+  // (allocates their trace scratch).
+  template <typename T>
+  bool one_launch() const;
+  // One conjugate-gradient direction step: p <- z + (scal[bnum] / scal[bden]) p in place,
+  // y = A p, dot_out = p . y. Needs one_launch<double>() and aligned vectors; partial: a value
+  // per CTA (at most two per SM), counter zero.
+  void apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden, double* partial,
+                       unsigned* counter, double* dot_out, cudaStream_t s) const;
+  template <typename T>
+  sipg::ApplyArgs<T> apply_args(const T* x, T* y) const;
   void refresh_tau(cudaStream_t s);
   void refresh_bc();  // neighbour records after bct changed (synchronous)
   sipg::BlockArgs block_args(int mode, int ref_volume, double* out, bool with_pin) const;

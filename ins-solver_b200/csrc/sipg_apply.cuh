@@ -114,6 +114,14 @@ struct ApplyArgs {
   const T* fgeo;          // tensor-core path: face coefficients K x NF x 4 (launch_face_geo)
   int nvec = 1;           // tensor-core path: components applied by one launch (x, y, c K x NP apart, nrec K x NF)
   const uint8_t* slip = nullptr;  // nvec > 1: per element, bit f set where face f is a slip face
+  // tensor-core path, FP64, inside a conjugate-gradient iteration (pz not null): x <- pz +
+  // (scal[bnum] / scal[bden]) x is formed and stored in place first, and dot_out = x . y
+  // (partial: one value per CTA; counter zero before and after)
+  const T* pz = nullptr;
+  const double* scal = nullptr;
+  int bnum = 0, bden = 0;
+  double *dot_partial = nullptr, *dot_out = nullptr;
+  unsigned* dot_counter = nullptr;
   int tcgen05 = 0;        // tensor-core path, FP32: tcgen05 kernels where the order has them (else mma.sync)
 };
 

@@ -47,6 +47,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <type_traits>
 
@@ -327,8 +328,8 @@ __device__ __forceinline__ void mma_nodes(T (&c)[Frag<T>::R][2], const T (&a)[Fr
 }
 
 // ---------------------------------------------------------------- pass 1
-// VEC: a.nvec components per launch.
-template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC>
+// VEC: a.nvec components per launch. CG: the step's direction update and dot product ride along.
+template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC, bool CG>
 __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
                                                                        T* __restrict__ trace) {
   using X = Tc<T, DIM, P>;
@@ -364,9 +365,22 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
     }
   pdl_wait();  // x, factor, c, y and the trace buffer belong to the preceding kernels
   T u[NT][R][2];
+  T beta = T(0);
+  if (CG) beta = (T)(a.scal[a.bnum] / a.scal[a.bden]);
   auto load_x = [&](int v) {
-    const int comp = VEC ? v / ntiles : 0, e0 = (v - comp * ntiles) * TE;
-    load_nodes<T, DIM, P>(a.x + comp * per, e0, min(TE, a.K - e0), u, g, t);
+    const int comp = VEC ? v / ntiles : 0, e0 = (v - comp * ntiles) * TE, ne = min(TE, a.K - e0);
+    load_nodes<T, DIM, P>(a.x + comp * per, e0, ne, u, g, t);
+    if (CG) {
+      T z[NT][R][2];
+      load_nodes<T, DIM, P>(a.pz + comp * per, e0, ne, z, g, t);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri)
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci) u[nt][ri][ci] = z[nt][ri][ci] + beta * u[nt][ri][ci];
+      store_nodes<T, DIM, P>(const_cast<T*>(a.x) + comp * per, e0, ne, u, g, t);
+    }
   };
   if (vt < nvt) load_x(vt);
   cp_wait_all();
@@ -539,7 +553,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
 }
 
 // ---------------------------------------------------------------- pass 2
-// Slip face of the vector operator, folded in here (3 instead of 7 launches per apply; at
+// Slip face of the vector operator, folded in here (2 instead of 7 launches per apply; at
 // p = 3, 16^3 x 6 in FP64 163 -> 58 us per apply with the components batched, where a kernel
 // over the boundary elements alone took 45 us): as vmf_3d_mult_avg_jump.h:9-41, the exterior state mirrors the
 // interior one, u+ = u - 2 n (n . u) and likewise the fluxes q, so that the jump and the average
@@ -569,8 +583,8 @@ __device__ __forceinline__ void slip_exterior(const ApplyArgs<T>& a, const T* tr
   p1.y = um[3] - n2 * s[3];
 }
 
-// VEC: a.nvec components per launch.
-template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC>
+// VEC: a.nvec components per launch. CG: the step's direction update and dot product ride along.
+template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC, bool CG>
 __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T> a, const T* __restrict__ blob,
                                                                      const T* __restrict__ trace) {
   using X = Tc<T, DIM, P>;
@@ -626,6 +640,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
     }
   };
   if (vt < nvt) load_conn(vt);
+  double dot = 0.0;  // CG: this lane's part of x . y
   pdl_wait();
   cp_wait_all();
   __syncthreads();
@@ -711,6 +726,50 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
           y[nt][ri][ci] = yold[nt][ri][ci] + (pinned ? T(0) : a.alpha * y[nt][ri][ci]);
         }
     store_nodes<T, DIM, P>(yb, e0, ne, y, g, t);
+    if (CG) {
+      T x[NT][R][2];  // zero past the tile's elements and nodes, where y is not
+      load_nodes<T, DIM, P>(a.x + (size_t)comp * a.K * NP, e0, ne, x, g, t);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ri = 0; ri < R; ++ri)
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci)
+            if (g + 8 * ri < ne) dot += (double)x[nt][ri][ci] * (double)y[nt][ri][ci];
+    }
+  }
+  if (CG) {
+    // two-stage sum in a fixed order: warps, then the last CTA over the CTAs' partials
+    __shared__ double sh[WARPS];
+    __shared__ bool last;
+    auto cta_sum = [&](double v) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      __syncthreads();
+      if (lane == 0) sh[warp] = v;
+      __syncthreads();
+      double s = 0.0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) s += sh[w];
+      return s;
+    };
+    dot = cta_sum(dot);
+    if (threadIdx.x == 0) {
+      a.dot_partial[blockIdx.x] = dot;
+      __threadfence();
+      last = atomicAdd(a.dot_counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      double v = 0.0;
+      for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) v += ((volatile double*)a.dot_partial)[b];
+      v = cta_sum(v);
+      if (threadIdx.x == 0) {
+        *a.dot_out = v;
+        *a.dot_counter = 0u;
+      }
+    }
   }
 }
 
@@ -817,30 +876,50 @@ constexpr size_t smem2() {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <typename Kern, typename T, typename TT>
-cudaError_t launch_pass(Kern k, const ApplyArgs<T>& a, const T* blob, TT* trace, int warps, size_t bytes, int ntiles,
-                        int num_sms, cudaStream_t s) {
-  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+// The kernel's opt-in to its shared memory and its resident CTAs per SM, once per device (they
+// take the host about as long as the launch itself).
+template <auto K>
+cudaError_t kernel_setup(int warps, size_t bytes, int& per_sm) {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> known[kMaxDevices];
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
+  per_sm = dev < kMaxDevices ? known[dev].load(std::memory_order_acquire) : 0;
+  if (per_sm > 0) return cudaSuccess;
+  err = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err != cudaSuccess) return err;
+  int n = 0;
+  err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K, warps * 32, bytes);
+  if (err != cudaSuccess) return err;
+  per_sm = std::max(n, 1);
+  if (dev < kMaxDevices) known[dev].store(per_sm, std::memory_order_release);
+  return cudaSuccess;
+}
+
+template <auto K, typename T, typename TT>
+cudaError_t launch_pass(const ApplyArgs<T>& a, const T* blob, TT* trace, int warps, size_t bytes, int ntiles,
+                        int num_sms, cudaStream_t s) {
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, warps * 32, bytes);
-  const int grid = std::min(ntiles, num_sms * std::max(per_sm, 1));
+  cudaError_t err = kernel_setup<K>(warps, bytes, per_sm);
+  if (err != cudaSuccess) return err;
+  const int grid = std::min(ntiles, num_sms * per_sm);
   if (grid > 0) {
-    err = pdl_launch(k, dim3(grid), dim3(warps * 32), bytes, s, a, blob, trace);
+    err = pdl_launch(K, dim3(grid), dim3(warps * 32), bytes, s, a, blob, trace);
     if (err != cudaSuccess) return err;
     note_launch();
   }
   return cudaSuccess;
 }
 
-template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC>
+template <typename T, int DIM, int P, int WARPS, int MINB, bool VEC, bool CG>
 cudaError_t launch_passes(const ApplyArgs<T>& a, const T* blob, T* trace, int ntiles, int num_sms, cudaStream_t s) {
   static_assert(smem1<T, DIM, P>(WARPS) <= (size_t)kSmemBudget && smem2<T, DIM, P>() <= (size_t)kSmemBudget,
                 "the operands do not fit");
-  cudaError_t err = launch_pass(sipg_volume_kernel<T, DIM, P, WARPS, MINB, VEC>, a, blob, trace, WARPS,
+  cudaError_t err = launch_pass<sipg_volume_kernel<T, DIM, P, WARPS, MINB, VEC, CG>>(a, blob, trace, WARPS,
                                 smem1<T, DIM, P>(WARPS), ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
-  return launch_pass(sipg_face_kernel<T, DIM, P, 8, 2, VEC>, a, blob + Tc<T, DIM, P>::N1, (const T*)trace, 8,
+  return launch_pass<sipg_face_kernel<T, DIM, P, 8, 2, VEC, CG>>(a, blob + Tc<T, DIM, P>::N1, (const T*)trace, 8,
                      smem2<T, DIM, P>(), ntiles, num_sms, s);
 }
 
@@ -862,8 +941,16 @@ cudaError_t launch_tc_t(const ApplyArgs<T>& a, const T* blob, T* trace, int num_
   const int ntiles = (a.K + X::TE - 1) / X::TE * a.nvec;
   constexpr bool two = 2 * (smem1<T, DIM, P>(8) + 1024) <= (size_t)kSmemBudget + 1024;
   constexpr int W = two ? 8 : 12, B = two ? 2 : 1;
-  const cudaError_t err = a.nvec > 1 ? launch_passes<T, DIM, P, W, B, true>(a, blob, trace, ntiles, num_sms, s)
-                                     : launch_passes<T, DIM, P, W, B, false>(a, blob, trace, ntiles, num_sms, s);
+  cudaError_t err;
+  if constexpr (std::is_same<T, double>::value) {
+    if (a.pz) {
+      err = a.nvec > 1 ? launch_passes<T, DIM, P, W, B, true, true>(a, blob, trace, ntiles, num_sms, s)
+                       : launch_passes<T, DIM, P, W, B, false, true>(a, blob, trace, ntiles, num_sms, s);
+      return err != cudaSuccess ? err : cudaGetLastError();
+    }
+  }
+  err = a.nvec > 1 ? launch_passes<T, DIM, P, W, B, true, false>(a, blob, trace, ntiles, num_sms, s)
+                   : launch_passes<T, DIM, P, W, B, false, false>(a, blob, trace, ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
   return cudaGetLastError();
 }

@@ -203,19 +203,12 @@ __global__ void k_beta_flex(double* scal) {
   scal[S_RZ] = scal[S_RZN];
 }
 
-__global__ void k_loop_check(double* scal, cudaGraphConditionalHandle h, int max_iter) {
-  const double it = scal[S_ITER] + 1.0;
-  scal[S_ITER] = it;
-  const double pap = scal[S_PAP], rr = scal[S_RR];
-  double st = 0.0;
-  if (!(pap > 0.0) || !isfinite(rr)) st = 2.0;
-  else if (sqrt(rr) <= scal[S_TOL]) st = 1.0;
-  else if (it >= (double)max_iter) st = 3.0;
-  else if ((scal[S_CHUNK] -= 1.0) <= 0.0) st = 4.0;
-  if (st != 0.0) {
-    scal[S_STATUS] = st;
-    cudaGraphSetConditional(h, 0);
-  }
+__global__ void k_loop_check(double* scal, cudaGraphConditionalHandle h, int max_iter) { loop_check(scal, h, max_iter); }
+
+// beta = 0 for the first direction step (p = z)
+__global__ void k_beta_zero(double* scal) {
+  scal[S_BETA] = 0.0;
+  scal[S_RZP] = 1.0;
 }
 
 struct sipg_solver {
@@ -273,7 +266,7 @@ struct sipg_solver {
     }
   }
   template <typename F>
-  void capture_loop(F&& body);
+  void capture_loop(F&& body);  // body(while-node handle)
   ~sipg_solver() {
     drop_graphs();
     if (ev0) cudaEventDestroy(ev0);
@@ -1037,7 +1030,7 @@ void sipg_solver::capture_iteration(int par, F&& body) {
   bool ok = true;
   record_launches(&nodes);  // recorded, not launched
   try {
-    body();
+    body(0);
   } catch (...) {
     ok = false;
   }
@@ -1072,6 +1065,7 @@ void sipg_solver::capture_loop(F&& body) {
   cudaGraphNodeParams cp{};
   cudaGraphNode_t node = nullptr;
   if (ok) ok = cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+  ok = ok && h != 0;  // 0 stands for no loop in the body
   if (ok) {
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = h;
@@ -1085,9 +1079,7 @@ void sipg_solver::capture_loop(F&& body) {
     bool body_ok = true;
     record_launches(&nodes);  // recorded, not launched
     try {
-      body();
-      k_loop_check<<<1, 1, 0, stream>>>(S(), h, o.max_iter);
-      note_launch();
+      body(h);
     } catch (...) {
       body_ok = false;
     }
@@ -1179,9 +1171,30 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
     // the dots ride on the vector passes next to them
     const bool fused = kind == SIPG_SOLVER_PMULTIGRID && o.precision == SIPG_FP32;
     const int mean_slot = o.nullspace ? (int)S_SUM : -1;
-    auto body = [&] {
-      op->apply<double>(Pv, AP, stream);
-      dot(Pv, AP, S_PAP);  // cg3_alpha_pre
+    // the direction update p = z + beta p and p . Ap ride on the operator where it runs as one
+    // pair of launches (then p is formed at the start of an iteration, else at its end)
+    const bool ride = op->one_launch<double>();
+    if (ride) {
+      k_beta_zero<<<1, 1, 0, stream>>>(S());
+      note_launch();
+    }
+    const bool jac = !o.nullspace && (kind == SIPG_SOLVER_JACOBI || kind == SIPG_SOLVER_BLOCK_JACOBI);
+    // loop: the while-node the iteration is captured into (0: none)
+    auto body = [&](cudaGraphConditionalHandle loop) {
+      if (ride) {
+        op->apply_direction(Z, Pv, AP, S(), S_BETA, S_RZP, rw.partial, rw.counter, S() + S_PAP, stream);
+      } else {
+        op->apply<double>(Pv, AP, stream);
+        dot(Pv, AP, S_PAP);  // cg3_alpha_pre
+      }
+      if (jac) {  // update_ans + update_res, preconditioner, beta and the stopping test in one pass
+        if (kind == SIPG_SOLVER_JACOBI)
+          cg_update_precond(x, R, Pv, AP, Z, dinv.as<double>(), 0, n, S(), loop, o.max_iter, rw, stream);
+        else
+          cg_update_precond(x, R, Pv, AP, Z, blocks.as<double>(), op->Np, n, S(), loop, o.max_iter, rw, stream);
+        if (!ride) update_p<double>(Pv, Z, n, S(), S_BETA, S_RZP, stream);
+        return;
+      }
       if (fused) {
         // update_ans + update_res, projection, r . r, r . z_old, r to FP32
         if (o.nullspace) cg_update_xr_sum(x, R, Pv, AP, n, S(), S_RZ, S_PAP, S() + S_SUM, S_TMP - S_SUM, rw, stream);
@@ -1191,11 +1204,6 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
         // z to FP64, projection, r . z_new
         if (o.nullspace) to_f64_sum(Z, lv[0].z.as<float>(), n, S() + S_SUM, rw, stream);
         finish_z_dot(Z, o.nullspace ? nullptr : lv[0].z.as<float>(), R, n, S(), mean_slot, S() + S_RZN, rw, stream);
-      } else if (!o.nullspace && (kind == SIPG_SOLVER_JACOBI || kind == SIPG_SOLVER_BLOCK_JACOBI)) {
-        // update_ans + update_res with r . r and r . z_old; z = M^-1 r with r . z_new
-        cg_update_xr_rzo(x, R, Pv, AP, Z, n, S(), S_RZ, S_PAP, S() + S_RR, S_RZO - S_RR, rw, stream);
-        if (kind == SIPG_SOLVER_JACOBI) precond_dot(Z, R, dinv.as<double>(), 0, n, S() + S_RZN, rw, stream);
-        else precond_dot(Z, R, blocks.as<double>(), op->Np, n, S() + S_RZN, rw, stream);
       } else {
         cg_update_xr(x, R, Pv, AP, n, S(), S_RZ, S_PAP, S() + S_RR, rw, stream);  // update_ans + update_res
         if (o.nullspace) {
@@ -1209,7 +1217,11 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
       }
       k_beta_flex<<<1, 1, 0, stream>>>(S());  // cg3_compute_beta_pre_flex
       note_launch();
-      update_p<double>(Pv, Z, n, S(), S_BETA, S_RZP, stream);
+      if (!ride) update_p<double>(Pv, Z, n, S(), S_BETA, S_RZP, stream);
+      if (loop) {
+        k_loop_check<<<1, 1, 0, stream>>>(S(), loop, o.max_iter);
+        note_launch();
+      }
     };
     auto after = [&](int it_now) {
       iter = it_now;
@@ -1243,7 +1255,7 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
         SIPG_CUDA(cudaGraphLaunch(gx[0], stream));
         note_launch((unsigned)gnodes[0]);
       } else {
-        body();
+        body(0);
       }
       read_scalars();
       after(iter + 1);

@@ -217,50 +217,86 @@ __global__ void __launch_bounds__(kRedThreads) k_finish_z_dot(double* z, const f
   finish<1>(v, partial, counter, out, 1);
 }
 
-// x += alpha p ; r -= alpha Ap ; out[0] = r . r, out[stride] = r . zo
-__global__ void __launch_bounds__(kRedThreads) k_cg_update_xr_rzo(double* x, double* r, const double* p,
-                                                                  const double* Ap, const double* zo, size_t n,
-                                                                  const double* scal, int num, int den,
-                                                                  double* partial, unsigned* counter, double* out,
-                                                                  int stride) {
+// One Jacobi-PCG update (cg_update_precond in vecops.cuh) as one pass: separate kernels for the
+// x / r update, the preconditioner, its dot and the scalars were three more launches per
+// iteration and read r, z and the diagonal again. A CTA takes whole blocks of Np rows (BLK) so
+// that a row of z = B r finds the block's new r in shared memory. Memory-bound for long vectors
+// (9 streams; launch-bound below about 1e5 values).
+template <bool BLK>
+__global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, double* r, const double* p,
+                                                                   const double* Ap, double* z, const double* B,
+                                                                   int Np, size_t n, double* scal,
+                                                                   cudaGraphConditionalHandle loop, int max_iter,
+                                                                   double* partial, unsigned* counter) {
+  __shared__ double sr[BLK ? kRedThreads : 1];
   pdl_enter();
-  const double alpha = scal[num] / scal[den];
-  double v[2] = {0.0, 0.0};
-#pragma unroll 4
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * p[i];
-    double ri = r[i] - alpha * Ap[i];
-    r[i] = ri;
-    v[0] += ri * ri;
-    v[1] += ri * zo[i];
-  }
-  block_sum<2>(v);
-  finish<2>(v, partial, counter, out, stride);
-}
-
-// z = B r (row-major blocks; point Jacobi z = dinv r when Np == 0) ; out = r . z
-__global__ void __launch_bounds__(kRedThreads) k_precond_dot(double* z, const double* r, const double* B, int Np,
-                                                             size_t n, double* partial, unsigned* counter,
-                                                             double* out) {
-  pdl_enter();
-  double v[1] = {0.0};
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double zi;
-    if (Np > 0) {
-      const size_t b = i / Np;
-      const int row = (int)(i - b * Np);
-      const double* Bb = B + (b * Np + row) * Np;
-      const double* rb = r + b * Np;
-      zi = 0.0;
-      for (int j = 0; j < Np; ++j) zi += Bb[j] * rb[j];
-    } else {
-      zi = B[i] * r[i];
+  const double alpha = scal[S_RZ] / scal[S_PAP];
+  double v[3] = {0.0, 0.0, 0.0};  // r . r, r . z_old, r . z
+  if (BLK) {
+    const int rows = kRedThreads / Np * Np;  // of a CTA
+    const bool mine = (int)threadIdx.x < rows;
+    const int b0 = (int)threadIdx.x / Np * Np;
+    for (size_t i0 = blockIdx.x * (size_t)rows; i0 < n; i0 += (size_t)gridDim.x * rows) {
+      const size_t i = i0 + threadIdx.x;
+      const bool act = mine && i < n;
+      double ri = 0.0, zo = 0.0;
+      if (act) {
+        x[i] += alpha * p[i];
+        ri = r[i] - alpha * Ap[i];
+        r[i] = ri;
+        zo = z[i];
+      }
+      __syncthreads();  // the previous blocks' rows have been read
+      sr[threadIdx.x] = ri;
+      __syncthreads();
+      if (act) {
+        const double* Bi = B + i * Np;
+        double zi = 0.0;
+        for (int j = 0; j < Np; ++j) zi += Bi[j] * sr[b0 + j];
+        z[i] = zi;
+        v[0] += ri * ri;
+        v[1] += ri * zo;
+        v[2] += ri * zi;
+      }
     }
-    z[i] = zi;
-    v[0] += r[i] * zi;
+  } else {
+#pragma unroll 2
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+      x[i] += alpha * p[i];
+      const double ri = r[i] - alpha * Ap[i];
+      r[i] = ri;
+      const double zi = B[i] * ri;
+      v[0] += ri * ri;
+      v[1] += ri * z[i];
+      v[2] += ri * zi;
+      z[i] = zi;
+    }
   }
-  block_sum<1>(v);
-  finish<1>(v, partial, counter, out, 1);
+  block_sum<3>(v);
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) partial[blockIdx.x * 4 + k] = v[k];
+    __threadfence();
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) acc[k] += ((volatile double*)partial)[b * 4 + k];
+  __syncthreads();
+  block_sum<3>(acc);
+  if (threadIdx.x == 0) {
+    *counter = 0u;
+    scal[S_RR] = acc[0];
+    scal[S_BETA] = acc[2] - acc[1];
+    scal[S_RZP] = scal[S_RZ];
+    scal[S_RZ] = acc[2];
+    if (loop) loop_check(scal, loop, max_iter);
+  }
 }
 
 template <typename T>
@@ -1013,16 +1049,15 @@ void cg_update_xr_sum(double* x, double* r, const double* p, const double* Ap, s
              w.counter, out, stride);
   note_launch();
 }
-void cg_update_xr_rzo(double* x, double* r, const double* p, const double* Ap, const double* zo, size_t n,
-                      const double* scal, int num, int den, double* out, int stride, const RedWork& w,
-                      cudaStream_t s) {
-  pdl_launch(k_cg_update_xr_rzo, dim3(red_grid(n)), dim3(kRedThreads), 0, s, x, r, p, Ap, zo, n, scal, num, den,
-             w.partial, w.counter, out, stride);
-  note_launch();
-}
-void precond_dot(double* z, const double* r, const double* B, int Np, size_t n, double* out, const RedWork& w,
-                 cudaStream_t s) {
-  pdl_launch(k_precond_dot, dim3(red_grid(n)), dim3(kRedThreads), 0, s, z, r, B, Np, n, w.partial, w.counter, out);
+void cg_update_precond(double* x, double* r, const double* p, const double* Ap, double* z, const double* B, int Np,
+                       size_t n, double* scal, cudaGraphConditionalHandle loop, int max_iter, const RedWork& w,
+                       cudaStream_t s) {
+  if (Np > 0)
+    pdl_launch(k_cg_update_precond<true>, dim3(red_grid(n)), dim3(kRedThreads), 0, s, x, r, p, Ap, z, B, Np, n, scal,
+               loop, max_iter, w.partial, w.counter);
+  else
+    pdl_launch(k_cg_update_precond<false>, dim3(red_grid(n)), dim3(kRedThreads), 0, s, x, r, p, Ap, z, B, Np, n, scal,
+               loop, max_iter, w.partial, w.counter);
   note_launch();
 }
 void resid_prep(double* r, float* r32, const double* zo, size_t n, const double* scal, int mean_slot, double* out,

@@ -73,18 +73,37 @@ void cg_update_xr_sum(double* x, double* r, const double* p, const double* Ap, s
 //   r -= mean (scal[mean_slot] / n, none when mean_slot < 0) ; r32 = r ; out = (r . r, r . zo)
 void resid_prep(double* r, float* r32, const double* zo, size_t n, const double* scal, int mean_slot, double* out,
                 int stride, const RedWork& w, cudaStream_t s);
-//   x += alpha p ; r -= alpha Ap ; out = (r . r, r . zo)
-void cg_update_xr_rzo(double* x, double* r, const double* p, const double* Ap, const double* zo, size_t n,
-                      const double* scal, int num, int den, double* out, int stride, const RedWork& w,
-                      cudaStream_t s);
-//   z = B r (row-major Np x Np blocks; Np == 0: z = B r elementwise, point Jacobi) ; out = r . z
-void precond_dot(double* z, const double* r, const double* B, int Np, size_t n, double* out, const RedWork& w,
-                 cudaStream_t s);
 //   z = z32 ; out = sum z
 void to_f64_sum(double* z, const float* z32, size_t n, double* out, const RedWork& w, cudaStream_t s);
 //   z = (z32 ? z32 : z) - mean (as above) ; out = r . z
 void finish_z_dot(double* z, const float* z32, const double* r, size_t n, const double* scal, int mean_slot,
                   double* out, const RedWork& w, cudaStream_t s);
+// One preconditioned conjugate-gradient update with point (Np == 0, B the reciprocal diagonal)
+// or element-block Jacobi (row-major Np x Np blocks): x += alpha p ; r -= alpha Ap with alpha =
+// scal[S_RZ] / scal[S_PAP] ; scal[S_RR] = r . r ; rzo = r . z ; z = B r ; then, from the one that
+// finishes last, the flexible beta (scal[S_BETA] = r . z - rzo, S_RZP, S_RZ) and, with `loop`
+// not 0, the stopping test of the while-node it belongs to (as loop_check).
+void cg_update_precond(double* x, double* r, const double* p, const double* Ap, double* z, const double* B, int Np,
+                       size_t n, double* scal, cudaGraphConditionalHandle loop, int max_iter, const RedWork& w,
+                       cudaStream_t s);
+// Stopping test of the device-resident outer loop, by one thread at the end of its body: ends the
+// while-node `loop` once converged, broken down, at the iteration limit or at the end of a chunk.
+#ifdef __CUDACC__
+__device__ __forceinline__ void loop_check(double* scal, cudaGraphConditionalHandle loop, int max_iter) {
+  const double it = scal[S_ITER] + 1.0;
+  scal[S_ITER] = it;
+  const double pap = scal[S_PAP], rr = scal[S_RR];
+  double st = 0.0;
+  if (!(pap > 0.0) || !isfinite(rr)) st = 2.0;
+  else if (sqrt(rr) <= scal[S_TOL]) st = 1.0;
+  else if (it >= (double)max_iter) st = 3.0;
+  else if ((scal[S_CHUNK] -= 1.0) <= 0.0) st = 4.0;
+  if (st != 0.0) {
+    scal[S_STATUS] = st;
+    cudaGraphSetConditional(loop, 0);
+  }
+}
+#endif
 // p = z + beta p   with beta = scal[num] / scal[den]
 template <typename T>
 void update_p(T* p, const T* z, size_t n, const double* scal, int num, int den, cudaStream_t s);
