@@ -4,10 +4,11 @@
 // u (x) u (ins_3d_advec_0), its strong-form divergence (mesh->div), the
 // Lax-Friedrichs face fluxes (ins_3d_advec_1 interior, ins_3d_advec_2 boundary:
 // no-slip, slip, natural outflow), their LIFT, and the extrapolated velocity
-// (ins_3d_advec_3): velT = a0 u + a1 u_old - dt (b0 N + b1 N_old).
-// One warp per element (lane = node / face node), FP64; the reference matrices
-// D_r and LIFT sit in shared memory. The boundary kernel's wave speed is the
-// floor of the largest |n . u| over the face (the reference stores it in an int,
+// (ins_3d_advec_3): velT = a0 u + a1 u_old - dt (b0 N + b1 N_old). The advection runs
+// eight elements per warp on the FP64 tensor cores (k_advection), the other kernels
+// one warp per element (lane = node / face node) with the reference matrices D_r and
+// LIFT in shared memory. The boundary kernel's wave speed is the floor of the
+// largest |n . u| over the face (the reference stores it in an int,
 // ins_3d_advec_2.h:44), kept here so the results are the reference's.
 #include <cuda_runtime.h>
 
@@ -21,6 +22,7 @@
 #include "ins_step.cuh"
 #include "runtime.hpp"
 #include "sipg_apply.cuh"
+#include "tc_frag.cuh"
 #include "vecops.cuh"
 
 namespace sipg {
@@ -30,8 +32,26 @@ constexpr int kAdvWarps = 8;
 
 struct AdvTables {
   DevBuf mats;  // Dr, Ds, Dt (Np x Np), LIFT (Np x Nf Nfp), row-major
+  DevBuf adv;   // advection operands in fragment order: D_r (3 x NT x NT blocks), LIFT (FT x NT)
   DevBuf weak;  // Drw, Dsw, Dtw = M^-1 D_r^T M (Np x Np), LIFT: the weak-form divergence
 };
+
+template <int P>
+std::vector<double> advection_operands(const RefElement& r) {
+  using X = Tc<double, 3, P>;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT;
+  std::vector<double> out((size_t)(3 * NT * NT + FT * NT) * X::BLK, 0.0);
+  const double* D[3] = {r.Dr.data(), r.Ds.data(), r.Dt.data()};
+  auto col = [](int m) { return tc_node_col<double, 3, P>(m); };
+  for (int q = 0; q < 3; ++q)
+    for (int m = 0; m < NP; ++m)
+      for (int n = 0; n < NP; ++n) out[q * NT * NT * X::BLK + tc_slot(NT, col(n), col(m))] = D[q][m * NP + n];
+  for (int f = 0; f < NF; ++f)
+    for (int j = 0; j < NFP; ++j)
+      for (int m = 0; m < NP; ++m)
+        out[3 * NT * NT * X::BLK + tc_slot(NT, f * X::TRP + j, col(m))] = r.LIFT[(size_t)m * NF * NFP + f * NFP + j];
+  return out;
+}
 
 const AdvTables& adv_tables(int order) {
   static std::mutex mu;
@@ -50,6 +70,12 @@ const AdvTables& adv_tables(int order) {
   auto t = std::make_unique<AdvTables>();
   t->mats = DevBuf(m.size() * sizeof(double));
   t->mats.upload(m.data(), m.size() * sizeof(double));
+  const std::vector<double> ops = order == 1   ? advection_operands<1>(r)
+                                  : order == 2 ? advection_operands<2>(r)
+                                  : order == 3 ? advection_operands<3>(r)
+                                               : advection_operands<4>(r);
+  t->adv = DevBuf(ops.size() * sizeof(double));
+  t->adv.upload(ops.data(), ops.size() * sizeof(double));
   // weak derivatives: (M D_w f)_i = int d(phi_i)/dr f, i.e. D_w = M^-1 D^T M
   const int Np = r.Np;
   std::vector<double> w;
@@ -77,7 +103,6 @@ const AdvTables& adv_tables(int order) {
 }
 
 struct AdvArgs {
-  const double* mats;
   const int8_t* itab;  // fmask, perm_pos
   const double* geof;
   const int* nbr;
@@ -90,140 +115,207 @@ struct AdvArgs {
   int K;
 };
 
+// Eight elements per warp (the M dimension of the FP64 MMA):
+//   N_c = sum_r H_cr . D_r^T + F_c . LIFT^T,  H_cr = sum_d G_rd u_c u_d,
+// the H fragments formed from the velocity fragments, the face fluxes F as fragments of face-node
+// pairs. The eight elements' velocities are staged per warp for the gathers at their own face
+// nodes; neighbour values come from global memory (an outer face reads the element's own node and
+// replaces it by its type's exterior state). Lane t of a quad holds the normal and type of its
+// element's face t. Measured (with the one-warp-per-element kernel, whose matrix entries came
+// from shared memory at every multiply-add): p = 3, 32^3 x 6 tets
+// 738 -> 189 us (2,480 B per element: 39 % of the HBM rate; 28 MMAs per element: 41 % of the
+// FP64 pipe; latency of the neighbour gathers at 16 warps per SM).
 template <int P>
-__global__ void __launch_bounds__(kAdvWarps * 32) k_advection(const AdvArgs a) {
-  using Cf = Cfg<3, P>;
-  constexpr int NP = Cf::NP, NFP = Cf::NFP, NF = 4, NFNFP = NF * NFP, NG = 10;
-  extern __shared__ double sm[];
-  const double* sD = sm;                       // 3 x NP x NP
-  const double* sL = sm + 3 * NP * NP;         // NP x NFNFP
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* sU = sm + 3 * NP * NP + NP * NFNFP + warp * (12 * NP + 4 * NFNFP);
-  double* sH = sU + 3 * NP;    // [3][3][NP]: H[c][r] = sum_d G[r][d] u_c u_d
-  double* sF = sH + 9 * NP;    // [3][NFNFP] face fluxes
-  double* sS = sF + 3 * NFNFP; // [NFNFP] boundary wave speeds
-  for (int i = threadIdx.x; i < 3 * NP * NP + NP * NFNFP; i += blockDim.x) sm[i] = a.mats[i];
+struct AdvCfg {
+  using X = Tc<double, 3, P>;
+  static constexpr int WARPS = 8, US = X::NP | 1;                     // staged velocity row
+  static constexpr int NB = (3 * X::NT * X::NT + X::FT * X::NT) * X::BLK;  // operand values
+  static constexpr int NTAB = 4 * 6 * X::TRP;                         // neighbour nodes [face][orientation][node]
+  static constexpr size_t smem = (size_t)(NB + WARPS * 24 * US) * sizeof(double) + NTAB;
+};
+
+// PAIR: every array on a 16-byte boundary.
+template <int P, bool PAIR>
+__global__ void __launch_bounds__(AdvCfg<P>::WARPS * 32, 2) k_advection(const AdvArgs a, const double* __restrict__ ops) {
+  using C = AdvCfg<P>;
+  using X = typename C::X;
+  using F = Frag<double>;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = 4, NT = X::NT, FT = X::FT, TRP = X::TRP, US = C::US;
+  extern __shared__ __align__(16) double sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double* sU = sm + C::NB + warp * 24 * US;  // [3][8][US]
+  uint8_t* tab = reinterpret_cast<uint8_t*>(sm + C::NB + C::WARPS * 24 * US);
+  copy_blob(sm, ops, C::NB * (int)sizeof(double));
+  for (int i = threadIdx.x; i < C::NTAB; i += blockDim.x) {
+    const int gf = i / (6 * TRP), sg = i / TRP % 6, j = min(i % TRP, NFP - 1);
+    tab[i] = (uint8_t)a.itab[gf * NFP + a.itab[NF * NFP + sg * NFP + j]];
+  }
+  int fb_m0[FT], fb_m1[FT];  // the lane's face-node pairs: volume nodes (a padding node repeats its partner)
+#pragma unroll
+  for (int fb = 0; fb < FT; ++fb) {
+    const int k0 = 8 * fb + 2 * t, f = k0 / TRP, j0 = k0 % TRP;
+    fb_m0[fb] = a.itab[f * NFP + j0];
+    fb_m1[fb] = j0 + 1 < NFP ? a.itab[f * NFP + j0 + 1] : fb_m0[fb];
+  }
+  cp_wait_all();
   __syncthreads();
-  const int8_t* fmask = a.itab;
-  const int8_t* perm = a.itab + NF * NFP;
+  const double* BL = sm + 3 * NT * NT * X::BLK;
   const size_t n = (size_t)a.K * NP;
-  for (int e = blockIdx.x * kAdvWarps + warp; e < a.K; e += gridDim.x * kAdvWarps) {
-    double g[NG];
+  const int ntiles = (a.K + 7) / 8;
+  for (int tile = warp * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * C::WARPS) {
+    const int e0 = tile * 8, ne = min(8, a.K - e0), e = min(e0 + g, a.K - 1);
+    double G[3][3];
 #pragma unroll
-    for (int k = 0; k < NG; ++k) g[k] = __ldg(a.geof + (size_t)e * NG + k);
-    __syncwarp();
-    for (int i = lane; i < NP; i += 32) {
-      double uc[3];
+    for (int k = 0; k < 9; ++k) G[k / 3][k % 3] = a.geof[(size_t)e * 10 + k];
+    const int nbt = a.nbr[(size_t)e * NF + t];
+    const uint32_t code = a.fcode[e];
+    double u[3][NT][1][2];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        uc[c] = a.u[c * n + (size_t)e * NP + i];
-        sU[c * NP + i] = uc[c];
-      }
+    for (int c = 0; c < 3; ++c) load_nodes<double, 3, P, PAIR>(a.u + c * n, e0, ne, u[c], g, t);
+    const int kindt = nbt < 0 ? a.vel_bc[-nbt - 1] : -1;
+    __syncwarp();  // the previous tile's gathers are done
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          const int m = frag_node<double, 3, P>(nt, ci, t);
+          if (m < NP) sU[(c * 8 + g) * US + m] = u[c][nt][0][ci];
+        }
+    // unit normal and fscale (the length of the unnormalised normal) of face t
+    double nv[3], fst;
+    {
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        nv[d] = t == 0 ? -G[2][d] : t == 1 ? -G[1][d] : t == 2 ? (G[0][d] + G[1][d]) + G[2][d] : -G[0][d];
+      fst = sqrt(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
+      const double inv = 1.0 / fst;
+      nv[0] *= inv; nv[1] *= inv; nv[2] *= inv;
+    }
+    double acc[3][NT][1][2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) acc[c][nt][0][0] = acc[c][nt][0][1] = 0.0;
+#pragma unroll
+    for (int kb = 0; kb < NT; ++kb) {
+      double w[3][3][2];  // u_c u_d
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          double s = 0.0;
+        for (int d = c; d < 3; ++d)
 #pragma unroll
-          for (int d = 0; d < 3; ++d) s += g[r * 3 + d] * (uc[c] * uc[d]);
-          sH[(c * 3 + r) * NP + i] = s;
-        }
-    }
-    __syncwarp();
-    // face fluxes (ins_3d_advec_1 / ins_3d_advec_2)
-    for (int m = lane; m < NFNFP; m += 32) {
-      const int f = m / NFP, j = m - f * NFP;
-      double nv[3], sJ;
-      simplex_face_normal<3>(g, f, nv, &sJ);
-      const double fs = sJ / g[9];
-      const int o = fmask[f * NFP + j];
-      const double uM[3] = {sU[o], sU[NP + o], sU[2 * NP + o]};
-      const double lvel = nv[0] * uM[0] + nv[1] * uM[1] + nv[2] * uM[2];
-      const int nb = __ldg(a.nbr + (size_t)e * NF + f);
-      if (nb >= 0) {
-        const int code = (__ldg(a.fcode + e) >> (8 * f)) & 0xff;
-        const int gf = code & 3, sg = code >> 2;
-        const int nn = fmask[gf * NFP + perm[sg * NFP + j]];
-        double uP[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) uP[c] = a.u[c * n + (size_t)nb * NP + nn];
-        double gn[NG], np_[3], sJn;
-#pragma unroll
-        for (int k = 0; k < NG; ++k) gn[k] = __ldg(a.geof + (size_t)nb * NG + k);
-        simplex_face_normal<3>(gn, gf, np_, &sJn);
-        const double rvel = np_[0] * uP[0] + np_[1] * uP[1] + np_[2] * uP[2];
-        const double nuP = nv[0] * uP[0] + nv[1] * uP[1] + nv[2] * uP[2];
-        const double lam = fmax(fabs(lvel), fabs(rvel));
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sF[c * NFNFP + m] = 0.5 * fs * (-(uM[c] * lvel - uP[c] * nuP) - lam * (uP[c] - uM[c]));
-        sS[m] = -1.0;
-      } else {
-        const int kind = __ldg(a.vel_bc + (-nb - 1));
-        double uR[3];
-        if (kind == 0) {
-          uR[0] = uR[1] = uR[2] = 0.0;
-        } else if (kind == 1) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) uR[c] = uM[c] - lvel * nv[c];
-        } else {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) uR[c] = uM[c];
-        }
-        const double rvel = nv[0] * uR[0] + nv[1] * uR[1] + nv[2] * uR[2];
-        sS[m] = fmax(fabs(lvel), fabs(rvel));
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sF[c * NFNFP + m] = 0.5 * fs * (-(uM[c] * lvel - uR[c] * rvel));  // + wave term below
-      }
-    }
-    __syncwarp();
-    // boundary wave term: - floor(max over the face of the speeds) (uR - uM)
-    for (int m = lane; m < NFNFP; m += 32) {
-      if (sS[m] < 0.0) continue;
-      const int f = m / NFP, j = m - f * NFP;
-      double mx = 0.0;
-      for (int k = 0; k < NFP; ++k) mx = fmax(mx, sS[f * NFP + k]);
-      const double lam = (double)(int)mx;
-      if (lam == 0.0) continue;
-      double nv[3], sJ;
-      simplex_face_normal<3>(g, f, nv, &sJ);
-      const double fs = sJ / g[9];
-      const int o = fmask[f * NFP + j];
-      const double uM[3] = {sU[o], sU[NP + o], sU[2 * NP + o]};
-      const double lvel = nv[0] * uM[0] + nv[1] * uM[1] + nv[2] * uM[2];
-      const int kind = __ldg(a.vel_bc + (-__ldg(a.nbr + (size_t)e * NF + f) - 1));
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double uR = kind == 0 ? 0.0 : kind == 1 ? uM[c] - lvel * nv[c] : uM[c];
-        sF[c * NFNFP + m] += 0.5 * fs * (-lam * (uR - uM[c]));
-      }
-    }
-    __syncwarp();
-    // N = sum_r D_r H_r + LIFT flux, then velT
-    for (int i = lane; i < NP; i += 32) {
-      double Nc[3] = {0.0, 0.0, 0.0};
+          for (int ci = 0; ci < 2; ++ci) w[c][d][ci] = w[d][c][ci] = u[c][kb][0][ci] * u[d][kb][0][ci];
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        const double* Dr = sD + r * NP * NP + i * NP;
-        for (int k = 0; k < NP; ++k) {
-          const double dv = Dr[k];
+        double h[3][1][2];
 #pragma unroll
-          for (int c = 0; c < 3; ++c) Nc[c] += dv * sH[(c * 3 + r) * NP + k];
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci)
+            h[c][0][ci] = G[r][0] * w[c][0][ci] + G[r][1] * w[c][1][ci] + G[r][2] * w[c][2][ci];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          const double2 b = ldb(sm, (r * NT + kb) * NT + nt, lane);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) mma_nodes<double, 3, P>(acc[c][nt], h[c], b, kb);
         }
       }
-      const double* Li = sL + i * NFNFP;
-      for (int k = 0; k < NFNFP; ++k) {
-        const double lv = Li[k];
+    }
+    __syncwarp();
+    // boundary wave speeds: the floor of the largest |n . u| over the face, both sides
+    double lamb[NF] = {0.0, 0.0, 0.0, 0.0};
+    if (__any_sync(0xffffffffu, nbt < 0)) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) Nc[c] += lv * sF[c * NFNFP + k];
+      for (int fb = 0; fb < FT; ++fb) {
+        const int f = (8 * fb + 2 * t) / TRP, src = (lane & ~3) + f;
+        double q[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) q[d] = __shfl_sync(0xffffffffu, nv[d], src);
+        const int kind = __shfl_sync(0xffffffffu, kindt, src);
+        double mx = 0.0;
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          const double* um = sU + g * US + (ci ? fb_m1[fb] : fb_m0[fb]);
+          const double lvel = q[0] * um[0] + q[1] * um[8 * US] + q[2] * um[16 * US];
+          // exterior: nothing (no-slip), the tangential part (slip), the same (outflow)
+          mx = fmax(mx, fabs(lvel));
+          if (kind == 1) {
+            double rv = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) rv += q[d] * (um[d * 8 * US] - lvel * q[d]);
+            mx = fmax(mx, fabs(rv));
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < NF; ++k)
+          if (f == k) lamb[k] = fmax(lamb[k], mx);
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const size_t idx = c * n + (size_t)e * NP + i;
-        a.N[idx] = Nc[c];
-        const double gc = c == 1 ? a.grav : 0.0;
-        a.velT[idx] =
-            (a.a0 * sU[c * NP + i] + a.a1 * a.u_old[idx]) - a.dt * (a.b0 * (Nc[c] + gc) + a.b1 * (a.N_old[idx] + gc));
+      for (int k = 0; k < NF; ++k) {
+        lamb[k] = fmax(lamb[k], __shfl_xor_sync(0xffffffffu, lamb[k], 1));
+        lamb[k] = (double)(int)fmax(lamb[k], __shfl_xor_sync(0xffffffffu, lamb[k], 2));
       }
+    }
+    // face fluxes and their lift
+#pragma unroll
+    for (int fb = 0; fb < FT; ++fb) {
+      const int k0 = 8 * fb + 2 * t, f = k0 / TRP, j0 = k0 % TRP, src = (lane & ~3) + f;
+      double q[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) q[d] = __shfl_sync(0xffffffffu, nv[d], src);
+      const double hfs = 0.5 * __shfl_sync(0xffffffffu, fst, src);
+      const int nb = __shfl_sync(0xffffffffu, nbt, src), kind = __shfl_sync(0xffffffffu, kindt, src);
+      const unsigned cf = (code >> (8 * f)) & 255u;
+      const uint8_t* pos = tab + ((cf & 3u) * 6 + (cf >> 2)) * TRP + j0;
+      double fl[3][1][2];
+#pragma unroll
+      for (int ci = 0; ci < 2; ++ci) {
+        const int m = ci ? fb_m1[fb] : fb_m0[fb];
+        const size_t idx = nb >= 0 ? (size_t)nb * NP + pos[ci] : (size_t)e * NP + m;
+        double uM[3], uP[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          uM[c] = sU[(c * 8 + g) * US + m];
+          uP[c] = a.u[c * n + idx];
+        }
+        const double lvel = q[0] * uM[0] + q[1] * uM[1] + q[2] * uM[2];
+        if (kind == 0 || kind == 1)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) uP[c] = kind == 0 ? 0.0 : uM[c] - lvel * q[c];
+        const double nuP = q[0] * uP[0] + q[1] * uP[1] + q[2] * uP[2];
+        double lam = fmax(fabs(lvel), fabs(nuP));
+        if (nb < 0) lam = f == 0 ? lamb[0] : f == 1 ? lamb[1] : f == 2 ? lamb[2] : lamb[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          fl[c][0][ci] = j0 + ci < NFP ? hfs * (-(uM[c] * lvel - uP[c] * nuP) - lam * (uP[c] - uM[c])) : 0.0;
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const double2 b = ldb(BL, fb * NT + nt, lane);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) F::mma(acc[c][nt], fl[c], b);
+      }
+    }
+    // N and velT
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      double uo[NT][1][2], no[NT][1][2], um[NT][1][2];
+      load_nodes<double, 3, P, PAIR>(a.u_old + c * n, e0, ne, uo, g, t);
+      load_nodes<double, 3, P, PAIR>(a.N_old + c * n, e0, ne, no, g, t);
+      store_nodes<double, 3, P, PAIR>(a.N + c * n, e0, ne, acc[c], g, t);
+      const double gc = c == 1 ? a.grav : 0.0;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          const int m = frag_node<double, 3, P>(nt, ci, t);
+          const double uv = m < NP ? sU[(c * 8 + g) * US + m] : 0.0;
+          um[nt][0][ci] = (a.a0 * uv + a.a1 * uo[nt][0][ci]) -
+                          a.dt * (a.b0 * (acc[c][nt][0][ci] + gc) + a.b1 * (no[nt][0][ci] + gc));
+        }
+      store_nodes<double, 3, P, PAIR>(a.velT + c * n, e0, ne, um, g, t);
     }
   }
 }
@@ -336,14 +428,15 @@ void launch_pressure_neumann_t(const PnArgs& a, cudaStream_t s) {
 }
 
 template <int P>
-void launch_advection_t(const AdvArgs& a, cudaStream_t s) {
-  using Cf = Cfg<3, P>;
-  constexpr int NP = Cf::NP, NFNFP = 4 * Cf::NFP;
-  const size_t smem = (size_t)(3 * NP * NP + NP * NFNFP + kAdvWarps * (12 * NP + 4 * NFNFP)) * sizeof(double);
-  auto k = k_advection<P>;
-  SIPG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = std::max(1, std::min((a.K + kAdvWarps - 1) / kAdvWarps, num_sms() * 8));
-  k<<<grid, kAdvWarps * 32, smem, s>>>(a);
+void launch_advection_t(const AdvArgs& a, const double* ops, cudaStream_t s) {
+  using C = AdvCfg<P>;
+  bool pair = true;
+  for (const void* p : {(const void*)a.u, (const void*)a.u_old, (const void*)a.N_old, (const void*)a.N, (const void*)a.velT})
+    pair = pair && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+  auto k = pair ? k_advection<P, true> : k_advection<P, false>;
+  SIPG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
+  const int grid = std::max(1, std::min((a.K + 7) / 8, num_sms() * 2));
+  k<<<grid, C::WARPS * 32, C::smem, s>>>(a, ops);
   note_launch();
   SIPG_CUDA(cudaGetLastError());
 }
@@ -603,8 +696,8 @@ void advection_device(sipg_mesh* m, int order, double dt, double a0, double a1, 
   if (m->dim != 3) throw Error(SIPG_INVALID_ARG, "the advection step is 3D");
   if (order < 1 || order > 4) throw Error(SIPG_INVALID_ARG, "order must be 1..4");
   m->ensure_device();
+  const double* ops = adv_tables(order).adv.as<double>();
   AdvArgs a;
-  a.mats = adv_tables(order).mats.as<double>();
   a.itab = dev_ref(3, order).itab.as<int8_t>();
   a.geof = m->geof64.as<double>();
   a.nbr = m->nbr.as<int>();
@@ -623,10 +716,10 @@ void advection_device(sipg_mesh* m, int order, double dt, double a0, double a1, 
   a.grav = grav;
   a.K = m->K;
   switch (order) {
-    case 1: launch_advection_t<1>(a, s); break;
-    case 2: launch_advection_t<2>(a, s); break;
-    case 3: launch_advection_t<3>(a, s); break;
-    default: launch_advection_t<4>(a, s); break;
+    case 1: launch_advection_t<1>(a, ops, s); break;
+    case 2: launch_advection_t<2>(a, ops, s); break;
+    case 3: launch_advection_t<3>(a, ops, s); break;
+    default: launch_advection_t<4>(a, ops, s); break;
   }
 }
 

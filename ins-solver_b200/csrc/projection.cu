@@ -40,6 +40,7 @@
 #include "../../include/sipg_b200.h"
 #include "capi_util.hpp"
 #include "pdl.cuh"
+#include "tc_frag.cuh"
 #include "vecops.cuh"
 
 namespace sipg {
@@ -518,14 +519,16 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
 }
 
 
-// Right-hand side of the pressure solve, two elements per warp (one at p = 4 in 3D):
+// Right-hand side of the pressure solve, eight elements per warp on the FP64 tensor cores:
 //   rhs = J M ( -(div_c velT) / dt + LIFT dPdN_new ),  dPdN_new = b0 dPdN + b1 dPdN_old,
 // div_c the central-flux divergence (volume sum_k D_k (G u)_k plus LIFT of
-// fscale n . (u+ - u-) / 2 on interior faces); dPdN_old <- dPdN_new.
+// fscale n . (u+ - u-) / 2 on interior faces); dPdN_old <- dPdN_new. With M LIFT = EMAT the mass
+// is folded into the operands: rhs = sum_k w_k . (M D_k)^T + F . EMAT^T,
+//   w_k = -(J / dt) (G u)_k,  F = J (dPdN_new - fscale n . (u+ - u-) / (2 dt)).
 struct PrRhsArgs {
   int K;
   const double* geof;
-  const double* mats;
+  const double* ops;       // M D_k (D x NT x NT blocks), EMAT (FT x NT), in fragment order
   double dt, b0, b1;
   const int* nbr;
   const uint32_t* fcode;
@@ -536,189 +539,171 @@ struct PrRhsArgs {
   double* rhs;             // K x Np
 };
 
+// Measured (with two elements per warp and the matrices read from shared memory at every
+// multiply-add): p = 3, 32^3 x 6 tets 313 -> 116 us
+// (1,060 B per element without dPdN_old: latency of the gathers at the face nodes).
 template <int D, int P>
-__global__ void __launch_bounds__(kProjWarps * 32) k_pr_rhs(const PrRhsArgs a) {
-  constexpr int NP = proj_np(D, P), NPE = proj_npe(D, P), NPL = (NP + 31) / 32, NG = D == 3 ? 10 : 5;
-  constexpr int NF = D + 1, NFP = proj_nfp(D, P), NFPE = proj_nfpe(D, P), MAT = proj_mat_doubles<D, P>();
-  constexpr int E = proj_epw(D, P);  // elements per warp: each matrix read serves all of them
-  constexpr int WB = E * ((D + 1) * NPE + 2 * NF * NFPE);
-  extern __shared__ double sm[];
-  const double* sD = sm;
-  const double* sM = sm + 2 * D * MAT;
-  const double* sL = sm + proj_nmat(D) * MAT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* sGU = sm + proj_blob_doubles<D, P>() + warp * WB;  // [E][D][NPE]
-  double* sPre = sGU + E * D * NPE;                          // [E][NPE]
-  double* sF1 = sPre + E * NPE;                              // [E][NF][NFPE] fscale n . (u+ - u-) / 2
-  double* sF2 = sF1 + E * NF * NFPE;                         // [E][NF][NFPE] dPdN_new
-  for (int i = threadIdx.x; i < proj_blob_doubles<D, P>(); i += blockDim.x) sm[i] = a.mats[i];
-  for (int i = lane; i < WB; i += 32) sGU[i] = 0.0;
+struct PrRhsCfg {
+  using X = Tc<double, D, P>;
+  static constexpr int WARPS = 8, US = X::NP | 1;
+  static constexpr int NPERM = Cfg<D, P>::NPERM;
+  static constexpr int NB = (D * X::NT * X::NT + X::FT * X::NT) * X::BLK;
+  static constexpr int NTAB = X::NF * NPERM * X::TRP;  // neighbour nodes [face][orientation][node]
+  static constexpr size_t smem = (size_t)(NB + WARPS * D * 8 * US) * sizeof(double) + NTAB;
+};
+
+// PAIR: velT and rhs on a 16-byte boundary.
+template <int D, int P, bool PAIR>
+__global__ void __launch_bounds__(PrRhsCfg<D, P>::WARPS * 32, 2) k_pr_rhs(const PrRhsArgs a) {
+  using C = PrRhsCfg<D, P>;
+  using X = typename C::X;
+  using F = Frag<double>;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT, FT = X::FT, TRP = X::TRP, US = C::US,
+                NG = D == 3 ? 10 : 5;
+  extern __shared__ __align__(16) double sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double* sU = sm + C::NB + warp * D * 8 * US;  // [D][8][US]
+  uint8_t* tab = reinterpret_cast<uint8_t*>(sm + C::NB + C::WARPS * D * 8 * US);
+  copy_blob(sm, a.ops, C::NB * (int)sizeof(double));
+  for (int i = threadIdx.x; i < C::NTAB; i += blockDim.x) {
+    const int gf = i / (C::NPERM * TRP), sg = i / TRP % C::NPERM, j = min(i % TRP, NFP - 1);
+    tab[i] = (uint8_t)a.itab[gf * NFP + a.itab[NF * NFP + sg * NFP + j]];
+  }
+  int fb_m0[FT], fb_m1[FT];  // the lane's face-node pairs: volume nodes (padding repeats a valid node)
+#pragma unroll
+  for (int fb = 0; fb < FT; ++fb) {
+    const int k0 = 8 * fb + 2 * t, f = min(k0 / TRP, NF - 1), j0 = k0 % TRP;
+    fb_m0[fb] = a.itab[f * NFP + j0];
+    fb_m1[fb] = j0 + 1 < NFP ? a.itab[f * NFP + j0 + 1] : fb_m0[fb];
+  }
+  cp_wait_all();
   __syncthreads();
+  const double* BE = sm + D * NT * NT * X::BLK;
   const size_t n = (size_t)a.K * NP;
-  const int8_t* fmask = a.itab;
-  const int8_t* npos = a.itab + NF * NFP;
   const double inv_dt = 1.0 / a.dt;
-  for (int e0 = (blockIdx.x * kProjWarps + warp) * E; e0 < a.K; e0 += gridDim.x * kProjWarps * E) {
-    double G[E][3][3], J[E];
-    bool valid[E];
+  const int ntiles = (a.K + 7) / 8;
+  for (int tile = warp * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * C::WARPS) {
+    const int e0 = tile * 8, ne = min(8, a.K - e0), e = min(e0 + g, a.K - 1);
+    double G[D][D];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      valid[e] = e0 + e < a.K;
-      const double* g = a.geof + (size_t)(valid[e] ? e0 + e : e0) * NG;
+    for (int k = 0; k < D * D; ++k) G[k / D][k % D] = a.geof[(size_t)e * NG + k];
+    const double J = a.geof[(size_t)e * NG + NG - 1];
+    const int nbt = t < NF ? a.nbr[(size_t)e * NF + t] : -1;  // lane t of the quad: face t
+    const uint32_t code = a.fcode[e];
+    double u[D][NT][1][2];
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
+    for (int c = 0; c < D; ++c) load_nodes<double, D, P, PAIR>(a.velT + c * n, e0, ne, u[c], g, t);
+    __syncwarp();  // the previous tile's gathers are done
 #pragma unroll
-        for (int c = 0; c < 3; ++c) G[e][k][c] = 0.0;
-      if (D == 3) {
+    for (int c = 0; c < D; ++c)
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
+      for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) G[e][k][c] = __ldg(g + k * 3 + c);
-        J[e] = __ldg(g + 9);
-      } else {
-        G[e][0][0] = __ldg(g + 0); G[e][0][1] = __ldg(g + 1);
-        G[e][1][0] = __ldg(g + 2); G[e][1][1] = __ldg(g + 3);
-        J[e] = __ldg(g + 4);
-      }
-    }
-    __syncwarp();  // the previous elements' reads of the buffers are done
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-#pragma unroll
-      for (int u = 0; u < NPL; ++u) {
-        const int i = lane + 32 * u;
-        if (i < NP) {
-          double uc[D];
-#pragma unroll
-          for (int c = 0; c < D; ++c) uc[c] = valid[e] ? __ldg(a.velT + c * n + (size_t)(e0 + e) * NP + i) : 0.0;
-#pragma unroll
-          for (int k = 0; k < D; ++k) {
-            double s = 0.0;
-#pragma unroll
-            for (int c = 0; c < D; ++c) s += G[e][k][c] * uc[c];
-            sGU[(e * D + k) * NPE + i] = s;
-          }
+        for (int ci = 0; ci < 2; ++ci) {
+          const int m = frag_node<double, D, P>(nt, ci, t);
+          if (m < NP) sU[(c * 8 + g) * US + m] = u[c][nt][0][ci];
         }
-      }
-    // face terms: the warp's neighbour indices and face codes first (one lane per
-    // element face), then every lane issues all of its face nodes' loads before it uses
-    // any of them (the neighbour's velocities wait on the neighbour index)
-    constexpr int NFN = NF * NFP, ITEMS = (E * NFN + 31) / 32;
-    int nbv = -1;
-    uint32_t codev = 0;
-    if (lane < E * NF) {
-      const int e = lane / NF, f = lane - (lane / NF) * NF;
-      if (e0 + e < a.K) {
-        nbv = __ldg(a.nbr + (size_t)(e0 + e) * NF + f);
-        codev = __ldg(a.fcode + e0 + e);
-      }
-    }
-    double vP[ITEMS][D], vM[ITEMS][D], dnv[ITEMS];
-    int nbi[ITEMS];
+    double y[NT][1][2];
 #pragma unroll
-    for (int u = 0; u < ITEMS; ++u) {
-      const int it = lane + 32 * u;
-      const int e = min(it / NFN, E - 1), m = it - (it / NFN) * NFN, f = m / NFP, k = m - f * NFP;
-      const bool act = it < E * NFN && e0 + e < a.K;
-      const int nb = __shfl_sync(0xffffffffu, nbv, e * NF + f);
-      const uint32_t code = __shfl_sync(0xffffffffu, codev, e * NF + f);
-      nbi[u] = act ? nb : -1;
-      dnv[u] = 0.0;
+    for (int nt = 0; nt < NT; ++nt) y[nt][0][0] = y[nt][0][1] = 0.0;
+    const double s = -J * inv_dt;
 #pragma unroll
-      for (int d = 0; d < D; ++d) vP[u][d] = vM[u][d] = 0.0;
-      if (act) {
-        const int el = e0 + e;
-        if (nb >= 0) {
-          const int cf = (code >> (8 * f)) & 0xff;
-          const int fr = cf & 3, sg = cf >> 2;
-          const int nn = fmask[fr * NFP + npos[sg * NFP + k]], o = fmask[f * NFP + k];
+    for (int kb = 0; kb < NT; ++kb)
 #pragma unroll
-          for (int d = 0; d < D; ++d) {
-            vP[u][d] = __ldg(a.velT + d * n + (size_t)nb * NP + nn);
-            vM[u][d] = __ldg(a.velT + d * n + (size_t)el * NP + o);
-          }
+      for (int k = 0; k < D; ++k) {
+        double w[1][2];
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          double v = 0.0;
+#pragma unroll
+          for (int c = 0; c < D; ++c) v += G[k][c] * u[c][kb][0][ci];
+          w[0][ci] = s * v;
         }
-        const size_t fi = (size_t)el * NF * NFP + m;
-        dnv[u] = (a.dPdN ? a.b0 * a.dPdN[fi] : 0.0) + (a.dPdN_old ? a.b1 * a.dPdN_old[fi] : 0.0);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) mma_nodes<double, D, P>(y[nt], w, ldb(sm, (k * NT + kb) * NT + nt, lane), kb);
       }
-    }
-#pragma unroll
-    for (int u = 0; u < ITEMS; ++u) {
-      const int it = lane + 32 * u;
-      if (it >= E * NFN) continue;
-      const int e = it / NFN, m = it - e * NFN, f = m / NFP, k = m - f * NFP;
-      double un = 0.0;
-      if (nbi[u] >= 0) {
-#pragma unroll
-        for (int ee = 0; ee < E; ++ee) {
-          if (ee != e) continue;
-#pragma unroll
-          for (int d = 0; d < D; ++d) {
-            double v;  // fscale n_d of face f (the unnormalised outward normal)
-            if (D == 3)
-              v = f == 0 ? -G[ee][2][d] : f == 1 ? -G[ee][1][d] : f == 2 ? (G[ee][0][d] + G[ee][1][d]) + G[ee][2][d]
-                                                                           : -G[ee][0][d];
-            else
-              v = f == 0 ? -G[ee][1][d] : f == 1 ? G[ee][0][d] + G[ee][1][d] : -G[ee][0][d];
-            un += v * (0.5 * (vP[u][d] - vM[u][d]));
-          }
-        }
-      }
-      if (e0 + e < a.K && a.dPdN_old) a.dPdN_old[(size_t)(e0 + e) * NF * NFP + m] = dnv[u];
-      sF1[(e * NF + f) * NFPE + k] = un;
-      sF2[(e * NF + f) * NFPE + k] = dnv[u];
-    }
     __syncwarp();
 #pragma unroll
-    for (int u = 0; u < NPL; ++u) {
-      const int i = lane + 32 * u;
-      if (i < NP) {
-        double vol[E], l1[E], l2[E], y[E];
+    for (int fb = 0; fb < FT; ++fb) {
+      const int k0 = 8 * fb + 2 * t, f = k0 / TRP, j0 = k0 % TRP;
+      const bool pad = X::KF % 8 != 0 && f >= NF;
+      const int nb = __shfl_sync(0xffffffffu, nbt, (lane & ~3) + (pad ? 0 : f));
+      const unsigned cf = pad ? 0u : (code >> (8 * f)) & 255u;
+      const uint8_t* pos = tab + ((cf & 3u) * C::NPERM + (cf >> 2)) * TRP + j0;
+      double fv[1][2] = {{0.0, 0.0}};
+      if (!pad) {
+        double v[D];  // fscale n, the unnormalised outward normal
 #pragma unroll
-        for (int e = 0; e < E; ++e) vol[e] = l1[e] = l2[e] = 0.0;
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-          mat_vec<NP, NPE, E>(sD + k * MAT, sGU + k * NPE, D * NPE, i, y);
-#pragma unroll
-          for (int e = 0; e < E; ++e) vol[e] += y[e];
+        for (int d = 0; d < D; ++d) {
+          if (D == 3)
+            v[d] = f == 0 ? -G[D - 1][d] : f == 1 ? -G[1][d] : f == 2 ? (G[0][d] + G[1][d]) + G[D - 1][d] : -G[0][d];
+          else
+            v[d] = f == 0 ? -G[1][d] : f == 1 ? G[0][d] + G[1][d] : -G[0][d];
         }
 #pragma unroll
-        for (int f = 0; f < NF; ++f) {
-          mat_vec<NP, NFPE, E>(sL + f * NP * NFPE, sF1 + f * NFPE, NF * NFPE, i, y);
+        for (int ci = 0; ci < 2; ++ci) {
+          if (j0 + ci >= NFP) continue;
+          double un = 0.0;
+          if (nb >= 0) {
+            const size_t idx = (size_t)nb * NP + pos[ci];
+            const int m = ci ? fb_m1[fb] : fb_m0[fb];
 #pragma unroll
-          for (int e = 0; e < E; ++e) l1[e] += y[e];
-          mat_vec<NP, NFPE, E>(sL + f * NP * NFPE, sF2 + f * NFPE, NF * NFPE, i, y);
-#pragma unroll
-          for (int e = 0; e < E; ++e) l2[e] += y[e];
+            for (int d = 0; d < D; ++d) un += v[d] * (0.5 * (a.velT[d * n + idx] - sU[(d * 8 + g) * US + m]));
+          }
+          double dn = 0.0;
+          if (g < ne) {
+            const size_t fi = ((size_t)e * NF + f) * NFP + j0 + ci;
+            dn = (a.dPdN ? a.b0 * a.dPdN[fi] : 0.0) + (a.dPdN_old ? a.b1 * a.dPdN_old[fi] : 0.0);
+            if (a.dPdN_old) a.dPdN_old[fi] = dn;
+          }
+          fv[0][ci] = J * (dn - un * inv_dt);
         }
-#pragma unroll
-        for (int e = 0; e < E; ++e) sPre[e * NPE + i] = -(vol[e] + l1[e]) * inv_dt + l2[e];
       }
-    }
-    __syncwarp();
 #pragma unroll
-    for (int u = 0; u < NPL; ++u) {
-      const int i = lane + 32 * u;
-      if (i < NP) {
-        double y[E];
-        mat_vec<NP, NPE, E>(sM, sPre, NPE, i, y);
-#pragma unroll
-        for (int e = 0; e < E; ++e)
-          if (valid[e]) a.rhs[(size_t)(e0 + e) * NP + i] = J[e] * y[e];
-      }
+      for (int nt = 0; nt < NT; ++nt) F::mma(y[nt], fv, ldb(BE, fb * NT + nt, lane));
     }
+    store_nodes<double, D, P, PAIR>(a.rhs, e0, ne, y, g, t);
   }
 }
 
 template <int D, int P>
-__host__ __device__ constexpr int pr_rhs_smem_doubles() {
-  return proj_blob_doubles<D, P>() +
-         kProjWarps * proj_epw(D, P) * ((D + 1) * proj_npe(D, P) + 2 * (D + 1) * proj_nfpe(D, P));
+std::vector<double> pr_rhs_operands(const RefElement& r) {
+  using X = Tc<double, D, P>;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = X::NF, NT = X::NT;
+  std::vector<double> out(PrRhsCfg<D, P>::NB, 0.0);
+  const double* Dk[3] = {r.Dr.data(), r.Ds.data(), r.Dt.data()};
+  auto col = [](int m) { return tc_node_col<double, D, P>(m); };
+  for (int k = 0; k < D; ++k)
+    for (int m = 0; m < NP; ++m)
+      for (int j = 0; j < NP; ++j) {
+        double v = 0.0;
+        for (int i = 0; i < NP; ++i) v += r.M[(size_t)m * NP + i] * Dk[k][(size_t)i * NP + j];
+        out[k * NT * NT * X::BLK + tc_slot(NT, col(j), col(m))] = v;
+      }
+  for (int f = 0; f < NF; ++f)
+    for (int j = 0; j < NFP; ++j)
+      for (int m = 0; m < NP; ++m)
+        out[D * NT * NT * X::BLK + tc_slot(NT, f * X::TRP + j, col(m))] = r.EMAT[(size_t)m * NF * NFP + f * NFP + j];
+  return out;
+}
+
+std::vector<double> pr_rhs_operands(int dim, int order, const RefElement& r) {
+  switch (dim * 10 + order) {
+    case 21: return pr_rhs_operands<2, 1>(r);
+    case 22: return pr_rhs_operands<2, 2>(r);
+    case 23: return pr_rhs_operands<2, 3>(r);
+    case 24: return pr_rhs_operands<2, 4>(r);
+    case 31: return pr_rhs_operands<3, 1>(r);
+    case 32: return pr_rhs_operands<3, 2>(r);
+    case 33: return pr_rhs_operands<3, 3>(r);
+    default: return pr_rhs_operands<3, 4>(r);
+  }
 }
 
 // Reference-element matrices in the kernel's layouts, per (device, dim, order).
 struct ProjMats {
   DevBuf blob;
+  DevBuf rhs_ops;  // pressure right-hand side (PrRhsArgs::ops)
   int Np = 0;
 };
 
@@ -759,6 +744,9 @@ const ProjMats& proj_mats(int dim, int order) {
   pm->Np = Np;
   pm->blob = DevBuf(b.size() * sizeof(double));
   pm->blob.upload(b.data(), b.size() * sizeof(double));
+  const std::vector<double> ro = pr_rhs_operands(dim, order, ref);
+  pm->rhs_ops = DevBuf(ro.size() * sizeof(double));
+  pm->rhs_ops.upload(ro.data(), ro.size() * sizeof(double));
   SIPG_CUDA(cudaDeviceSynchronize());
   slot = std::move(pm);
   return *slot;
@@ -790,7 +778,7 @@ const double* proj_h_device(sipg_mesh* m) {
 // Opt the kernel into its dynamic shared memory and return its resident CTAs per
 // SM, once per (kernel, device): the attribute belongs to the current device.
 template <typename Kern>
-int kernel_setup(Kern kern, size_t smem) {
+int kernel_setup(Kern kern, size_t smem, int threads = kProjWarps * 32) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, int> per_sm;  // (kernel, device)
   int dev = 0;
@@ -800,7 +788,7 @@ int kernel_setup(Kern kern, size_t smem) {
   if (!n) {
     SIPG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int b = 0;
-    SIPG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, kProjWarps * 32, smem));
+    SIPG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, threads, smem));
     n = std::max(b, 1);
   }
   return n;
@@ -904,14 +892,13 @@ void project_host(sipg_mesh* m, int order, double dt, double factor, const doubl
 
 template <int D, int P>
 void launch_pr_rhs(const PrRhsArgs& a, cudaStream_t s) {
-  constexpr size_t smem = pr_rhs_smem_doubles<D, P>() * sizeof(double);
-  static_assert(smem <= 227 * 1024, "pressure rhs shared memory");
-  auto kern = k_pr_rhs<D, P>;
-  const int per_sm = kernel_setup(kern, smem);
-  const int epc = kProjWarps * proj_epw(D, P);  // elements per CTA round
-  const int need = (a.K + epc - 1) / epc;
-  const int grid = std::max(1, std::min(need, per_sm * num_sms()));
-  kern<<<grid, kProjWarps * 32, smem, s>>>(a);
+  using C = PrRhsCfg<D, P>;
+  static_assert(C::smem <= 227 * 1024, "pressure rhs shared memory");
+  const bool pair = ((reinterpret_cast<uintptr_t>(a.velT) | reinterpret_cast<uintptr_t>(a.rhs)) & 15) == 0;
+  auto kern = pair ? k_pr_rhs<D, P, true> : k_pr_rhs<D, P, false>;
+  const int per_sm = kernel_setup(kern, C::smem, C::WARPS * 32);
+  const int grid = std::max(1, std::min((a.K + 7) / 8, per_sm * num_sms()));
+  kern<<<grid, C::WARPS * 32, C::smem, s>>>(a);
   SIPG_CUDA(cudaGetLastError());
   note_launch();
 }
@@ -927,7 +914,7 @@ void pressure_rhs_device(sipg_mesh* m, int order, double dt, double b0, double b
   PrRhsArgs a{};
   a.K = m->K;
   a.geof = m->geof64.as<double>();
-  a.mats = proj_mats(m->dim, order).blob.as<double>();
+  a.ops = proj_mats(m->dim, order).rhs_ops.as<double>();
   a.dt = dt;
   a.b0 = b0;
   a.b1 = b1;
