@@ -13,21 +13,20 @@
 // unpreconditioned in 2D (ins_proj_cg_2d.h), stopping on the absolute residual
 // (3D |r|_2 < 1e-8, 2D |r|_2^2 < 1e-16) or after 100 iterations.
 //
-// Here the whole sequence is one kernel. A warp owns two elements (one at
-// p = 4 in 3D), a lane per node: it reads velT, grad p, the geometric factors
-// and h once, iterates both elements' CG in registers and shared memory, and
-// writes velTT once. The solve is bound by shared-memory bandwidth (the
-// reference-element matrices are read from shared memory at every product), so
-// the kernel minimises shared traffic per multiply-add: each matrix entry read
-// serves both elements of the warp, matrix entries and vector values are read
-// in 16-byte pairs (column pairs of Np rows; vectors padded to an even length
-// with zeros), and in 3D the mass term J M p of the operator is carried by the
-// recursion J M p_new = r_new + beta J M p (since J M z = r for z = (1/J) M^-1 r)
-// instead of three mass products per iteration. Dot products are xor-butterfly
-// warp reductions, which leave the same bits in every lane, so the stopping
-// tests are warp-uniform; an element that has stopped idles while the other
-// finishes. The counters the reference accumulates (cells, converged cells,
-// iterations) are summed per warp and added once per warp.
+// Here the whole sequence is one kernel: it reads velT, grad p, the geometric factors
+// and h once, iterates the elements' CG on chip and writes velTT once. In 3D eight
+// elements per warp run on the FP64 tensor cores (k_proj_tc); the mass term J M p of the
+// operator is carried by the recursion J M p_new = r_new + beta J M p (since J M z = r
+// for z = (1/J) M^-1 r) instead of mass products. In 2D, where the unpreconditioned
+// iteration takes tens of steps that differ between elements, a warp owns two elements,
+// a lane per node (k_proj_cg): bound by shared-memory bandwidth (the matrices are read
+// at every product), it minimises the reads per multiply-add: each matrix entry serves
+// both elements, entries and vector values are read in 16-byte pairs (column pairs of Np
+// rows; vectors padded to an even length with zeros). Dot products are xor-butterfly
+// reductions, which leave the same bits in every lane, so the stopping tests are uniform;
+// an element that has stopped idles while the others of its warp finish. The counters the
+// reference accumulates (cells, converged cells, iterations) are summed per warp and
+// added once per warp.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,11 +53,10 @@ __host__ __device__ constexpr int proj_np(int D, int P) {
 }
 // Np rounded up to even: vectors and matrix columns are read in pairs.
 __host__ __device__ constexpr int proj_npe(int D, int P) { return (proj_np(D, P) + 1) & ~1; }
-// Elements per warp: two while a node per lane covers the element, else one.
-__host__ __device__ constexpr int proj_epw(int D, int P) { return proj_np(D, P) <= 32 ? 2 : 1; }
-// Matrices in the blob: D_k for products (D), D_k^T for products (D), M, and M^-1 in 3D;
-// each stored as Npe/2 column pairs of Np rows: A(i, 2q + t) at (q * Np + i) * 2 + t.
-__host__ __device__ constexpr int proj_nmat(int D) { return 2 * D + 1 + (D == 3 ? 1 : 0); }
+constexpr int kProjEpw = 2;  // elements per warp (2D: a node per lane covers the element)
+// Matrices in the 2D blob: D_k for products (D), D_k^T for products (D), M; each stored as
+// Npe/2 column pairs of Np rows: A(i, 2q + t) at (q * Np + i) * 2 + t.
+__host__ __device__ constexpr int proj_nmat(int D) { return 2 * D + 1; }
 template <int D, int P>
 __host__ __device__ constexpr int proj_mat_doubles() { return proj_np(D, P) * proj_npe(D, P); }
 __host__ __device__ constexpr int proj_nfp(int D, int P) { return D == 2 ? P + 1 : (P + 1) * (P + 2) / 2; }
@@ -74,7 +72,7 @@ __host__ __device__ constexpr int proj_blob_doubles() {
 template <int D, int P>
 __host__ __device__ constexpr int proj_warp_doubles() {
   // per element: A (D x Npe), B (D x Npe), C (Npe), face jumps ((D + 1) x Nfpe)
-  return proj_epw(D, P) * ((2 * D + 1) * proj_npe(D, P) + (D + 1) * proj_nfpe(D, P));
+  return kProjEpw * ((2 * D + 1) * proj_npe(D, P) + (D + 1) * proj_nfpe(D, P));
 }
 template <int D, int P>
 __host__ __device__ constexpr int proj_smem_doubles() {
@@ -127,16 +125,15 @@ __device__ __forceinline__ void mat_vec(const double* __restrict__ A, const doub
   for (int e = 0; e < E; ++e) y[e] += y1[e];
 }
 
-// E elements per warp (a lane per node, NPL nodes per lane). GRAD: the pressure
+// 2D: E elements per warp (a lane per node). GRAD: the pressure
 // gradient is computed here from the pressure (central flux, then / rho) instead
 // of being read.
-template <int D, int P, bool GRAD>
+template <int P, bool GRAD>
 __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
-  constexpr int NP = proj_np(D, P), NPE = proj_npe(D, P), NPL = (NP + 31) / 32, NG = D == 3 ? 10 : 5;
+  constexpr int D = 2, NP = proj_np(D, P), NPE = proj_npe(D, P), NPL = (NP + 31) / 32, NG = 5;
   constexpr int NF = D + 1, NFP = proj_nfp(D, P), NFPE = proj_nfpe(D, P);
-  constexpr int E = proj_epw(D, P), MAT = proj_mat_doubles<D, P>();
+  constexpr int E = kProjEpw, MAT = proj_mat_doubles<D, P>();
   constexpr int WB = proj_warp_doubles<D, P>();  // per-warp buffer
-  constexpr bool kPre = D == 3;
   const int K = a.K;
   const double* __restrict__ geof = a.geof;
   const double* __restrict__ hK = a.hK;
@@ -147,7 +144,6 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
   const double* sD = sm;                  // D_k, k < D
   const double* sDt = sm + D * MAT;       // D_k^T
   const double* sM = sm + 2 * D * MAT;    // M
-  const double* sMi = sm + (2 * D + 1) * MAT;  // M^-1 (3D)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double* sL = sm + proj_nmat(D) * MAT;  // LIFT, per face an Np x Nfpe pair block
   double* sA = sm + proj_blob_doubles<D, P>() + warp * WB;  // [E][D][NPE]
@@ -160,11 +156,11 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
   __syncthreads();
 
   const size_t n = (size_t)K * NP;
-  const double tol = kPre ? 1e-8 : 1e-16;
+  const double tol = 1e-16;  // of |r|^2
   unsigned long long n_conv = 0, n_iter = 0;
 
   for (int e0 = (blockIdx.x * kProjWarps + warp) * E; e0 < K; e0 += gridDim.x * kProjWarps * E) {
-    double G[E][3][3], J[E], pen[E], inv_J[E];
+    double G[E][D][D], J[E], pen[E];
     bool valid[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -172,30 +168,16 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
       valid[e] = el < K;
       const int ec = valid[e] ? el : e0;
       const double* g = geof + (size_t)ec * NG;
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) G[e][k][c] = 0.0;
-      if (D == 3) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) G[e][k][c] = __ldg(g + k * 3 + c);
-        J[e] = __ldg(g + 9);
-      } else {
-        G[e][0][0] = __ldg(g + 0); G[e][0][1] = __ldg(g + 1);
-        G[e][1][0] = __ldg(g + 2); G[e][1][1] = __ldg(g + 3);
-        J[e] = __ldg(g + 4);
-      }
+      G[e][0][0] = __ldg(g + 0); G[e][0][1] = __ldg(g + 1);
+      G[e][1][0] = __ldg(g + 2); G[e][1][1] = __ldg(g + 3);
+      J[e] = __ldg(g + 4);
       pen[e] = factor * (__ldg(hK + ec) / ((double)P + 1.0));
-      inv_J[e] = 1.0 / J[e];
     }
 
-    double x[E][D][NPL], r[E][D][NPL], z[E][D][NPL], p[E][D][NPL], ap[E][D][NPL], q[E][D][NPL];
+    double x[E][D][NPL], r[E][D][NPL], p[E][D][NPL], ap[E][D][NPL], q[E][D][NPL];
 
-    // ap = pen * G^T D^T (J M (D G v)) + mass, v read from sB; mass = J M v when
-    // explicit_mass (also returned in q), else the q carried by the caller.
-    auto apply = [&](bool explicit_mass) {
+    // q = J M v, ap = pen * G^T D^T (J M (D G v)) + q, v read from sB
+    auto apply = [&] {
 #pragma unroll
       for (int u = 0; u < NPL; ++u) {  // (G v)_k -> sA
         const int i = lane + 32 * u;
@@ -248,14 +230,13 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
           double w[D][E];
 #pragma unroll
           for (int k = 0; k < D; ++k) mat_vec<NP, NPE, E>(sDt + k * MAT, sA, D * NPE, i, w[k]);
-          if (explicit_mass)
 #pragma unroll
-            for (int c = 0; c < D; ++c) {
-              double s[E];
-              mat_vec<NP, NPE, E>(sM, sB + c * NPE, D * NPE, i, s);
+          for (int c = 0; c < D; ++c) {
+            double s[E];
+            mat_vec<NP, NPE, E>(sM, sB + c * NPE, D * NPE, i, s);
 #pragma unroll
-              for (int e = 0; e < E; ++e) q[e][c][u] = J[e] * s[e];
-            }
+            for (int e = 0; e < E; ++e) q[e][c][u] = J[e] * s[e];
+          }
 #pragma unroll
           for (int e = 0; e < E; ++e)
 #pragma unroll
@@ -286,34 +267,17 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
       }
       __syncwarp();
     };
-    // z = (1/J) M^-1 r (3D) or r (2D); rz = r . z per element (warp sums)
-    auto precondition = [&](double (&rz)[E]) {
-      if (kPre) stage(r);
+    // r . r per element
+    auto norms = [&](double (&rr)[E]) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) rz[e] = 0.0;
+      for (int e = 0; e < E; ++e) {
+        double v = 0.0;
 #pragma unroll
-      for (int u = 0; u < NPL; ++u) {
-        const int i = lane + 32 * u;
+        for (int u = 0; u < NPL; ++u)
 #pragma unroll
-        for (int c = 0; c < D; ++c) {
-          double s[E];
-          if (kPre && i < NP) {
-            mat_vec<NP, NPE, E>(sMi, sB + c * NPE, D * NPE, i, s);
-#pragma unroll
-            for (int e = 0; e < E; ++e) s[e] = inv_J[e] * s[e];
-          } else {
-#pragma unroll
-            for (int e = 0; e < E; ++e) s[e] = i < NP ? r[e][c][u] : 0.0;
-          }
-#pragma unroll
-          for (int e = 0; e < E; ++e) {
-            z[e][c][u] = s[e];
-            rz[e] += r[e][c][u] * s[e];
-          }
-        }
+          for (int c = 0; c < D; ++c) v += r[e][c][u] * r[e][c][u];
+        rr[e] = warp_sum(v);
       }
-#pragma unroll
-      for (int e = 0; e < E; ++e) rz[e] = warp_sum(rz[e]);
     };
 
     // grad p: read, or (GRAD) computed with the central flux and divided by rho
@@ -367,16 +331,9 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
 #pragma unroll
               for (int k = 0; k < D; ++k) g += G[e][k][d] * dr[k][e];
               // fscale n of each face (the unnormalised outward normal)
-              if (D == 3) {
-                g += -G[e][2][d] * lf[0][e];
-                g += -G[e][1][d] * lf[1][e];
-                g += ((G[e][0][d] + G[e][1][d]) + G[e][2][d]) * lf[2][e];
-                g += -G[e][0][d] * lf[3][e];
-              } else {
-                g += -G[e][1][d] * lf[0][e];
-                g += (G[e][0][d] + G[e][1][d]) * lf[1][e];
-                g += -G[e][0][d] * lf[2][e];
-              }
+              g += -G[e][1][d] * lf[0][e];
+              g += (G[e][0][d] + G[e][1][d]) * lf[1][e];
+              g += -G[e][0][d] * lf[2][e];
               gp[e][d][u] = g * rinv;
             }
           }
@@ -411,43 +368,31 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
         }
       }
     stage(x);
-    apply(true);  // q = J M x is the right-hand side, ap = A x
+    apply();  // q = J M x is the right-hand side, ap = A x
     double res[E], rz[E];
     bool active[E];
     int it[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      double s = 0.0;
-#pragma unroll
-      for (int u = 0; u < NPL; ++u)
-#pragma unroll
-        for (int c = 0; c < D; ++c) {
-          r[e][c][u] = q[e][c][u] - ap[e][c][u];
-          s += r[e][c][u] * r[e][c][u];
-        }
-      s = warp_sum(s);
-      res[e] = kPre ? sqrt(s) : s;
-      it[e] = 0;
-      active[e] = valid[e] && res[e] > tol;
-    }
-    precondition(rz);
 #pragma unroll
     for (int e = 0; e < E; ++e)
 #pragma unroll
       for (int u = 0; u < NPL; ++u)
 #pragma unroll
         for (int c = 0; c < D; ++c) {
-          p[e][c][u] = z[e][c][u];
-          q[e][c][u] = r[e][c][u];  // J M p = J M z = r (3D)
+          r[e][c][u] = q[e][c][u] - ap[e][c][u];
+          p[e][c][u] = r[e][c][u];
         }
-
+    norms(rz);
     bool any = false;
 #pragma unroll
-    for (int e = 0; e < E; ++e) any |= active[e];
+    for (int e = 0; e < E; ++e) {
+      res[e] = rz[e];
+      it[e] = 0;
+      active[e] = valid[e] && res[e] > tol;
+      any |= active[e];
+    }
     while (any) {
       stage(p);
-      apply(!kPre);  // 3D: J M p is carried in q
-      double pap[E];
+      apply();
 #pragma unroll
       for (int e = 0; e < E; ++e) {
         double s = 0.0;
@@ -455,43 +400,32 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
         for (int u = 0; u < NPL; ++u)
 #pragma unroll
           for (int c = 0; c < D; ++c) s += p[e][c][u] * ap[e][c][u];
-        pap[e] = warp_sum(s);
-      }
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const double alpha = rz[e] / pap[e];
-        double s = 0.0;
-#pragma unroll
-        for (int u = 0; u < NPL; ++u)
-#pragma unroll
-          for (int c = 0; c < D; ++c) {
-            if (active[e]) {
-              x[e][c][u] += alpha * p[e][c][u];
-              r[e][c][u] -= alpha * ap[e][c][u];
-            }
-            s += r[e][c][u] * r[e][c][u];
-          }
-        s = warp_sum(s);
-        if (active[e]) {
-          res[e] = kPre ? sqrt(s) : s;
-          if (res[e] < tol) active[e] = false;  // the reference's break: not counted
-        }
-      }
-      double rz_new[E];
-      precondition(rz_new);
-      any = false;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        if (active[e]) {
-          const double beta = rz_new[e] / rz[e];
-          rz[e] = rz_new[e];
+        const double alpha = rz[e] / warp_sum(s);
+        if (active[e])
 #pragma unroll
           for (int u = 0; u < NPL; ++u)
 #pragma unroll
             for (int c = 0; c < D; ++c) {
-              p[e][c][u] = z[e][c][u] + beta * p[e][c][u];
-              if (kPre) q[e][c][u] = r[e][c][u] + beta * q[e][c][u];
+              x[e][c][u] += alpha * p[e][c][u];
+              r[e][c][u] -= alpha * ap[e][c][u];
             }
+      }
+      double rr[E];
+      norms(rr);
+      any = false;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        if (active[e]) {
+          res[e] = rr[e];
+          if (res[e] < tol) active[e] = false;  // the reference's break: not counted
+        }
+        if (active[e]) {
+          const double beta = rr[e] / rz[e];
+          rz[e] = rr[e];
+#pragma unroll
+          for (int u = 0; u < NPL; ++u)
+#pragma unroll
+            for (int c = 0; c < D; ++c) p[e][c][u] = r[e][c][u] + beta * p[e][c][u];
           ++it[e];
           active[e] = res[e] > tol && it[e] < kProjMaxIter;
         }
@@ -518,6 +452,315 @@ __global__ void __launch_bounds__(kProjWarps * 32) k_proj_cg(const ProjArgs a) {
   }
 }
 
+
+// The 3D projection on the FP64 tensor cores, eight elements per warp (the M dimension of the MMA):
+// the same iteration as k_proj_cg with every product batched over the warp's elements, a quad of
+// lanes per element. (G v)_k feeds the divergence product and its result, d, the product with
+// D_k^T M (one operand) straight from fragment registers; x and r stay in registers, p and the
+// carried J M p in a lane-private part of shared memory. The initial residual is -pen J G^T (D^T M d)
+// itself, without the mass product on both sides of b - A x. An element that has stopped idles until
+// its warp's last one has. GRAD: grad p = G^T (D_k pr + s_fk LIFT_f (p+ - p-) / 2), the faces'
+// unnormalised normals being sums of the rows of G (s_fk = 0, +-1), divided by rho.
+// Against k_proj_cg, which reads each matrix entry from shared memory for two elements:
+// p = 1 / 2 / 3 at 32^3 x 6 tets 361 / 857 / 1,430 -> 44 / 162 / 364 us, p = 4 at 24^3 x 6
+// 3,421 -> 667 us (about 40 % of the FP64 pipe's rate counting issued MMAs; one or two
+// iterations per element, 12 warps per SM).
+template <int P>
+struct ProjTc {
+  using X = Tc<double, 3, P>;
+  static constexpr int WARPS = P < 4 ? 12 : 6, US = X::NP | 1;
+  static constexpr int NN = X::NT * X::NT * X::BLK;
+  static constexpr int OD = 0, OT = 3 * NN, OM = 6 * NN, OL = 7 * NN;  // D_k, D_k^T M, M^-1, LIFT
+  static constexpr int NB = OL + X::FT * X::NT * X::BLK;
+  static constexpr int NV = 3 * X::NT * 2;                               // values per lane of a vector
+  static constexpr int WB = 2 * NV * 32 > 8 * US ? 2 * NV * 32 : 8 * US; // p and q, or the staged pressure
+  static constexpr int NTAB = 4 * 6 * X::TRP;
+  static constexpr size_t smem = (size_t)(NB + WARPS * WB) * sizeof(double) + NTAB;
+};
+
+__device__ __forceinline__ double quad_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+template <int P, bool GRAD, bool PAIR>
+__global__ void __launch_bounds__(ProjTc<P>::WARPS * 32, 1) k_proj_tc(const ProjArgs a, const double* __restrict__ ops) {
+  using C = ProjTc<P>;
+  using X = typename C::X;
+  using F = Frag<double>;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = 4, NT = X::NT, FT = X::FT, TRP = X::TRP, US = C::US, NV = C::NV;
+  extern __shared__ __align__(16) double sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double* W = sm + C::NB + warp * C::WB;
+  double* sp = W + lane;             // p: value i at sp[32 i]
+  double* sq = W + NV * 32 + lane;   // J M p
+  uint8_t* tab = reinterpret_cast<uint8_t*>(sm + C::NB + C::WARPS * C::WB);
+  copy_blob(sm, ops, C::NB * (int)sizeof(double));
+  for (int i = threadIdx.x; i < C::NTAB; i += blockDim.x) {
+    const int gf = i / (6 * TRP), sg = i / TRP % 6, j = min(i % TRP, NFP - 1);
+    tab[i] = (uint8_t)a.itab[gf * NFP + a.itab[NF * NFP + sg * NFP + j]];
+  }
+  cp_wait_all();
+  __syncthreads();
+  const size_t n = (size_t)a.K * NP;
+  const int ntiles = (a.K + 7) / 8;
+  unsigned long long n_conv = 0, n_iter = 0;
+  for (int tile = warp * gridDim.x + blockIdx.x; tile < ntiles; tile += gridDim.x * C::WARPS) {
+    const int e0 = tile * 8, ne = min(8, a.K - e0), e = min(e0 + g, a.K - 1);
+    const bool valid = g < ne;
+    double G[3][3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) G[k / 3][k % 3] = a.geof[(size_t)e * 10 + k];
+    const double J = a.geof[(size_t)e * 10 + 9], invJ = 1.0 / J;
+    const double penJ = a.factor * (a.hK[e] / ((double)P + 1.0)) * J;
+    double x[3][NT][1][2], r[3][NT][1][2];
+    // x = velT - dt grad p
+#pragma unroll
+    for (int c = 0; c < 3; ++c) load_nodes<double, 3, P, PAIR>(a.velT + c * n, e0, ne, x[c], g, t);
+    if (GRAD) {
+      double pr[NT][1][2], dr[3][NT][1][2];
+      load_nodes<double, 3, P, PAIR>(a.pr, e0, ne, pr, g, t);
+      __syncwarp();
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          const int m = frag_node<double, 3, P>(nt, ci, t);
+          if (m < NP) W[g * US + m] = pr[nt][0][ci];
+        }
+      const int4 nb4 = *reinterpret_cast<const int4*>(a.nbr + (size_t)e * NF);
+      const uint32_t code = a.fcode[e];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) dr[k][nt][0][0] = dr[k][nt][0][1] = 0.0;
+#pragma unroll
+      for (int kb = 0; kb < NT; ++kb)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            mma_nodes<double, 3, P>(dr[k][nt], pr[kb], ldb(sm + C::OD, (k * NT + kb) * NT + nt, lane), kb);
+      __syncwarp();
+#pragma unroll
+      for (int fb = 0; fb < FT; ++fb) {
+        const int k0 = 8 * fb + 2 * t, f = k0 / TRP, j0 = k0 % TRP;
+        const int nb = f == 0 ? nb4.x : f == 1 ? nb4.y : f == 2 ? nb4.z : nb4.w;
+        const unsigned cf = (code >> (8 * f)) & 255u;
+        const uint8_t* pos = tab + ((cf & 3u) * 6 + (cf >> 2)) * TRP + j0;
+        double jv[2] = {0.0, 0.0};
+        if (nb >= 0)  // boundary faces add nothing
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci)
+            if (j0 + ci < NFP)
+              jv[ci] = 0.5 * (a.pr[(size_t)nb * NP + pos[ci]] - W[g * US + a.itab[f * NFP + j0 + ci]]);
+        const int flo = 8 * fb / TRP, fhi = (8 * fb + 6) / TRP;  // faces of the block
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          // s_fk: face 0: -(row 2), face 1: -(row 1), face 2: rows 0 + 1 + 2, face 3: -(row 0)
+          const bool any = (flo <= 2 && fhi >= 2) || (k == 0 && fhi >= 3) || (k == 1 && flo <= 1 && fhi >= 1) ||
+                           (k == 2 && flo <= 0);
+          if (!any) continue;
+          const double sk = f == 2 ? 1.0 : ((f == 0 && k == 2) || (f == 1 && k == 1) || (f == 3 && k == 0)) ? -1.0 : 0.0;
+          const double fa[1][2] = {{sk * jv[0], sk * jv[1]}};
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) F::mma(dr[k][nt], fa, ldb(sm + C::OL, fb * NT + nt, lane));
+        }
+      }
+      double ri[NT][1][2];
+      if (a.rho) load_nodes<double, 3, P, PAIR>(a.rho, e0, ne, ri, g, t);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          const bool in = valid && frag_node<double, 3, P>(nt, ci, t) < NP;
+          const double rinv = in ? (a.rho ? 1.0 / ri[nt][0][ci] : 1.0) : 0.0;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double gp = rinv * (G[0][c] * dr[0][nt][0][ci] + G[1][c] * dr[1][nt][0][ci] + G[2][c] * dr[2][nt][0][ci]);
+            x[c][nt][0][ci] -= a.dt * gp;
+          }
+        }
+      __syncwarp();  // the staged pressure has been read: W holds p and q from here on
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double gp[NT][1][2];
+        load_nodes<double, 3, P, PAIR>(a.dp + c * n, e0, ne, gp, g, t);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci) x[c][nt][0][ci] -= a.dt * gp[nt][0][ci];
+      }
+    }
+    // w_c = pen J sum_k G_kc D_k^T M (sum_k D_k (G v)_k), v(c, nt, ci) read through `v`
+    double w[3][NT][1][2];
+    auto penalty = [&](auto&& v) {
+      double d[NT][1][2];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) d[nt][0][0] = d[nt][0][1] = 0.0;
+#pragma unroll
+      for (int kb = 0; kb < NT; ++kb) {
+        double vc[3][2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci) vc[c][ci] = v(c, kb, ci);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          double gv[1][2];
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci) gv[0][ci] = G[k][0] * vc[0][ci] + G[k][1] * vc[1][ci] + G[k][2] * vc[2][ci];
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            mma_nodes<double, 3, P>(d[nt], gv, ldb(sm + C::OD, (k * NT + kb) * NT + nt, lane), kb);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        double wk[3][1][2];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          wk[k][0][0] = wk[k][0][1] = 0.0;
+#pragma unroll
+          for (int kb = 0; kb < NT; ++kb)
+            mma_nodes<double, 3, P>(wk[k], d[kb], ldb(sm + C::OT, (k * NT + kb) * NT + nt, lane), kb);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci)
+            w[c][nt][0][ci] = penJ * (G[0][c] * wk[0][0][ci] + G[1][c] * wk[1][0][ci] + G[2][c] * wk[2][0][ci]);
+      }
+    };
+    // z = (1/J) M^-1 r into w; returns r . z of the element
+    auto precondition = [&] {
+      double rz = 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+          w[c][nt][0][0] = w[c][nt][0][1] = 0.0;
+#pragma unroll
+          for (int kb = 0; kb < NT; ++kb)
+            mma_nodes<double, 3, P>(w[c][nt], r[c][kb], ldb(sm + C::OM, kb * NT + nt, lane), kb);
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci) {
+            w[c][nt][0][ci] *= invJ;
+            rz += r[c][nt][0][ci] * w[c][nt][0][ci];
+          }
+        }
+      return quad_sum(rz);
+    };
+    penalty([&](int c, int nt, int ci) { return x[c][nt][0][ci]; });
+    double rr = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int ci = 0; ci < 2; ++ci) {
+          r[c][nt][0][ci] = -w[c][nt][0][ci];
+          rr += r[c][nt][0][ci] * r[c][nt][0][ci];
+        }
+    const double tol = 1e-8;
+    double res = sqrt(quad_sum(rr));
+    int it = 0;
+    bool active = valid && res > tol;
+    double rz = 0.0;
+    if (__any_sync(0xffffffffu, active)) {
+      rz = precondition();
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = i / (2 * NT), nt = i / 2 % NT, ci = i % 2;
+        sp[32 * i] = w[c][nt][0][ci];
+        sq[32 * i] = r[c][nt][0][ci];  // J M p = J M z = r
+      }
+    }
+    while (__any_sync(0xffffffffu, active)) {
+      penalty([&](int c, int nt, int ci) { return sp[32 * ((c * NT + nt) * 2 + ci)]; });
+      double pap = 0.0;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = i / (2 * NT), nt = i / 2 % NT, ci = i % 2;
+        w[c][nt][0][ci] += sq[32 * i];
+        pap += sp[32 * i] * w[c][nt][0][ci];
+      }
+      const double alpha = rz / quad_sum(pap);
+      rr = 0.0;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = i / (2 * NT), nt = i / 2 % NT, ci = i % 2;
+        if (active) {
+          x[c][nt][0][ci] += alpha * sp[32 * i];
+          r[c][nt][0][ci] -= alpha * w[c][nt][0][ci];
+        }
+        rr += r[c][nt][0][ci] * r[c][nt][0][ci];
+      }
+      rr = quad_sum(rr);
+      if (active) {
+        res = sqrt(rr);
+        if (res < tol) active = false;  // the reference's break: not counted
+      }
+      if (!__any_sync(0xffffffffu, active)) break;
+      const double rz_new = precondition();
+      if (active) {
+        const double beta = rz_new / rz;
+        rz = rz_new;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const int c = i / (2 * NT), nt = i / 2 % NT, ci = i % 2;
+          sp[32 * i] = w[c][nt][0][ci] + beta * sp[32 * i];
+          sq[32 * i] = r[c][nt][0][ci] + beta * sq[32 * i];
+        }
+        ++it;
+        active = res > tol && it < kProjMaxIter;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) store_nodes<double, 3, P, PAIR>(a.velTT + c * n, e0, ne, x[c], g, t);
+    if (valid && t == 0) {
+      n_iter += (unsigned long long)it;
+      n_conv += (it < kProjMaxIter && !isnan(res)) ? 1ull : 0ull;
+    }
+  }
+  if (a.stats) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      n_conv += __shfl_xor_sync(0xffffffffu, n_conv, o);
+      n_iter += __shfl_xor_sync(0xffffffffu, n_iter, o);
+    }
+    if (lane == 0) {
+      atomicAdd(a.stats + 0, n_conv);
+      atomicAdd(a.stats + 1, n_iter);
+    }
+  }
+}
+
+template <int P>
+std::vector<double> proj_operands(const RefElement& r) {
+  using C = ProjTc<P>;
+  using X = typename C::X;
+  constexpr int NP = X::NP, NFP = X::NFP, NF = 4, NT = X::NT;
+  std::vector<double> out(C::NB, 0.0);
+  const double* Dk[3] = {r.Dr.data(), r.Ds.data(), r.Dt.data()};
+  auto col = [](int m) { return tc_node_col<double, 3, P>(m); };
+  for (int m = 0; m < NP; ++m)
+    for (int j = 0; j < NP; ++j) {
+      for (int k = 0; k < 3; ++k) {
+        out[C::OD + k * C::NN + tc_slot(NT, col(j), col(m))] = Dk[k][(size_t)m * NP + j];
+        double v = 0.0;
+        for (int i = 0; i < NP; ++i) v += Dk[k][(size_t)i * NP + m] * r.M[(size_t)i * NP + j];
+        out[C::OT + k * C::NN + tc_slot(NT, col(j), col(m))] = v;  // (D_k^T M)[m][j]
+      }
+      out[C::OM + tc_slot(NT, col(j), col(m))] = r.Minv[(size_t)m * NP + j];
+    }
+  for (int f = 0; f < NF; ++f)
+    for (int j = 0; j < NFP; ++j)
+      for (int m = 0; m < NP; ++m)
+        out[C::OL + tc_slot(NT, f * X::TRP + j, col(m))] = r.LIFT[(size_t)m * NF * NFP + f * NFP + j];
+  return out;
+}
 
 // Right-hand side of the pressure solve, eight elements per warp on the FP64 tensor cores:
 //   rhs = J M ( -(div_c velT) / dt + LIFT dPdN_new ),  dPdN_new = b0 dPdN + b1 dPdN_old,
@@ -702,9 +945,9 @@ std::vector<double> pr_rhs_operands(int dim, int order, const RefElement& r) {
 
 // Reference-element matrices in the kernel's layouts, per (device, dim, order).
 struct ProjMats {
-  DevBuf blob;
+  DevBuf blob;     // 2D projection (k_proj_cg)
+  DevBuf proj_ops; // 3D projection on the tensor cores (ProjTc)
   DevBuf rhs_ops;  // pressure right-hand side (PrRhsArgs::ops)
-  int Np = 0;
 };
 
 const ProjMats& proj_mats(int dim, int order) {
@@ -717,33 +960,36 @@ const ProjMats& proj_mats(int dim, int order) {
   if (slot) return *slot;
   const DevRef& dr = dev_ref(dim, order);
   const RefElement& ref = dr.ref;
-  const int Np = ref.Np, Npe = (Np + 1) & ~1;
-  const size_t MAT = (size_t)Np * Npe;
-  const int Nfpe0 = (ref.Nfp + 1) & ~1;
-  std::vector<double> b((size_t)proj_nmat(dim) * MAT + (size_t)(dim + 1) * Np * Nfpe0, 0.0);  // pads stay zero
-  // A(i, j) of matrix m at m * MAT + ((j / 2) * Np + i) * 2 + j % 2; rm: row-major source
-  auto put = [&](int m, const std::vector<double>& rm, bool transpose) {
-    for (int i = 0; i < Np; ++i)
-      for (int j = 0; j < Np; ++j)
-        b[m * MAT + ((size_t)(j / 2) * Np + i) * 2 + j % 2] = transpose ? rm[(size_t)j * Np + i] : rm[(size_t)i * Np + j];
-  };
-  const std::vector<double>* Dk[3] = {&ref.Dr, &ref.Ds, &ref.Dt};
-  for (int k = 0; k < dim; ++k) {
-    put(k, *Dk[k], false);
-    put(dim + k, *Dk[k], true);
-  }
-  put(2 * dim, ref.M, false);
-  if (dim == 3) put(2 * dim + 1, ref.Minv, false);
-  const int Nf = dim + 1, Nfp = ref.Nfp, Nfpe = (Nfp + 1) & ~1;
-  double* lift = b.data() + (size_t)proj_nmat(dim) * MAT;
-  for (int f = 0; f < Nf; ++f)
-    for (int i = 0; i < Np; ++i)
-      for (int k = 0; k < Nfp; ++k)
-        lift[(size_t)f * Np * Nfpe + ((size_t)(k / 2) * Np + i) * 2 + k % 2] = ref.LIFT[(size_t)i * Nf * Nfp + f * Nfp + k];
   auto pm = std::make_unique<ProjMats>();
-  pm->Np = Np;
-  pm->blob = DevBuf(b.size() * sizeof(double));
-  pm->blob.upload(b.data(), b.size() * sizeof(double));
+  if (dim == 2) {  // k_proj_cg's matrices
+    const int Np = ref.Np, Npe = (Np + 1) & ~1, Nf = 3, Nfp = ref.Nfp, Nfpe = (Nfp + 1) & ~1;
+    const size_t MAT = (size_t)Np * Npe;
+    std::vector<double> b((size_t)proj_nmat(2) * MAT + (size_t)Nf * Np * Nfpe, 0.0);  // pads stay zero
+    // A(i, j) of matrix m at m * MAT + ((j / 2) * Np + i) * 2 + j % 2; rm: row-major source
+    auto put = [&](int m, const std::vector<double>& rm, bool transpose) {
+      for (int i = 0; i < Np; ++i)
+        for (int j = 0; j < Np; ++j)
+          b[m * MAT + ((size_t)(j / 2) * Np + i) * 2 + j % 2] = transpose ? rm[(size_t)j * Np + i] : rm[(size_t)i * Np + j];
+    };
+    put(0, ref.Dr, false);
+    put(1, ref.Ds, false);
+    put(2, ref.Dr, true);
+    put(3, ref.Ds, true);
+    put(4, ref.M, false);
+    double* lift = b.data() + (size_t)proj_nmat(2) * MAT;
+    for (int f = 0; f < Nf; ++f)
+      for (int i = 0; i < Np; ++i)
+        for (int k = 0; k < Nfp; ++k)
+          lift[(size_t)f * Np * Nfpe + ((size_t)(k / 2) * Np + i) * 2 + k % 2] = ref.LIFT[(size_t)i * Nf * Nfp + f * Nfp + k];
+    pm->blob = DevBuf(b.size() * sizeof(double));
+    pm->blob.upload(b.data(), b.size() * sizeof(double));
+  }
+  if (dim == 3) {
+    const std::vector<double> po = order == 1 ? proj_operands<1>(ref) : order == 2 ? proj_operands<2>(ref)
+                                   : order == 3 ? proj_operands<3>(ref) : proj_operands<4>(ref);
+    pm->proj_ops = DevBuf(po.size() * sizeof(double));
+    pm->proj_ops.upload(po.data(), po.size() * sizeof(double));
+  }
   const std::vector<double> ro = pr_rhs_operands(dim, order, ref);
   pm->rhs_ops = DevBuf(ro.size() * sizeof(double));
   pm->rhs_ops.upload(ro.data(), ro.size() * sizeof(double));
@@ -794,13 +1040,28 @@ int kernel_setup(Kern kern, size_t smem, int threads = kProjWarps * 32) {
   return n;
 }
 
-template <int D, int P, bool GRAD>
+template <int P, bool GRAD>
+void launch_proj_tc(const ProjArgs& a, const double* ops, cudaStream_t s) {
+  using C = ProjTc<P>;
+  static_assert(C::smem <= 227 * 1024, "projection shared memory");
+  bool pair = true;
+  for (const double* p : {a.dp, a.pr, a.rho, a.velT, (const double*)a.velTT})
+    pair = pair && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+  auto kern = pair ? k_proj_tc<P, GRAD, true> : k_proj_tc<P, GRAD, false>;
+  const int per_sm = kernel_setup(kern, C::smem, C::WARPS * 32);
+  const int grid = std::max(1, std::min((a.K + 7) / 8, per_sm * num_sms()));
+  kern<<<grid, C::WARPS * 32, C::smem, s>>>(a, ops);
+  SIPG_CUDA(cudaGetLastError());
+  note_launch();
+}
+
+template <int P, bool GRAD>
 void launch_proj(const ProjArgs& a, cudaStream_t s) {
-  constexpr size_t smem = proj_smem_doubles<D, P>() * sizeof(double);
+  constexpr size_t smem = proj_smem_doubles<2, P>() * sizeof(double);
   static_assert(smem <= 227 * 1024, "projection shared memory");
-  auto kern = k_proj_cg<D, P, GRAD>;
+  auto kern = k_proj_cg<P, GRAD>;
   const int per_sm = kernel_setup(kern, smem);
-  const int epc = kProjWarps * proj_epw(D, P);  // elements per CTA round
+  const int epc = kProjWarps * kProjEpw;  // elements per CTA round
   const int need = (a.K + epc - 1) / epc;
   const int grid = std::max(1, std::min(need, per_sm * num_sms()));
   kern<<<grid, kProjWarps * 32, smem, s>>>(a);
@@ -836,20 +1097,22 @@ void project_device(sipg_mesh* m, int order, double dt, double factor, const dou
   a.stats = stats;
   if (stats) SIPG_CUDA(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), s));
   if (m->K == 0) return;
-#define SIPG_PROJ(D, P)                        \
-  (grad ? launch_proj<D, P, true>(a, s) : launch_proj<D, P, false>(a, s))
+  const double* ops = proj_mats(m->dim, order).proj_ops.as<double>();
+#define SIPG_PROJ_TC(P) (grad ? launch_proj_tc<P, true>(a, ops, s) : launch_proj_tc<P, false>(a, ops, s))
+#define SIPG_PROJ(P) (grad ? launch_proj<P, true>(a, s) : launch_proj<P, false>(a, s))
   switch (m->dim * 10 + order) {
-    case 21: SIPG_PROJ(2, 1); break;
-    case 22: SIPG_PROJ(2, 2); break;
-    case 23: SIPG_PROJ(2, 3); break;
-    case 24: SIPG_PROJ(2, 4); break;
-    case 31: SIPG_PROJ(3, 1); break;
-    case 32: SIPG_PROJ(3, 2); break;
-    case 33: SIPG_PROJ(3, 3); break;
-    case 34: SIPG_PROJ(3, 4); break;
+    case 21: SIPG_PROJ(1); break;
+    case 22: SIPG_PROJ(2); break;
+    case 23: SIPG_PROJ(3); break;
+    case 24: SIPG_PROJ(4); break;
+    case 31: SIPG_PROJ_TC(1); break;
+    case 32: SIPG_PROJ_TC(2); break;
+    case 33: SIPG_PROJ_TC(3); break;
+    case 34: SIPG_PROJ_TC(4); break;
     default: throw Error(SIPG_INVALID_ARG, "project_velocity: dimension");
   }
 #undef SIPG_PROJ
+#undef SIPG_PROJ_TC
 }
 
 // The host-buffer variants: inputs and output through device copies kept on the
