@@ -214,23 +214,31 @@ __global__ void k_d2f(float* dst, const double* src, size_t n) {
     dst[i] = (float)src[i];
 }
 
-// One thread per (row r, element e), e fastest: block reads are coalesced and
-// there are Np threads per element row to hide the gather latency.
+// One thread per (RB consecutive rows, element e), e fastest: block reads are coalesced; a thread
+// gathers its element's and neighbours' x once for its RB rows. With small blocks (Np <= 6) one
+// row per thread keeps enough threads to hide the gather latency; with larger ones the gathers,
+// scattered 8-byte loads that every row repeated, bound the kernel (L1 91 % busy).
+// FP64 p = 3, 24^3 x 6 tets: 343 us with one row per thread, 238 / 210 / 225 / 234 with 2 / 4 / 5 /
+// 10 (16,320 B per element: 97 % of the HBM rate); 8^3 x 6: 22.7, 15.6 / 18.9 / 25.0 / 59.8; p = 4,
+// 16^3 x 6: 279 -> 194 with 5; p = 2, 24^3 x 6: 70.7 -> 57.5 with 2; in 2D one row is best.
 // V4: x rows read as one 16-byte load (FP32, Np = 4, x 16-byte aligned).
-template <typename T, int NP, int NF, bool V4 = false>
+template <typename T, int NP, int NF, int RB = 1, bool V4 = false>
 __global__ void __launch_bounds__(256) k_bsr(int K, const T* __restrict__ v, const int* __restrict__ nbr,
                                              const T* __restrict__ x, T* y, T alpha, T beta, const T* c) {
+  static_assert(NP % RB == 0, "row groups");
   pdl_enter();
   const size_t K_ = (size_t)K;
-  const size_t total = K_ * NP;
+  const size_t total = K_ * (NP / RB);
   for (size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x; tid < total; tid += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(tid / K_);
-    const int e = (int)(tid - (size_t)r * K_);
+    const int rg = (int)(tid / K_);
+    const int e = (int)(tid - (size_t)rg * K_), r = rg * RB;
     int ks[NF + 1];
     ks[0] = e;
 #pragma unroll
     for (int f = 0; f < NF; ++f) ks[f + 1] = nbr[(size_t)e * NF + f];
-    T acc = T(0);
+    T acc[RB];
+#pragma unroll
+    for (int q = 0; q < RB; ++q) acc[q] = T(0);
 #pragma unroll
     for (int s = 0; s <= NF; ++s) {
       const int k = ks[s];
@@ -246,11 +254,16 @@ __global__ void __launch_bounds__(256) k_bsr(int K, const T* __restrict__ v, con
         for (int c = 0; c < NP; ++c) xv[c] = xk[c];
       }
 #pragma unroll
-      for (int c = 0; c < NP; ++c) acc += vs[(size_t)c * K_] * xv[c];
+      for (int c = 0; c < NP; ++c)
+#pragma unroll
+        for (int q = 0; q < RB; ++q) acc[q] += vs[(size_t)(q * NP + c) * K_] * xv[c];
     }
-    T o = alpha * acc;
-    if (beta != T(0)) o += beta * c[(size_t)e * NP + r];
-    y[(size_t)e * NP + r] = o;
+#pragma unroll
+    for (int q = 0; q < RB; ++q) {
+      T o = alpha * acc[q];
+      if (beta != T(0)) o += beta * c[(size_t)e * NP + r + q];
+      y[(size_t)e * NP + r + q] = o;
+    }
   }
 }
 
@@ -503,19 +516,23 @@ void bsr_apply(const BsrOp& B, const T* x, T* y, T alpha, T beta, cudaStream_t s
   }
   const T* v = std::is_same<T, double>::value ? (const T*)B.v64.p : (const T*)B.v32.p;
   if (!v) throw Error(SIPG_INVALID_ARG, "assembled blocks missing for this precision");
-  const int g = (int)std::max<size_t>(1, std::min<size_t>(((size_t)B.K * B.Np + 255) / 256, 148 * 32));
+  auto run = [&](auto kern, int rb) {
+    const int g = (int)std::max<size_t>(1, std::min<size_t>(((size_t)B.K * (B.Np / rb) + 255) / 256, 148 * 32));
+    pdl_launch(kern, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
+  };
   const bool v4 = std::is_same<T, float>::value && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  if (B.dim == 3 && B.Np == 4 && v4)
-    pdl_launch(k_bsr<T, 4, 4, true>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 3 && B.Np == 4) pdl_launch(k_bsr<T, 4, 4>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 3 && B.Np == 10) pdl_launch(k_bsr<T, 10, 4>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 2 && B.Np == 3) pdl_launch(k_bsr<T, 3, 3>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 2 && B.Np == 6) pdl_launch(k_bsr<T, 6, 3>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
+  if (B.dim == 3 && B.Np == 4 && v4) run(k_bsr<T, 4, 4, 1, true>, 1);
+  else if (B.dim == 3 && B.Np == 4) run(k_bsr<T, 4, 4>, 1);
+  else if (B.dim == 3 && B.Np == 10) run(k_bsr<T, 10, 4, 2>, 2);
+  else if (B.dim == 2 && B.Np == 3) run(k_bsr<T, 3, 3>, 1);
+  else if (B.dim == 2 && B.Np == 6) run(k_bsr<T, 6, 3>, 1);
   // orders 3 and 4 (the over-integrated operator's blocks)
-  else if (B.dim == 3 && B.Np == 20) pdl_launch(k_bsr<T, 20, 4>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 3 && B.Np == 35) pdl_launch(k_bsr<T, 35, 4>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 2 && B.Np == 10) pdl_launch(k_bsr<T, 10, 3>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
-  else if (B.dim == 2 && B.Np == 15) pdl_launch(k_bsr<T, 15, 3>, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
+  // four rows per thread while that leaves 1024 threads per SM
+  else if (B.dim == 3 && B.Np == 20 && (long long)B.K * 5 >= num_sms() * 1024LL) run(k_bsr<T, 20, 4, 4>, 4);
+  else if (B.dim == 3 && B.Np == 20) run(k_bsr<T, 20, 4, 2>, 2);
+  else if (B.dim == 3 && B.Np == 35) run(k_bsr<T, 35, 4, 5>, 5);
+  else if (B.dim == 2 && B.Np == 10) run(k_bsr<T, 10, 3>, 1);
+  else if (B.dim == 2 && B.Np == 15) run(k_bsr<T, 15, 3>, 1);
   else throw Error(SIPG_INVALID_ARG, "no assembled apply for this element");
   note_launch();
   SIPG_CUDA(cudaGetLastError());
