@@ -9,9 +9,9 @@
 //            simplified Newton x -= s grad s / |grad s|^2 (100 steps, converged when
 //            the step^2 < max(1e-18, 1e-4 h^2)) and kept if converged inside the
 //            element;
-//   nearest  the closest kept sample to every node, by brute force over the samples
-//            staged through shared memory, four nodes per thread (the reference
-//            queries a KD-tree);
+//   nearest  the closest kept sample to every node: a warp of 64 nodes compares them
+//            with the cells' samples whose bounding spheres can hold a closest one (the
+//            reference queries a KD-tree);
 //   newton   from that sample, the Lagrange-multiplier Newton iteration for the
 //            closest point of the zero set of the sample element's polynomial (4 x 4
 //            pivoted solve, steps clamped to h / 2, a fall-back step when the system
@@ -300,49 +300,113 @@ __global__ void __launch_bounds__(kRThreads) k_reinit_sample(ReinitArgs a, int n
   }
 }
 
-// closest kept sample to every node: brute force, the samples staged through shared
-// memory and compared against NPT nodes per thread; ties go to the first sample
-constexpr int kNpt = 4;
-__global__ void __launch_bounds__(kRThreads) k_reinit_nearest(ReinitArgs a, int nkept) {
-  __shared__ double sx[kRThreads], sy[kRThreads], sz[kRThreads];
+// Closest kept sample to every node, a warp per 64 consecutive nodes; ties go to the first sample.
+// Samples come in groups (a cell's, at most 32) with a bounding sphere each, the warp's nodes have
+// one too (centre c, radius R). The group with the least |c - c_g| + r_g gives every node a sample
+// within B, the largest of the nodes' distances to it; groups with |c - c_g| - r_g - R > B hold no
+// closest one. The rest are compared in order, which gives the result of a comparison with all
+// samples. At 24^3 x 6 tets, p = 3 (1.7 M nodes, a sphere): 12.6 ms comparing with all -> 2.3 ms.
+constexpr int kNpt = 2, kGroup = 32;
+struct SampleGroup {
+  double x, y, z, r;  // bounding sphere
+  int first, count;   // kept samples
+};
+
+__global__ void __launch_bounds__(kRThreads) k_reinit_nearest(ReinitArgs a, const SampleGroup* __restrict__ groups,
+                                                              int ngroups) {
+  constexpr int NW = kRThreads / 32;
+  __shared__ double sx[NW][kGroup], sy[NW][kGroup], sz[NW][kGroup];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t n = (size_t)a.K * a.Np;
-  const size_t node0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * kNpt;
-  double px[kNpt], py[kNpt], pz[kNpt], best[kNpt];
+  const size_t node0 = ((size_t)blockIdx.x * NW + warp) * 32 * kNpt + lane;  // then every 32nd
+  if (node0 - lane >= n) return;
+  double p[kNpt][3], best[kNpt];
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   int bi[kNpt];
 #pragma unroll
   for (int q = 0; q < kNpt; ++q) {
-    const size_t node = node0 + q;
-    const bool act = node < n;
-    px[q] = act ? a.xyz[node] : 0.0;
-    py[q] = act ? a.xyz[n + node] : 0.0;
-    pz[q] = act ? a.xyz[2 * n + node] : 0.0;
+    const size_t node = min(node0 + 32 * q, n - 1);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      p[q][d] = a.xyz[d * n + node];
+      lo[d] = fmin(lo[d], p[q][d]);
+      hi[d] = fmax(hi[d], p[q][d]);
+    }
     best[q] = INFINITY;
     bi[q] = -1;
   }
-  for (int s0 = 0; s0 < nkept; s0 += kRThreads) {
-    __syncthreads();
-    const int sidx = s0 + threadIdx.x;
-    sx[threadIdx.x] = sidx < nkept ? a.csamples[(size_t)sidx * 3] : 0.0;
-    sy[threadIdx.x] = sidx < nkept ? a.csamples[(size_t)sidx * 3 + 1] : 0.0;
-    sz[threadIdx.x] = sidx < nkept ? a.csamples[(size_t)sidx * 3 + 2] : 0.0;
-    __syncthreads();
-    const int m = min(kRThreads, nkept - s0);
-    for (int k = 0; k < m; ++k) {
-      const double qx = sx[k], qy = sy[k], qz = sz[k];
+  double c[3], R = 0.0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+    c[d] = 0.5 * (lo[d] + hi[d]);
+    R += 0.25 * (hi[d] - lo[d]) * (hi[d] - lo[d]);
+  }
+  R = sqrt(R);
+  auto dist = [&](const SampleGroup& g) {
+    const double dx = g.x - c[0], dy = g.y - c[1], dz = g.z - c[2];
+    return sqrt(dx * dx + dy * dy + dz * dz);
+  };
+  auto compare = [&](int g) {  // the warp's nodes with a group's samples
+    const int first = groups[g].first, count = groups[g].count;
+    __syncwarp();
+    if (lane < count) {
+      sx[warp][lane] = a.csamples[(size_t)(first + lane) * 3];
+      sy[warp][lane] = a.csamples[(size_t)(first + lane) * 3 + 1];
+      sz[warp][lane] = a.csamples[(size_t)(first + lane) * 3 + 2];
+    }
+    __syncwarp();
+    for (int k = 0; k < count; ++k) {
+      const double qx = sx[warp][k], qy = sy[warp][k], qz = sz[warp][k];
 #pragma unroll
       for (int q = 0; q < kNpt; ++q) {
-        const double dx = qx - px[q], dy = qy - py[q], dz = qz - pz[q];
+        const double dx = qx - p[q][0], dy = qy - p[q][1], dz = qz - p[q][2];
         const double d2 = dx * dx + dy * dy + dz * dz;
         if (d2 < best[q]) {
           best[q] = d2;
-          bi[q] = s0 + k;
+          bi[q] = first + k;
         }
       }
+    }
+  };
+  // the group nearest by its bound, and B from it
+  double ub = INFINITY;
+  int gb = 0;
+  for (int g = lane; g < ngroups; g += 32) {
+    const double u = dist(groups[g]) + groups[g].r;
+    if (u < ub) { ub = u; gb = g; }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double u = __shfl_xor_sync(0xffffffffu, ub, o);
+    const int g = __shfl_xor_sync(0xffffffffu, gb, o);
+    if (u < ub || (u == ub && g < gb)) { ub = u; gb = g; }
+  }
+  if (ngroups > 0) {
+    compare(gb);
+    double B = 0.0;
+#pragma unroll
+    for (int q = 0; q < kNpt; ++q) {
+      B = fmax(B, best[q]);
+      best[q] = INFINITY;
+      bi[q] = -1;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) B = fmax(B, __shfl_xor_sync(0xffffffffu, B, o));
+    const double reach = (sqrt(B) + R) * (1.0 + 1e-9);  // room for the rounding of the distances
+    for (int g0 = 0; g0 < ngroups; g0 += 32) {
+      const int g = g0 + lane;
+      unsigned m = __ballot_sync(0xffffffffu, g < ngroups && !(dist(groups[min(g, ngroups - 1)]) - groups[min(g, ngroups - 1)].r > reach));
+      for (; m; m &= m - 1) compare(g0 + __ffs(m) - 1);
     }
   }
 #pragma unroll
   for (int q = 0; q < kNpt; ++q)
-    if (node0 + q < n) a.nearest[node0 + q] = bi[q] >= 0 ? a.cflat[bi[q]] : -1;
+    if (node0 + 32 * q < n) a.nearest[node0 + 32 * q] = bi[q] >= 0 ? a.cflat[bi[q]] : -1;
 }
 
 // 4 x 4 solve with partial pivoting; false when a pivot is below 1e4 machine epsilon
@@ -517,6 +581,13 @@ void ls_reinit_device(sipg_mesh* m, int order, const double* xyz, double* s, dou
   int ncells = 0;
   SIPG_CUDA(cudaMemcpyAsync(&ncells, w.count.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   SIPG_CUDA(cudaStreamSynchronize(st));
+  if (ncells > 1) {  // element order: neighbouring samples lie together, and ties do not depend on the run
+    std::vector<int> cells(ncells);
+    SIPG_CUDA(cudaMemcpyAsync(cells.data(), w.cells.p, ncells * sizeof(int), cudaMemcpyDeviceToHost, st));
+    SIPG_CUDA(cudaStreamSynchronize(st));
+    std::sort(cells.begin(), cells.end());
+    w.cells.upload(cells.data(), ncells * sizeof(int), st);
+  }
   const int nsamples = ncells * Np;
   ensure(w.samples, std::max<size_t>(1, (size_t)nsamples * 3) * sizeof(double));
   a.samples = w.samples.as<double>();
@@ -545,17 +616,42 @@ void ls_reinit_device(sipg_mesh* m, int order, const double* xyz, double* s, dou
       flat.push_back(i);
     }
   const int nkept = (int)flat.size();
+  // groups: a cell's kept samples (at most kGroup), with the sphere around their box's centre
+  std::vector<SampleGroup> groups;
+  for (int i = 0; i < nkept;) {
+    int m = 1;
+    while (i + m < nkept && m < kGroup && flat[i + m] / Np == flat[i] / Np) ++m;
+    const double* k0 = kept.data() + (size_t)i * 3;
+    double c[3], r2 = 0.0;
+    for (int d = 0; d < 3; ++d) {
+      double lo = k0[d], hi = k0[d];
+      for (int k = 1; k < m; ++k) {
+        lo = std::min(lo, k0[3 * k + d]);
+        hi = std::max(hi, k0[3 * k + d]);
+      }
+      c[d] = 0.5 * (lo + hi);
+    }
+    for (int k = 0; k < m; ++k) {
+      double q = 0.0;
+      for (int d = 0; d < 3; ++d) q += (k0[3 * k + d] - c[d]) * (k0[3 * k + d] - c[d]);
+      r2 = std::max(r2, q);
+    }
+    groups.push_back({c[0], c[1], c[2], std::sqrt(r2), i, m});
+    i += m;
+  }
+  ensure(w.groups, std::max<size_t>(1, groups.size()) * sizeof(SampleGroup));
   ensure(w.kept, std::max<size_t>(1, kept.size()) * sizeof(double));
   ensure(w.flat, std::max<size_t>(1, flat.size()) * sizeof(int));
   if (nkept) {
     w.kept.upload(kept.data(), kept.size() * sizeof(double), st);
     w.flat.upload(flat.data(), flat.size() * sizeof(int), st);
+    w.groups.upload(groups.data(), groups.size() * sizeof(SampleGroup), st);
   }
   a.csamples = w.kept.as<double>();
   a.cflat = w.flat.as<int>();
   const size_t nthreads = (n + kNpt - 1) / kNpt;
   const int g3 = (int)((nthreads + kRThreads - 1) / kRThreads);
-  k_reinit_nearest<<<g3, kRThreads, 0, st>>>(a, nkept);
+  k_reinit_nearest<<<g3, kRThreads, 0, st>>>(a, w.groups.as<SampleGroup>(), (int)groups.size());
   note_launch();
   SIPG_CUDA(cudaGetLastError());
   const int g4 = (int)std::max<size_t>(1, std::min<size_t>((n + kRThreads - 1) / kRThreads, (size_t)num_sms() * 16));
