@@ -695,7 +695,7 @@ void sipg_solver::setup_amg() {
     const size_t nn = (size_t)cinv_n * cinv_n;
     ensure(cinv64, nn * sizeof(double));
     ensure(cinv32, nn * sizeof(float));
-    ensure(cinv_work, ((size_t)2 * cinv_n + 1024) * sizeof(double));
+    ensure(cinv_work, dense_inverse_work(cinv_n) * sizeof(double));
     amg_bct = op->bct_host;
     amg_singular = singular;
     amg_frozen = true;

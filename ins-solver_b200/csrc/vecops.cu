@@ -669,135 +669,151 @@ __global__ void __launch_bounds__(128) k_inv_mass_n(T* __restrict__ y, const T* 
   }
 }
 
-// In-place blocked Gauss-Jordan inversion of a dense n x n matrix (row-major,
-// FP64). For each pivot block K of GJB rows and columns, with P = A_KK^-1:
-//   A_Kj <- P A_Kj                  (j not in K; k_gjb_row)
-//   A_ij <- A_ij - A_iK A_Kj        (i, j not in K, with the new A_Kj; k_gjb_update)
-//   A_iK <- -A_iK P, A_KK <- P      (i not in K; k_gjb_col)
-// which is scalar Gauss-Jordan applied GJB pivots at a time: the trailing update
-// is a rank-GJB product over 64 x 64 tiles instead of n rank-1 passes.
+// Blocked Gauss-Jordan inversion of a dense n x n matrix (row-major, FP64), a step from one buffer
+// to the other. For each pivot block K of GJB rows and columns, with P = A_KK^-1:
+//   A'_Kj = P A_Kj                  (j not in K)
+//   A'_ij = A_ij - A_iK (P A_Kj)    (i, j not in K)
+//   A'_iK = -A_iK P,  A'_KK = P     (i not in K)
+// which is scalar Gauss-Jordan applied GJB pivots at a time. One kernel per step, FP64 tensor cores
+// over 128 x 64 tiles: a CTA forms its columns of P A_K (columns of K: P itself, so that the same
+// product gives A'_iK), then the tile; the CTA of the next pivot block, scheduled first, inverts it
+// while the others work. n = 1,919 (60 steps): 4.1 ms as pivot, row, update and column kernels on
+// the CUDA cores (launch gaps included, the whole p = 3 set-up at 24^3 x 6 went 17.7 -> 14.3 ms);
+// now bound by the serial chain of the pivot block (32 reciprocals, about 20 us per step).
 // No pivoting: the coarsest algebraic operator is symmetric positive definite
 // (a singular one is shifted first), so every pivot block is.
-constexpr int GJB = 32;
+constexpr int GJB = 32, GJM = 128, GJN = 64;
+constexpr int GJA = GJB + 4, GJW = GJN + 8;  // shared row strides: fragment loads without bank conflicts
+constexpr size_t kGjbSmem = (size_t)(GJM * GJA + 2 * GJB * GJW + GJB * GJA) * sizeof(double);
 
-// P = A_KK^-1 by scalar Gauss-Jordan in one warp: lane i holds row i of the pivot block
-// in registers and the pivot row reaches every lane by shuffles (no barriers); P is
-// GJB x GJB (GJB = 32, one row per lane), zero outside the bs x bs block.
-static_assert(GJB == 32, "one pivot-block row per lane");
-__global__ void __launch_bounds__(32) k_gjb_pivot(const double* __restrict__ a, int n, int k0, int bs,
-                                                  double* __restrict__ P) {
-  const int i = threadIdx.x;
-  double row[GJB];
-#pragma unroll
-  for (int j = 0; j < GJB; ++j) row[j] = (i < bs && j < bs) ? a[(size_t)(k0 + i) * n + k0 + j] : 0.0;
-#pragma unroll
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// P = B^-1 of a GJB x GJB block by 256 threads: B in buf[0] (padded rows and columns of a block of
+// bs < GJB: identity), a step from one half of buf to the other; P is zero outside the bs x bs block.
+__device__ __forceinline__ void gjb_invert(double (*buf)[GJB][GJB + 1], int bs, double* __restrict__ P) {
+  const int c = threadIdx.x % GJB, r0 = threadIdx.x / GJB;
   for (int k = 0; k < GJB; ++k) {
-    if (k >= bs) break;  // uniform across the warp
-    const double r = 1.0 / __shfl_sync(0xffffffffu, row[k], k);
-    // the pivot row scaled by r (its column k stays until the column step)
-    if (i == k) {
+    const double(*o)[GJB + 1] = buf[k & 1];
+    double(*w)[GJB + 1] = buf[(k & 1) ^ 1];
+    const double rk = 1.0 / o[k][k], pr = c == k ? rk : o[k][c] * rk;
 #pragma unroll
-      for (int j = 0; j < GJB; ++j)
-        if (j != k) row[j] *= r;
+    for (int q = 0; q < GJB / 8; ++q) {
+      const int r = r0 + 8 * q;
+      const double f = o[r][k];
+      w[r][c] = r == k ? pr : (c == k ? 0.0 : o[r][c]) - f * pr;
     }
-    const double aik = row[k];
-#pragma unroll
-    for (int j = 0; j < GJB; ++j) {
-      const double akj = __shfl_sync(0xffffffffu, row[j], k);
-      if (i != k && j != k) row[j] -= aik * akj;
-    }
-    row[k] = i == k ? r : row[k] * -r;
+    __syncthreads();
   }
+  static_assert(GJB % 2 == 0, "the result is in buf[0]");
 #pragma unroll
-  for (int j = 0; j < GJB; ++j) P[i * GJB + j] = (i < bs && j < bs) ? row[j] : 0.0;
-}
-
-// Row panel: one thread per column j outside K.
-__global__ void __launch_bounds__(256) k_gjb_row(double* __restrict__ a, int n, int k0, int bs,
-                                                 const double* __restrict__ P) {
-  __shared__ double sp[GJB * GJB];
-  for (int t = threadIdx.x; t < GJB * GJB; t += blockDim.x) sp[t] = P[t];
-  __syncthreads();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n || (j >= k0 && j < k0 + bs)) return;
-  double col[GJB];
-#pragma unroll
-  for (int m = 0; m < GJB; ++m) col[m] = m < bs ? a[(size_t)(k0 + m) * n + j] : 0.0;
-#pragma unroll
-  for (int i = 0; i < GJB; ++i) {
-    if (i >= bs) break;
-    double s = 0.0;
-#pragma unroll
-    for (int m = 0; m < GJB; ++m) s += sp[i * GJB + m] * col[m];
-    a[(size_t)(k0 + i) * n + j] = s;
+  for (int q = 0; q < GJB / 8; ++q) {
+    const int r = r0 + 8 * q;
+    P[r * GJB + c] = r < bs && c < bs ? buf[0][r][c] : 0.0;
   }
 }
 
-// Trailing update over 64 x 64 tiles, 256 threads, 4 x 4 entries per thread
-// (rows ty + 16 u, columns tx + 16 v: coalesced loads and stores).
-__global__ void __launch_bounds__(256) k_gjb_update(double* __restrict__ a, int n, int k0, int bs) {
-  __shared__ double sc[64][GJB + 1];  // A_iK of the tile's rows
-  __shared__ double sw[GJB][64 + 1];  // A_Kj of the tile's columns
-  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  for (int t = threadIdx.x; t < 64 * GJB; t += 256) {
-    const int r = t / GJB, m = t % GJB;
-    sc[r][m] = (i0 + r < n && m < bs) ? a[(size_t)(i0 + r) * n + k0 + m] : 0.0;
-  }
-  for (int t = threadIdx.x; t < GJB * 64; t += 256) {
-    const int m = t / 64, c = t % 64;
-    sw[m][c] = (j0 + c < n && m < bs) ? a[(size_t)(k0 + m) * n + j0 + c] : 0.0;
+// Inverse of the first pivot block.
+__global__ void __launch_bounds__(256) k_gjb_first(const double* __restrict__ a, int n, double* __restrict__ P) {
+  __shared__ double buf[2][GJB][GJB + 1];
+  pdl_enter();
+  const int bs = min(GJB, n);
+  for (int t = threadIdx.x; t < GJB * GJB; t += 256) {
+    const int r = t / GJB, c = t % GJB;
+    buf[0][r][c] = r < bs && c < bs ? a[(size_t)r * n + c] : (r == c ? 1.0 : 0.0);
   }
   __syncthreads();
-  double acc[4][4] = {};
-#pragma unroll 8
-  for (int m = 0; m < GJB; ++m) {
-    double cv[4], wv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) cv[u] = sc[ty + 16 * u][m];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) wv[v] = sw[m][tx + 16 * v];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[u][v] += cv[u] * wv[v];
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = i0 + ty + 16 * u;
-    if (i >= n || (i >= k0 && i < k0 + bs)) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int j = j0 + tx + 16 * v;
-      if (j >= n || (j >= k0 && j < k0 + bs)) continue;
-      a[(size_t)i * n + j] -= acc[u][v];
-    }
-  }
+  gjb_invert(buf, bs, P);
 }
 
-// Column panel: one thread per row i; rows of K receive P.
-__global__ void __launch_bounds__(128) k_gjb_col(double* __restrict__ a, int n, int k0, int bs,
-                                                 const double* __restrict__ P) {
-  __shared__ double sp[GJB * GJB];
-  for (int t = threadIdx.x; t < GJB * GJB; t += blockDim.x) sp[t] = P[t];
-  __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double* row = a + (size_t)i * n + k0;
-  if (i >= k0 && i < k0 + bs) {
-    for (int j = 0; j < bs; ++j) row[j] = sp[(i - k0) * GJB + j];
-    return;
+// One step: out from a with the pivot block at k0 whose inverse is P; the next block's inverse to Pn.
+__global__ void __launch_bounds__(256, 2) k_gjb_step(const double* __restrict__ a, double* __restrict__ out, int n, int k0,
+                                                     const double* __restrict__ P, double* __restrict__ Pn) {
+  extern __shared__ __align__(16) double gsm[];
+  double* sA = gsm;                   // GJM x GJA: A_iK of the tile's rows
+  double* sR = sA + GJM * GJA;        // GJB x GJW: A_Kj of the tile's columns
+  double* sW = sR + GJB * GJW;        // GJB x GJW: P A_Kj (columns of K: P)
+  double* sP = sW + GJB * GJW;        // GJB x GJA
+  const int bs = min(GJB, n - k0), k1 = k0 + GJB;
+  // the next pivot block's tile comes first
+  const int tn = (n + GJN - 1) / GJN, next = k1 < n ? k1 / GJM * tn + k1 / GJN : 0;
+  const int tile = blockIdx.x == 0 ? next : (int)blockIdx.x == next ? 0 : blockIdx.x;
+  const int i0 = tile / tn * GJM, j0 = tile % tn * GJN;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  pdl_enter();
+  for (int q = threadIdx.x; q < GJM * GJB; q += 256) {
+    const int r = q / GJB, m = q % GJB;
+    sA[r * GJA + m] = i0 + r < n && m < bs ? a[(size_t)(i0 + r) * n + k0 + m] : 0.0;
   }
-  double rv[GJB];
+  for (int q = threadIdx.x; q < GJB * GJN; q += 256) {
+    const int m = q / GJN, c = q % GJN;
+    sR[m * GJW + c] = j0 + c < n && m < bs ? a[(size_t)(k0 + m) * n + j0 + c] : 0.0;
+  }
+  for (int q = threadIdx.x; q < GJB * GJB; q += 256) sP[q / GJB * GJA + q % GJB] = P[q];
+  __syncthreads();
+  {  // W: warp's 8 rows x 32 columns
+    const int r0 = (warp & 3) * 8, c0 = (warp >> 2) * 32;
+    double w[4][2] = {};
 #pragma unroll
-  for (int m = 0; m < GJB; ++m) rv[m] = m < bs ? row[m] : 0.0;
+    for (int k = 0; k < GJB; k += 4) {
+      const double av = sP[(r0 + g) * GJA + k + t];
 #pragma unroll
-  for (int j = 0; j < GJB; ++j) {
-    if (j >= bs) break;
-    double s = 0.0;
+      for (int v = 0; v < 4; ++v) dmma(w[v], av, sR[(k + t) * GJW + c0 + 8 * v + g]);
+    }
 #pragma unroll
-    for (int m = 0; m < GJB; ++m) s += rv[m] * sp[m * GJB + j];
-    row[j] = -s;
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int ci = 0; ci < 2; ++ci) {
+        const int c = c0 + 8 * v + 2 * t + ci, j = j0 + c;
+        sW[(r0 + g) * GJW + c] = j >= k0 && j < k0 + bs ? sP[(r0 + g) * GJA + j - k0] : w[v][ci];
+      }
+  }
+  __syncthreads();
+  double acc[2][8][2] = {};  // warp's 16 rows x 64 columns
+#pragma unroll
+  for (int k = 0; k < GJB; k += 4) {
+    double av[2], bv[8];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) av[u] = sA[(warp * 16 + 8 * u + g) * GJA + k + t];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) bv[v] = sW[(k + t) * GJW + 8 * v + g];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) dmma(acc[u][v], av[u], bv[v]);
+  }
+  const bool ahead = k1 < n && blockIdx.x == 0;
+  if (ahead) __syncthreads();  // sR becomes the next pivot block's buffer (2 x GJB x (GJB + 1) <= GJB x GJW)
+  static_assert(2 * (GJB + 1) <= GJW, "the pivot buffer fits over sR");
+  auto buf = reinterpret_cast<double(*)[GJB][GJB + 1]>(sR);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int i = i0 + warp * 16 + 8 * u + g;
+    const bool ik = i >= k0 && i < k0 + bs;
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+#pragma unroll
+      for (int ci = 0; ci < 2; ++ci) {
+        const int c = 8 * v + 2 * t + ci, j = j0 + c;
+        if (i < n && j < n) {
+          const bool jk = j >= k0 && j < k0 + bs;
+          const double val = ik ? sW[(i - k0) * GJW + c] : (jk ? 0.0 : a[(size_t)i * n + j]) - acc[u][v][ci];
+          out[(size_t)i * n + j] = val;
+          if (ahead && i >= k1 && i < k1 + GJB && j >= k1 && j < k1 + GJB) buf[0][i - k1][j - k1] = val;
+        }
+      }
+  }
+  if (ahead) {
+    const int bn = min(GJB, n - k1);
+    for (int q = threadIdx.x; q < GJB * GJB; q += 256) {
+      const int r = q / GJB, c = q % GJB;
+      if (r >= bn || c >= bn) buf[0][r][c] = r == c ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    gjb_invert(buf, bn, Pn);
   }
 }
 // Row sums, column sums and the total of a dense matrix (one thread per row /
@@ -1259,17 +1275,20 @@ void csr_cheb(int rows, const int* ptr, const int* idx, const T* val, const T* d
 void dense_inverse_device(double* a, int n, bool project_constants, double* work, cudaStream_t s) {
   const size_t nn = (size_t)n * n;
   const int g2 = (int)std::min<size_t>((nn + 255) / 256, 148 * 8);
-  double* P = work + 2 * (size_t)n;  // GJB x GJB pivot-block inverse
-  const int tiles = (n + 63) / 64;
-  for (int k0 = 0; k0 < n; k0 += GJB) {
-    const int bs = std::min(GJB, n - k0);
-    k_gjb_pivot<<<1, 32, 0, s>>>(a, n, k0, bs, P);
-    k_gjb_row<<<(n + 255) / 256, 256, 0, s>>>(a, n, k0, bs, P);
-    k_gjb_update<<<dim3(tiles, tiles), 256, 0, s>>>(a, n, k0, bs);
-    k_gjb_col<<<(n + 127) / 128, 128, 0, s>>>(a, n, k0, bs, P);
-    note_launch(4);
+  double* P[2] = {work + 2 * (size_t)n, work + 2 * (size_t)n + GJB * GJB};  // pivot-block inverses
+  double* buf[2] = {a, work + 2 * (size_t)n + 2 * GJB * GJB};
+  const int tiles = ((n + GJM - 1) / GJM) * ((n + GJN - 1) / GJN);
+  cudaError_t e = cudaFuncSetAttribute(k_gjb_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGjbSmem);
+  int cur = 0;
+  if (e == cudaSuccess) e = pdl_launch(k_gjb_first, dim3(1), dim3(256), 0, s, (const double*)a, n, P[0]);
+  note_launch();
+  for (int k0 = 0; k0 < n && e == cudaSuccess; k0 += GJB, cur ^= 1) {
+    e = pdl_launch(k_gjb_step, dim3(tiles), dim3(256), kGjbSmem, s, (const double*)buf[cur], buf[cur ^ 1], n, k0,
+                   (const double*)P[cur], P[cur ^ 1]);
+    note_launch();
   }
-  const cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && cur) e = cudaMemcpyAsync(a, buf[1], nn * sizeof(double), cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("dense inverse: ") + cudaGetErrorString(e));
   if (project_constants) {
     k_dense_sums<<<(2 * n + 255) / 256, 256, 0, s>>>(a, n, work, work + n);
