@@ -271,6 +271,7 @@ void sipg_op::apply_direction(const double* z, double* p, double* y, const doubl
   a.dot_partial = partial;
   a.dot_counter = counter;
   a.dot_out = dot_out;
+  a.done = scal + S_STATUS;
   SIPG_CUDA(launch_apply_tc<double>(mesh->dim, order, a, dref->tc64.as<double>(), trace64.as<double>(), num_sms(), s));
 }
 

@@ -123,7 +123,7 @@ struct sipg_op {
   template <typename T>
   bool one_launch() const;
   // One conjugate-gradient direction step: p <- z + (scal[bnum] / scal[bden]) p in place,
-  // y = A p, dot_out = p . y. Needs one_launch<double>() and aligned vectors; partial: a value
+  // y = A p, dot_out = p . y; nothing once scal[S_STATUS] is not 0. Needs one_launch<double>() and aligned vectors; partial: a value
   // per CTA (at most two per SM), counter zero.
   void apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden, double* partial,
                        unsigned* counter, double* dot_out, cudaStream_t s) const;

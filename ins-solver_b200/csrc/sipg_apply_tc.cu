@@ -166,6 +166,10 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
       fm[i][w] = v;
     }
   pdl_wait();  // x, factor, c, y and the trace buffer belong to the preceding kernels
+  if (CG && *a.done != 0.0) {
+    cp_wait_all();
+    return;
+  }
   T u[NT][R][2];
   T beta = T(0);
   if (CG) beta = (T)(a.scal[a.bnum] / a.scal[a.bden]);
@@ -444,6 +448,10 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
   if (vt < nvt) load_conn(vt);
   double dot = 0.0;  // CG: this lane's part of x . y
   pdl_wait();
+  if (CG && *a.done != 0.0) {
+    cp_wait_all();
+    return;
+  }
   cp_wait_all();
   __syncthreads();
   for (; vt < nvt; vt += stride) {

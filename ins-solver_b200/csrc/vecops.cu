@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, do
                                                                    double* partial, unsigned* counter) {
   __shared__ double sr[BLK ? kRedThreads : 1];
   pdl_enter();
+  if (scal[S_STATUS] != 0.0) return;
   const double alpha = scal[S_RZ] / scal[S_PAP];
   double v[3] = {0.0, 0.0, 0.0};  // r . r, r . z_old, r . z
   if (BLK) {

@@ -82,7 +82,8 @@ void finish_z_dot(double* z, const float* z32, const double* r, size_t n, const 
 // or element-block Jacobi (row-major Np x Np blocks): x += alpha p ; r -= alpha Ap with alpha =
 // scal[S_RZ] / scal[S_PAP] ; scal[S_RR] = r . r ; rzo = r . z ; z = B r ; then, from the one that
 // finishes last, the flexible beta (scal[S_BETA] = r . z - rzo, S_RZP, S_RZ) and, with `loop`
-// not 0, the stopping test of the while-node it belongs to (as loop_check).
+// not 0, the stopping test of the while-node it belongs to (as loop_check). Nothing is done once
+// scal[S_STATUS] is not 0.
 void cg_update_precond(double* x, double* r, const double* p, const double* Ap, double* z, const double* B, int Np,
                        size_t n, double* scal, cudaGraphConditionalHandle loop, int max_iter, const RedWork& w,
                        cudaStream_t s);
