@@ -256,7 +256,7 @@ bool sipg_op::one_launch() const {
   return ncomp == 1 || (tr.bytes >= one * ncomp && (size_t)mesh->K * Np * sizeof(T) % 16 == 0);
 }
 
-void sipg_op::apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden,
+int sipg_op::apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden,
                               double* partial, unsigned* counter, double* dot_out, cudaStream_t s) const {
   ApplyArgs<double> a = apply_args<double>(p, y);
   if (ncomp > 1) {
@@ -272,7 +272,10 @@ void sipg_op::apply_direction(const double* z, double* p, double* y, const doubl
   a.dot_counter = counter;
   a.dot_out = dot_out;
   a.done = scal + S_STATUS;
+  int count = 0;
+  a.dot_count = &count;
   SIPG_CUDA(launch_apply_tc<double>(mesh->dim, order, a, dref->tc64.as<double>(), trace64.as<double>(), num_sms(), s));
+  return count;
 }
 
 template <typename T>

@@ -123,9 +123,10 @@ struct sipg_op {
   template <typename T>
   bool one_launch() const;
   // One conjugate-gradient direction step: p <- z + (scal[bnum] / scal[bden]) p in place,
-  // y = A p, dot_out = p . y; nothing once scal[S_STATUS] is not 0. Needs one_launch<double>() and aligned vectors; partial: a value
-  // per CTA (at most two per SM), counter zero.
-  void apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden, double* partial,
+  // y = A p, p . y in dot_out or, where that is null, as the returned number of partial sums;
+  // nothing once scal[S_STATUS] is not 0. Needs one_launch<double>() and aligned vectors;
+  // partial: a value per CTA (of 256 threads: at most kRedBlocks), counter zero.
+  int apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden, double* partial,
                        unsigned* counter, double* dot_out, cudaStream_t s) const;
   template <typename T>
   sipg::ApplyArgs<T> apply_args(const T* x, T* y) const;

@@ -115,13 +115,15 @@ struct ApplyArgs {
   int nvec = 1;           // tensor-core path: components applied by one launch (x, y, c K x NP apart, nrec K x NF)
   const uint8_t* slip = nullptr;  // nvec > 1: per element, bit f set where face f is a slip face
   // tensor-core path, FP64, inside a conjugate-gradient iteration (pz not null): x <- pz +
-  // (scal[bnum] / scal[bden]) x is formed and stored in place first, and dot_out = x . y
-  // (partial: one value per CTA; counter zero before and after). Nothing is done once
-  // *done is not 0 (the loop has ended within a group of iterations)
+  // (scal[bnum] / scal[bden]) x is formed and stored in place first, and x . y is left as one
+  // partial sum per CTA (their number in *dot_count, on the host) or, with dot_out, summed
+  // there (counter zero before and after). Nothing is stored once *done is not 0 (the loop has
+  // ended within a group of iterations)
   const T* pz = nullptr;
   const double* scal = nullptr;
   int bnum = 0, bden = 0;
   double *dot_partial = nullptr, *dot_out = nullptr;
+  int* dot_count = nullptr;
   const double* done = nullptr;
   unsigned* dot_counter = nullptr;
   int tcgen05 = 0;        // tensor-core path, FP32: tcgen05 kernels where the order has them (else mma.sync)

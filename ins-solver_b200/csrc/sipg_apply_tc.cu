@@ -166,19 +166,27 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
       fm[i][w] = v;
     }
   pdl_wait();  // x, factor, c, y and the trace buffer belong to the preceding kernels
-  if (CG && *a.done != 0.0) {
-    cp_wait_all();
-    return;
-  }
   T u[NT][R][2];
   T beta = T(0);
-  if (CG) beta = (T)(a.scal[a.bnum] / a.scal[a.bden]);
+  // the loop's state, beta's operands and the first tile's rows are loaded together: one latency
+  double done = 0.0, bn = 0.0, bd = 1.0;
+  if (CG) {
+    done = *a.done;
+    bn = a.scal[a.bnum];
+    bd = a.scal[a.bden];
+  }
+  bool first = true;
   auto load_x = [&](int v) {
     const int comp = VEC ? v / ntiles : 0, e0 = (v - comp * ntiles) * TE, ne = min(TE, a.K - e0);
     load_nodes<T, DIM, P>(a.x + comp * per, e0, ne, u, g, t);
     if (CG) {
       T z[NT][R][2];
       load_nodes<T, DIM, P>(a.pz + comp * per, e0, ne, z, g, t);
+      if (first) {
+        first = false;
+        beta = (T)(bn / bd);
+        if (done != 0.0) return;
+      }
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -190,6 +198,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
   };
   if (vt < nvt) load_x(vt);
   cp_wait_all();
+  if (CG && done != 0.0) return;
   __syncthreads();
   for (; vt < nvt; vt += stride) {
     const int comp = VEC ? vt / ntiles : 0, tile = vt - comp * ntiles;
@@ -448,10 +457,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
   if (vt < nvt) load_conn(vt);
   double dot = 0.0;  // CG: this lane's part of x . y
   pdl_wait();
-  if (CG && *a.done != 0.0) {
-    cp_wait_all();
-    return;
-  }
+  const double done = CG ? *a.done : 0.0;  // looked at when the first tile's loads are under way
   cp_wait_all();
   __syncthreads();
   for (; vt < nvt; vt += stride) {
@@ -525,6 +531,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
         for (int r = 0; r < DIM; ++r) F::mma(y[nt], sv[r], ldb(B + X::BQ, (r * FT + fb) * NT + nt, lane));
       }
     }
+    if (CG && done != 0.0) break;
     if (vt + stride < nvt) load_conn(vt + stride);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
@@ -563,9 +570,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
       for (int w = 0; w < WARPS; ++w) s += sh[w];
       return s;
     };
+    if (done != 0.0) return;
     dot = cta_sum(dot);
+    if (threadIdx.x == 0) a.dot_partial[blockIdx.x] = dot;
+    if (!a.dot_out) return;
     if (threadIdx.x == 0) {
-      a.dot_partial[blockIdx.x] = dot;
       __threadfence();
       last = atomicAdd(a.dot_counter, 1u) == gridDim.x - 1;
     }
@@ -709,11 +718,12 @@ cudaError_t kernel_setup(int warps, size_t bytes, int& per_sm) {
 
 template <auto K, typename T, typename TT>
 cudaError_t launch_pass(const ApplyArgs<T>& a, const T* blob, TT* trace, int warps, size_t bytes, int ntiles,
-                        int num_sms, cudaStream_t s) {
+                        int num_sms, cudaStream_t s, int* ctas = nullptr) {
   int per_sm = 1;
   cudaError_t err = kernel_setup<K>(warps, bytes, per_sm);
   if (err != cudaSuccess) return err;
   const int grid = std::min(ntiles, num_sms * per_sm);
+  if (ctas) *ctas = grid;
   if (grid > 0) {
     err = pdl_launch(K, dim3(grid), dim3(warps * 32), bytes, s, a, blob, trace);
     if (err != cudaSuccess) return err;
@@ -730,7 +740,7 @@ cudaError_t launch_passes(const ApplyArgs<T>& a, const T* blob, T* trace, int nt
                                 smem1<T, DIM, P>(WARPS), ntiles, num_sms, s);
   if (err != cudaSuccess) return err;
   return launch_pass<sipg_face_kernel<T, DIM, P, 8, 2, VEC, CG>>(a, blob + Tc<T, DIM, P>::N1, (const T*)trace, 8,
-                     smem2<T, DIM, P>(), ntiles, num_sms, s);
+                     smem2<T, DIM, P>(), ntiles, num_sms, s, a.dot_count);
 }
 
 // Launch shape: two CTAs of 8 warps per SM (128 registers per thread), for pass 1 one of 12

@@ -203,7 +203,9 @@ __global__ void k_beta_flex(double* scal) {
   scal[S_RZ] = scal[S_RZN];
 }
 
-__global__ void k_loop_check(double* scal, cudaGraphConditionalHandle h, int max_iter) { loop_check(scal, h, max_iter); }
+__global__ void k_loop_check(double* scal, cudaGraphConditionalHandle h, int max_iter) {
+  loop_check(scal, h, max_iter, scal[S_ITER], scal[S_TOL], scal[S_CHUNK], scal[S_PAP], scal[S_RR]);
+}
 
 // beta = 0 for the first direction step (p = z), loop running
 __global__ void k_loop_start(double* scal) {
@@ -749,7 +751,7 @@ void sipg_solver::setup_body() {
     size_t b = n * sizeof(double);
     r = DevBuf(b); z = DevBuf(b); p = DevBuf(b); Ap = DevBuf(b);
     scal = DevBuf(S_COUNT * sizeof(double));
-    partial = DevBuf(kRedBlocks * 4 * sizeof(double));
+    partial = DevBuf(kRedBlocks * 5 * sizeof(double));  // RedWork's, then the operator's p . Ap
     counter = DevBuf(sizeof(unsigned));
     SIPG_CUDA(cudaMemsetAsync(counter.p, 0, sizeof(unsigned), stream));
     SIPG_CUDA(cudaMemsetAsync(scal.p, 0, S_COUNT * sizeof(double), stream));
@@ -1181,21 +1183,27 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
     // Iterations per pass of the while-node: a pass costs about 10 us besides its kernels, as
     // much as a whole Jacobi iteration of a small mesh (three launches). Those kernels do
     // nothing once the stopping test has ended the loop, so eight share a pass. 2D block-Jacobi
-    // solve of 8,192 triangles, p = 3: 62.1 -> 47.9 ms.
+    // solve of 8,192 triangles, p = 3: 62.1 -> 47.9 ms with eight,
+    // before the kernels themselves got shorter. A plain graph of 8, 16 or 32 iterations,
+    // launched again until the loop has ended, takes what the while-node takes (16.9, 16.5 and
+    // 16.5 against 16.8 us per iteration).
     const int group = jac && ride ? 8 : 1;
     // loop: the while-node the iteration is captured into (0: none)
     auto body = [&](cudaGraphConditionalHandle loop) {
+      int npap = 0;  // Jacobi: the update sums p . Ap's partials itself (kept apart from its own)
+      double* ppap = rw.partial + 4 * kRedBlocks;
       if (ride) {
-        op->apply_direction(Z, Pv, AP, S(), S_BETA, S_RZP, rw.partial, rw.counter, S() + S_PAP, stream);
+        npap = op->apply_direction(Z, Pv, AP, S(), S_BETA, S_RZP, ppap, rw.counter, jac ? nullptr : S() + S_PAP,
+                                   stream);
       } else {
         op->apply<double>(Pv, AP, stream);
         dot(Pv, AP, S_PAP);  // cg3_alpha_pre
       }
       if (jac) {  // update_ans + update_res, preconditioner, beta and the stopping test in one pass
         if (kind == SIPG_SOLVER_JACOBI)
-          cg_update_precond(x, R, Pv, AP, Z, dinv.as<double>(), 0, n, S(), loop, o.max_iter, rw, stream);
+          cg_update_precond(x, R, Pv, AP, Z, dinv.as<double>(), 0, n, S(), ppap, npap, loop, o.max_iter, rw, stream);
         else
-          cg_update_precond(x, R, Pv, AP, Z, blocks.as<double>(), op->Np, n, S(), loop, o.max_iter, rw, stream);
+          cg_update_precond(x, R, Pv, AP, Z, blocks.as<double>(), op->Np, n, S(), ppap, npap, loop, o.max_iter, rw, stream);
         if (!ride) update_p<double>(Pv, Z, n, S(), S_BETA, S_RZP, stream);
         return;
       }

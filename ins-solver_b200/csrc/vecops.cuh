@@ -83,22 +83,27 @@ void finish_z_dot(double* z, const float* z32, const double* r, size_t n, const 
 // scal[S_RZ] / scal[S_PAP] ; scal[S_RR] = r . r ; rzo = r . z ; z = B r ; then, from the one that
 // finishes last, the flexible beta (scal[S_BETA] = r . z - rzo, S_RZP, S_RZ) and, with `loop`
 // not 0, the stopping test of the while-node it belongs to (as loop_check). Nothing is done once
-// scal[S_STATUS] is not 0.
+// scal[S_STATUS] is not 0. npap > 0: p . Ap is the sum of npap partials (at pap), stored to
+// scal[S_PAP]; else it is there already.
 void cg_update_precond(double* x, double* r, const double* p, const double* Ap, double* z, const double* B, int Np,
-                       size_t n, double* scal, cudaGraphConditionalHandle loop, int max_iter, const RedWork& w,
-                       cudaStream_t s);
+                       size_t n, double* scal, const double* pap, int npap, cudaGraphConditionalHandle loop,
+                       int max_iter, const RedWork& w, cudaStream_t s);
 // Stopping test of the device-resident outer loop, by one thread at the end of its body: ends the
 // while-node `loop` once converged, broken down, at the iteration limit or at the end of a chunk.
 #ifdef __CUDACC__
-__device__ __forceinline__ void loop_check(double* scal, cudaGraphConditionalHandle loop, int max_iter) {
-  const double it = scal[S_ITER] + 1.0;
+__device__ __forceinline__ void loop_check(double* scal, cudaGraphConditionalHandle loop, int max_iter, double it,
+                                           double tol, double chunk, double pap, double rr) {
+  it += 1.0;
+  chunk -= 1.0;
   scal[S_ITER] = it;
-  const double pap = scal[S_PAP], rr = scal[S_RR];
   double st = 0.0;
   if (!(pap > 0.0) || !isfinite(rr)) st = 2.0;
-  else if (sqrt(rr) <= scal[S_TOL]) st = 1.0;
+  else if (sqrt(rr) <= tol) st = 1.0;
   else if (it >= (double)max_iter) st = 3.0;
-  else if ((scal[S_CHUNK] -= 1.0) <= 0.0) st = 4.0;
+  else {
+    scal[S_CHUNK] = chunk;
+    if (chunk <= 0.0) st = 4.0;
+  }
   if (st != 0.0) {
     scal[S_STATUS] = st;
     cudaGraphSetConditional(loop, 0);

@@ -74,6 +74,21 @@ def test_constant_factor_gives_the_nodal_operator(dim, n, p, bnd):
     assert rel_err(oi.apply_host(x), 2.0 * nodal.apply_host(x)) < 1e-12
 
 
+@pytest.mark.parametrize("n", [17, 18])
+def test_rows_per_thread_of_the_block_apply_follow_the_mesh(n):
+    """3D p = 3: from 30,311 elements on a thread of the block apply holds four rows, below
+    two. 29,478 and 34,992 elements give the nodal operator of a constant factor (the
+    assembled blocks round as in the small cases above)."""
+    gm = sipg.Mesh.box(3, n, jitter=0.1, seed=3)
+    oi, nodal = sipg.Operator(gm, 3, 1), sipg.Operator(gm, 3, 1)
+    for o in (oi, nodal):
+        o.set_bc_types(bct_of(gm.Kb, 2))
+    nq, nqs = oi.oi_sizes()
+    oi.set_factor_oi(np.ones((gm.K, nq)), np.ones((gm.K, 4, nqs)))
+    x = np.random.default_rng(n).uniform(-1.0, 1.0, (1, gm.K, oi.Np))
+    assert rel_err(oi.apply_host(x), nodal.apply_host(x)) < 1e-12
+
+
 def test_operator_is_symmetric_and_pinning_replaces_the_row_and_column():
     gm, om, op, bct, fv, fs = setup_case(3, 3, 3, 1, pin=True)
     rng = np.random.default_rng(2)

@@ -311,3 +311,23 @@ def test_2d_block_jacobi_cg_config_matches_oracle():
     assert info.status == sipg.SIPG_OK
     assert abs(info.iters - io.iters) <= 1
     assert np.linalg.norm(x - xo) / np.linalg.norm(xo) < 1e-9
+
+
+@pytest.mark.parametrize("max_iter", [1, 2, 8, 9, 10, 16, 17, 18, 64, 65, 66, 73, 400])
+@pytest.mark.parametrize("kind", [sipg.SOLVER_JACOBI, sipg.SOLVER_BLOCK_JACOBI], ids=["jacobi", "block"])
+def test_jacobi_loop_ends_within_a_group(kind, max_iter):
+    """The Jacobi loop holds several iterations per launch of its graph: whether the
+    iteration limit or the tolerance ends it at the first, the last or an inner
+    iteration of a group, the iterates are those of kernels launched one by one."""
+    c = W.poisson3d_two_phase(3, order=2, n_modes=64, pin=False)
+    bct = np.full_like(c["bc_types"], sipg.BC_DIRICHLET)  # no null space
+    out = {}
+    for graphs in (0, 2):
+        op = make_op(c["mesh"], 2, 1, c["factor"], bct=bct)
+        o = sipg.default_opts(kind)
+        o.rel_tol, o.abs_tol, o.max_iter, o.nullspace, o.graphs = 1e-9, 0.0, max_iter, 0, graphs
+        s = sipg.Solver(op, kind, o)
+        out[graphs] = [s.solve_host(c["rhs"]) for _ in range(2)]
+    for (xe, ie), (xg, ig) in zip(out[0], out[2]):
+        assert ie.iters == ig.iters <= max_iter and ie.status == ig.status
+        assert np.array_equal(xe, xg)
