@@ -225,8 +225,9 @@ __global__ void __launch_bounds__(kRedThreads) k_finish_z_dot(double* z, const f
 // operator's partials, by every CTA alike, while the first rows are under way, which takes the
 // operator's last-CTA reduction out of the chain. With the scalars of both kernels loaded at once
 // an iteration of 8,192 triangles, p = 3, takes 16.8 us instead of 19.7, of 512 triangles 11.4
-// instead of 14.6.
-template <bool BLK>
+// instead of 14.6. BLK: the first NB entries of a block row are loaded with the rows, not after
+// alpha (15.5 and 10.6 us); NB = 10 is a whole row at 2D p = 3 and 3D p = 2 and leaves no spill.
+template <bool BLK, int NB = 10>
 __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, double* r, const double* p,
                                                                    const double* Ap, double* z, const double* B,
                                                                    int Np, size_t n, double* scal, const double* pap,
@@ -249,6 +250,7 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, do
   const size_t step = (size_t)gridDim.x * rows;
   size_t i0 = blockIdx.x * (size_t)rows;
   double nx = 0.0, nr = 0.0, np = 0.0, na = 0.0, nz = 0.0, nb = 0.0;
+  double bb[BLK ? NB : 1];
   auto fetch = [&](size_t i) {
     if (mine && i < n) {
       nx = x[i];
@@ -257,6 +259,11 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, do
       na = Ap[i];
       nz = z[i];
       if (!BLK) nb = B[i];
+      if (BLK) {
+        const double* Bi = B + i * Np;
+#pragma unroll
+        for (int j = 0; j < NB; ++j) bb[j] = j < Np ? Bi[j] : 0.0;
+      }
     }
   };
   fetch(i0 + threadIdx.x);
@@ -275,8 +282,8 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, do
       x[i] = xi;
       r[i] = ri;
     }
-    fetch(i + step);
     double zi;
+    if (!BLK) fetch(i + step);
     if (BLK) {
       __syncthreads();  // the previous blocks' rows have been read
       sr[threadIdx.x] = ri;
@@ -284,8 +291,12 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, do
       zi = 0.0;
       if (act) {
         const double* Bi = B + i * Np;
-        for (int j = 0; j < Np; ++j) zi += Bi[j] * sr[b0 + j];
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          if (j < Np) zi += bb[j] * sr[b0 + j];
+        for (int j = NB; j < Np; ++j) zi += Bi[j] * sr[b0 + j];
       }
+      fetch(i + step);
     } else {
       zi = bi * ri;
     }
