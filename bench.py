@@ -425,7 +425,7 @@ def run_over_integrated(c, steps=5, warmup=3):
             "mixed_ms_per_solve": float(np.mean(ms)), "iters": int(infos[-1].iters),
             "true_rel_res": float(infos[-1].true_rel_res),
             "apply_fp64_ms": t64,
-            "roofline": {"kernel": "k_bsr<double,20,4> (over-integrated element blocks)", "bound": "hbm",
+            "roofline": {"kernel": "k_bsr<double,20,4,4> (over-integrated element blocks)", "bound": "hbm",
                          "achieved": bpe * K / (t64 * 1e-3) / 1e9, "peak": hbm, "peak_kind": peak_kind,
                          "unit": "GB/s", "frac": bpe * K / (t64 * 1e-3) / 1e9 / hbm, "bytes_per_elem": bpe,
                          "traffic": (tpe * K if (tpe := profile_value("oi_block_apply_fp64_p3_16cube.txt",
@@ -562,7 +562,7 @@ def run_ours(args):
                     "fp64_gdofs": K4 * Np4 / (t64 * 1e-3) / 1e9, "fp32_gdofs": K4 * Np4 / (t32 * 1e-3) / 1e9,
                     "fp64_ms": t64, "fp32_ms": t32,
                     "fp32_hbm_frac": b4 * K4 / (t32 * 1e-3) / 1e9 / hbm,
-                    "roofline": {"kernel": "sipg_trace_kernel<float,3,4,9> + sipg_apply_tc_kernel<float,3,4,7,1>",
+                    "roofline": {"kernel": "sipg_volume_kernel<float,3,4> + sipg_face_kernel<float,3,4>",
                                  "bound": "hbm", "achieved": b4 * K4 / (t32 * 1e-3) / 1e9, "peak": hbm,
                                  "peak_kind": peak_kind, "unit": "GB/s",
                                  "frac": b4 * K4 / (t32 * 1e-3) / 1e9 / hbm,
@@ -604,7 +604,7 @@ def run_ours(args):
                      "fp64_gdofs": n / (a64 * 1e-3) / 1e9, "fp32_tcgen05_ms": a32_tc5,
                      "fp32_tcgen05_gdofs": n / (a32_tc5 * 1e-3) / 1e9},
         "apply_c3": apply_c3,
-        "roofline": {"kernel": "sipg_trace_kernel<float,3,3> + sipg_apply_tc_kernel<float,3,3> "
+        "roofline": {"kernel": "sipg_volume_kernel<float,3,3> + sipg_face_kernel<float,3,3> "
                                "(one FP32 p=3 apply = 2 launches)",
                      "bound": "hbm", "achieved": achieved, "peak": hbm, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": achieved / hbm,
@@ -758,7 +758,7 @@ def run_projection(steps=20, cpu=True):
     dofs = 3 * K * Np
     out = {"workload": "velocity projection (div_div=1), 3D 32^3x6=196608 tets p=3, dt=1e-3, "
                        "velT and grad p U(-1,1)",
-           "kernel": "k_proj_cg<3,3> (one launch per projection)",
+           "kernel": "k_proj_tc<3> (one launch per projection)",
            "ms": ms, "gdofs": dofs / (ms * 1e-3) / 1e9, "converged": conv, "cells": K,
            "mean_iters": iters / K,
            "pressure_rhs": {"ms": ms_r, "hbm_gbs": rhs_bytes / (ms_r * 1e-3) / 1e9,
@@ -1083,7 +1083,7 @@ def run_profile(args):
     apply: the headline operator at --n (order --order, precision --precision),
            3 applies after set-up; with -k regex:"sipg_(trace|apply_tc)" -s 2 -c 2
            ncu captures the second apply's two kernels.
-    projection: the velocity projection workload at --n (3 launches of k_proj_cg).
+    projection: the velocity projection workload at --n (3 launches of k_proj_tc).
     pressure: the pressure step kernels at --n: sipg_pressure_rhs and
            sipg_pressure_projection alternately, 3 launches each.
     c3apply: the Helmholtz operator (I/(nu dt) - Laplacian) at --n, order --order,
@@ -1129,7 +1129,7 @@ def run_profile(args):
         d_do = sipg.DeviceVector(np.zeros((K, 4, Nfp)))
         d_rhs = sipg.DeviceVector(np.zeros((K, Np)))
         lib = sipg.lib()
-        for _ in range(3):  # k_pr_rhs and k_proj_cg<3,3,true> alternate
+        for _ in range(3):  # k_pr_rhs and k_proj_tc<3,true> alternate
             sipg.check(lib.sipg_pressure_rhs(mesh.h, PROJ_ORDER, C.c_double(PROJ_DT), C.c_double(2.0),
                                              C.c_double(-1.0), C.c_void_p(d_v.ptr), C.c_void_p(d_dn.ptr),
                                              C.c_void_p(d_do.ptr), C.c_void_p(d_rhs.ptr), C.c_void_p(0)))
