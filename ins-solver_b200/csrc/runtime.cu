@@ -240,7 +240,7 @@ ApplyArgs<T> sipg_op::apply_args(const T* x, T* y) const {
 
 template <typename T>
 bool sipg_op::one_launch() const {
-  if (oi || kernel == 1 || !nrec.p || (ncomp > 1 && (pin_elem >= 0 || kernel == 3))) return false;
+  if (oi || kernel == 1 || !nrec.p || (ncomp > 1 && pin_elem >= 0)) return false;
   DevBuf& tr = std::is_same<T, double>::value ? trace64 : trace32;
   const size_t one = tc_trace_values(mesh->dim, order, mesh->K) * sizeof(T);
   if (!tr.p) {
@@ -252,8 +252,9 @@ bool sipg_op::one_launch() const {
       tr = DevBuf(one);
     }
   }
-  // a vector operator needs all components' traces and every row on a 16-byte boundary
-  return ncomp == 1 || (tr.bytes >= one * ncomp && (size_t)mesh->K * Np * sizeof(T) % 16 == 0);
+  // a vector operator needs all components' traces and every row on a 16-byte boundary; the
+  // tcgen05 kernels take a component per launch
+  return ncomp == 1 || (kernel != 3 && tr.bytes >= one * ncomp && (size_t)mesh->K * Np * sizeof(T) % 16 == 0);
 }
 
 int sipg_op::apply_direction(const double* z, double* p, double* y, const double* scal, int bnum, int bden,
@@ -292,7 +293,7 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
   const bool tc_ok = (kernel == 0 || kernel >= 2) && nrec.p;
   if (tc_ok && ncomp > 1 && pin_elem < 0) {
     const T* tcc = f64 ? (const T*)dref->tc64.p : (const T*)dref->tc32.p;
-    const bool batch = one_launch<T>();
+    const bool batch = one_launch<T>();  // allocates the traces, whatever it answers here
     const DevBuf& tr = f64 ? trace64 : trace32;
     const size_t per = (size_t)mesh->K * Np;
     // every component in one pair of launches, slip faces included

@@ -118,8 +118,9 @@ struct sipg_op {
   template <typename T>
   // y = alpha A x + beta c, c = y when null (beta == 0: c is not read)
   void apply(const T* x, T* y, cudaStream_t s, T alpha = T(1), T beta = T(0), const T* c = nullptr) const;
-  // Whether a call on 16-byte aligned vectors runs as one pair of tensor-core launches
-  // (allocates their trace scratch).
+  // Whether a call on 16-byte aligned vectors runs as one pair of tensor-core launches.
+  // Allocates the trace scratch wherever the tensor-core kernels run at all, also component by
+  // component.
   template <typename T>
   bool one_launch() const;
   // One conjugate-gradient direction step: p <- z + (scal[bnum] / scal[bden]) p in place,

@@ -750,6 +750,7 @@ cudaError_t launch_passes(const ApplyArgs<T>& a, const T* blob, T* trace, int nt
 template <typename T, int DIM, int P>
 cudaError_t launch_tc_t(const ApplyArgs<T>& a, const T* blob, T* trace, int num_sms, cudaStream_t s) {
   using X = Tc<T, DIM, P>;
+  if (a.K > 0 && !trace) return cudaErrorInvalidValue;
   if constexpr (std::is_same<T, float>::value) {
     // FP32: the tcgen05 kernels (their constants follow the mma.sync blob)
     if (a.tcgen05 && tc5_supported(DIM, P)) return launch_apply_tc5(DIM, P, a, blob + X::NALL, trace, num_sms, s);

@@ -43,3 +43,18 @@ def test_vector_operator_with_slip_faces(dim, n, order):
         xd, yd = DevArray(x.astype(dtype)), DevArray(np.full(x.shape, 7.0, dtype))
         op.apply_device(prec, xd.p, yd.p)
         assert rel_err(yd.get().astype(np.float64), ref) < tol
+
+
+@pytest.mark.parametrize("kernel", [2, 3])
+@pytest.mark.parametrize("prec,dtype,tol", [(sipg.FP64, np.float64, TOL_FP64), (sipg.FP32, np.float32, TOL_TF32)],
+                         ids=["fp64", "fp32"])
+@pytest.mark.parametrize("dim,n,order", [(2, 4, 2), (3, 2, 3), (3, 3, 4)])
+def test_vector_operator_first_apply_with_a_selected_kernel(dim, n, order, kernel, prec, dtype, tol):
+    """The first apply of a vector operator allocates the trace scratch under every tensor-core
+    kernel selection, the component-by-component one (3) included."""
+    mesh, t, e, om, x, f, m, bct = random_case(dim, n, order, dim, seed=order + dim, slip=True, mm=True)
+    op = make_op(mesh, order, dim, f, m, bct=bct)
+    op.set_kernel(kernel)
+    xd, yd = DevArray(x.astype(dtype)), DevArray(np.full(x.shape, 7.0, dtype))
+    op.apply_device(prec, xd.p, yd.p)
+    assert rel_err(yd.get().astype(np.float64), O.mult(om, x, bct, f, m)) < tol
