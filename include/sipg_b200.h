@@ -133,8 +133,9 @@ int sipg_op_apply_host(sipg_op *op, const double *x, double *y);
 #define SIPG_STATIC_SCRATCH_BYTES (64u << 20)
 int sipg_op_apply_static_scratch(sipg_op *op, int precision, const void *x, void *y, void *stream);
 /* Kernel selection of apply(): 0 tensor cores where the operator allows it
- * (scalar operators: mma.sync TF32 MMAs for SIPG_FP32, FP64 MMAs for SIPG_FP64),
- * 1 the CUDA-core kernel, 2 the same tensor-core kernels as 0, 3 SIPG_FP32 on
+ * (scalar operators, and vector ones without a pinned DOF: mma.sync TF32 MMAs for
+ * SIPG_FP32, FP64 MMAs for SIPG_FP64; with SIPG_FP32 the terms of a vector operator's
+ * slip faces are FP32 multiply-adds on every path), 1 the CUDA-core kernel, 2 the same tensor-core kernels as 0, 3 SIPG_FP32 on
  * tcgen05 TF32 MMAs with TMEM accumulators where the order has those kernels
  * (3D p = 3; otherwise as 0). No reference counterpart (the reference has one
  * OP2 path). */

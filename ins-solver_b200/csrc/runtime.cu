@@ -296,28 +296,37 @@ void sipg_op::apply(const T* x, T* y, cudaStream_t s, T alpha, T beta, const T* 
     const bool batch = one_launch<T>();  // allocates the traces, whatever it answers here
     const DevBuf& tr = f64 ? trace64 : trace32;
     const size_t per = (size_t)mesh->K * Np;
-    // every component in one pair of launches, slip faces included
     auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    if (batch && aligned(x) && aligned(y) && (beta == T(0) || aligned(a.c))) {
-      a.ncomp = 1;
-      a.nvec = ncomp;
-      a.slip = slip.as<uint8_t>();
-      SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, a, tcc, tr.as<T>(), num_sms(), s));
-      return;
+    const bool one_pair = batch && aligned(x) && aligned(y) && (beta == T(0) || aligned(a.c));
+    // Slip faces ride on the pair in FP64. In FP32 their terms stay multiply-adds on FP32
+    // operands in a kernel of their own (the pair would round them to TF32, 10 bits), as do
+    // those of the component-by-component form; that kernel reads x after y has been written.
+    const bool slip_pass = any_slip && !(f64 && one_pair);
+    ApplyArgs<T> as = a;
+    if (slip_pass && x == y) {
+      ensure(slip_x, per * ncomp * sizeof(T));
+      SIPG_CUDA(cudaMemcpyAsync(slip_x.p, x, per * ncomp * sizeof(T), cudaMemcpyDeviceToDevice, s));
+      as.x = (const T*)slip_x.p;
     }
-    // else one scalar apply per component (its own boundary types; slip faces get no face
-    // terms there), then the slip faces' coupling terms
-    for (int comp = 0; comp < ncomp; ++comp) {
-      ApplyArgs<T> ac = a;
-      ac.ncomp = 1;
-      ac.x = x + comp * per;
-      ac.y = y + comp * per;
-      ac.c = a.c + comp * per;
-      ac.bct = bct.as<uint8_t>() + (size_t)comp * mesh->Kb;
-      ac.nrec = nrec.as<uint32_t>() + (size_t)comp * mesh->K * (mesh->dim + 1);
-      SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, ac, tcc, tr.as<T>(), num_sms(), s));
+    if (one_pair) {  // every component in one pair of launches
+      ApplyArgs<T> av = a;
+      av.ncomp = 1;
+      av.nvec = ncomp;
+      av.slip = f64 ? slip.as<uint8_t>() : nullptr;
+      SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, av, tcc, tr.as<T>(), num_sms(), s));
+    } else {  // one scalar apply per component (its own boundary types; slip faces get no face terms)
+      for (int comp = 0; comp < ncomp; ++comp) {
+        ApplyArgs<T> ac = a;
+        ac.ncomp = 1;
+        ac.x = x + comp * per;
+        ac.y = y + comp * per;
+        ac.c = a.c + comp * per;
+        ac.bct = bct.as<uint8_t>() + (size_t)comp * mesh->Kb;
+        ac.nrec = nrec.as<uint32_t>() + (size_t)comp * mesh->K * (mesh->dim + 1);
+        SIPG_CUDA(launch_apply_tc<T>(mesh->dim, order, ac, tcc, tr.as<T>(), num_sms(), s));
+      }
     }
-    SIPG_CUDA(launch_slip<T>(mesh->dim, order, a, mesh->belems.as<int>(), mesh->n_belem, s));
+    if (slip_pass) SIPG_CUDA(launch_slip<T>(mesh->dim, order, as, mesh->belems.as<int>(), mesh->n_belem, s));
     return;
   }
   const bool tc = tc_ok && ncomp == 1;
@@ -349,6 +358,11 @@ void sipg_op::refresh_tau(cudaStream_t s) {
 }
 
 void sipg_op::refresh_bc() {
+  any_slip = false;
+  for (int b = 0; ncomp > 1 && b < mesh->Kb && !any_slip; ++b) {
+    any_slip = true;
+    for (int c = 0; c < ncomp; ++c) any_slip = any_slip && bct_host[(size_t)c * mesh->Kb + b] == SIPG_BC_SLIP;
+  }
   if (!nrec.p) return;
   for (int c = 0; c < ncomp; ++c)
     SIPG_CUDA(launch_neighbour_records(mesh->dim, mesh->nbr.as<int>(), mesh->fcode.as<uint32_t>(),

@@ -102,6 +102,8 @@ struct sipg_op {
   std::vector<int> bct_host;  // ncomp x Kb
   sipg::DevBuf nrec;          // neighbour records of the tensor-core apply, ncomp x K x Nf (ApplyArgs::nrec)
   sipg::DevBuf slip;          // vector operators: slip faces per element (ApplyArgs::slip)
+  bool any_slip = false;      // a boundary face is of slip type in every component
+  mutable sipg::DevBuf slip_x;  // x of an in-place apply, for the slip kernel that follows it
   int pin_elem = -1, pin_node = -1;
   double pin_scale = 1.0;
   int eb64 = 0, eb32 = 0;
@@ -132,7 +134,7 @@ struct sipg_op {
   template <typename T>
   sipg::ApplyArgs<T> apply_args(const T* x, T* y) const;
   void refresh_tau(cudaStream_t s);
-  void refresh_bc();  // neighbour records after bct changed (synchronous)
+  void refresh_bc();  // neighbour records and slip faces after bct / bct_host changed (synchronous)
   sipg::BlockArgs block_args(int mode, int ref_volume, double* out, bool with_pin) const;
   void apply_bc_device(const double* bc, double* rhs, cudaStream_t s) const;
   void refresh_pin(cudaStream_t s);

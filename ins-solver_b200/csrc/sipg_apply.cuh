@@ -79,7 +79,7 @@ __device__ __forceinline__ void simplex_face_normal(const double* g, int f, doub
 enum : int { BC_DIRICHLET = 0, BC_NEUMANN = 1, BC_SLIP = 2 };
 
 // Codes of boundary faces in ApplyArgs::nrec, after the orientations (6 in 3D, 2 in 2D);
-// natural: Neumann, and slip faces, whose terms launch_slip adds
+// natural: Neumann, and slip faces, whose terms are formed apart (ApplyArgs::slip or launch_slip)
 enum : int { NREC_NATURAL = 6, NREC_DIRICHLET = 7 };
 
 // mm modes
@@ -113,7 +113,7 @@ struct ApplyArgs {
                           // a boundary face's own record with NREC_DIRICHLET or NREC_NATURAL
   const T* fgeo;          // tensor-core path: face coefficients K x NF x 4 (launch_face_geo)
   int nvec = 1;           // tensor-core path: components applied by one launch (x, y, c K x NP apart, nrec K x NF)
-  const uint8_t* slip = nullptr;  // nvec > 1: per element, bit f set where face f is a slip face
+  const uint8_t* slip = nullptr;  // nvec > 1, FP64: per element, bit f set where face f is a slip face
   // tensor-core path, FP64, inside a conjugate-gradient iteration (pz not null): x <- pz +
   // (scal[bnum] / scal[bden]) x is formed and stored in place first, and x . y is left as one
   // partial sum per CTA (their number in *dot_count, on the host) or, with dot_out, summed

@@ -368,9 +368,10 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_volume_kernel(ApplyArgs
 }
 
 // ---------------------------------------------------------------- pass 2
-// Slip face of the vector operator, folded in here (2 instead of 7 launches per apply; at
-// p = 3, 16^3 x 6 in FP64 163 -> 58 us per apply with the components batched, where a kernel
-// over the boundary elements alone took 45 us): as vmf_3d_mult_avg_jump.h:9-41, the exterior state mirrors the
+// Slip face of the vector operator, folded in here in FP64 (2 instead of 7 launches per apply; at
+// p = 3, 16^3 x 6 163 -> 58 us per apply with the components batched, where a kernel over the
+// boundary elements alone took 45 us; FP32 keeps that kernel, sipg_slip_kernel, since the MMAs here
+// would round its FP32 terms to TF32): as vmf_3d_mult_avg_jump.h:9-41, the exterior state mirrors the
 // interior one, u+ = u - 2 n (n . u) and likewise the fluxes q, so that the jump and the average
 // carry the normal components 2 n_c (n . u) and n_c (n . q) alone. `at`: the node pair's place in
 // the element's records; um: component comp's own (u, q) pairs.
@@ -511,9 +512,11 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) sipg_face_kernel(ApplyArgs<T
         }
         // exterior values: the neighbour's; a boundary face has its own, negated on Dirichlet faces
         const T sgn = sg == NREC_DIRICHLET ? T(-1) : T(1);
-        if (VEC && sg == NREC_NATURAL && !pad) {
-          const int e = min(e0 + g + 8 * ri, a.K - 1);
-          if (a.slip[e] >> f & 1) slip_exterior<T, DIM, P>(a, trace, e, f, 16 * fb + 4 * t, comp, um, p0, p1);
+        if constexpr (VEC && std::is_same<T, double>::value) {
+          if (sg == NREC_NATURAL && !pad) {
+            const int e = min(e0 + g + 8 * ri, a.K - 1);
+            if (a.slip[e] >> f & 1) slip_exterior<T, DIM, P>(a, trace, e, f, 16 * fb + 4 * t, comp, um, p0, p1);
+          }
         }
         const T s0 = um[0] - sgn * p0.x, s1 = um[2] - sgn * p1.x;
         fu[ri][0] = fg[0] * s0 - (um[1] - sgn * p0.y);
