@@ -30,6 +30,7 @@
 
 namespace sipg {
 void solver_set_cancel(sipg_solver* s, const std::atomic<int>* flag);
+size_t solver_state_bytes(const sipg_op* op, int kind, const sipg_solver_opts& o);
 }
 
 using Clock = std::chrono::steady_clock;
@@ -39,28 +40,6 @@ namespace {
 
 double ms_between(Clock::time_point a, Clock::time_point b) {
   return std::chrono::duration<double, std::milli>(b - a).count();
-}
-
-// Device bytes of a solver's state (work vectors, multigrid levels, assembled
-// blocks, algebraic coarse levels), estimated from the operator's sizes.
-size_t estimate_bytes(const sipg_op* op, int kind, const sipg_solver_opts& o) {
-  const size_t K = op->mesh->K, nc = op->ncomp, NF = op->mesh->dim + 1;
-  const size_t n = nc * K * op->Np;
-  size_t b = 10 * n * sizeof(double);  // Krylov vectors, host-transfer buffers
-  if (kind == SIPG_SOLVER_BLOCK_JACOBI) b += n * op->Np * sizeof(double);
-  if (kind == SIPG_SOLVER_PMULTIGRID) {
-    const size_t ts = o.precision == SIPG_FP32 ? 4 : 8;
-    for (int l = 0; l < o.n_levels && l < 4; ++l) {
-      const int p = l == 0 ? op->order : o.orders[l];
-      const size_t np = (size_t)(op->mesh->dim == 3 ? (p + 1) * (p + 2) * (p + 3) / 6 : (p + 1) * (p + 2) / 2);
-      const size_t nl = nc * K * np;
-      b += nl * (12 + 7 * ts);                              // inverse diagonals, level vectors
-      if (l > 0) b += K * np * 24 + K * NF * 2 * (np + 2) * 12;  // level operator, traces
-      if (l > 0 && p == 1) b += (NF + 1) * np * np * K * 12;  // assembled blocks
-    }
-    b += op->mesh->Nv * 400;  // algebraic coarse levels
-  }
-  return b + (1u << 20);
 }
 
 struct Request {
@@ -111,7 +90,7 @@ struct sipg_server {
   Resident* reserve(const Request& r) {
     for (auto& s : resident)
       if (s->matches(r)) return s->busy ? nullptr : s.get();
-    const size_t need = estimate_bytes(r.op, r.kind, r.opts);
+    const size_t need = solver_state_bytes(r.op, r.kind, r.opts);
     while (resident_bytes + need > o.hbm_budget_bytes) {
       Resident* lru = nullptr;
       for (auto& s : resident)
@@ -227,7 +206,7 @@ int sipg_server_submit(sipg_server* s, sipg_op* op, int kind, const sipg_solver_
     const size_t n = (size_t)op->ncomp * op->mesh->K * op->Np;
     r->b.assign(b, b + n);
     r->x = x;
-    if (estimate_bytes(op, kind, r->opts) > s->o.hbm_budget_bytes)
+    if (solver_state_bytes(op, kind, r->opts) > s->o.hbm_budget_bytes)
       throw Error(SIPG_OUT_OF_MEMORY, "request rejected: its solver state exceeds the HBM budget");
     r->t_submit = Clock::now();
     std::lock_guard<std::mutex> lk(s->mu);

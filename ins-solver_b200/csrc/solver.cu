@@ -228,9 +228,9 @@ struct sipg_solver {
   std::vector<Level> lv;
   std::vector<AmgDevLevel> al;
   DevCsr Pdg, Rdg;
-  DevBuf cinv64, cinv32, cinv_work;
+  DevBuf cinv64, cinv32;
   int cinv_n = 0;
-  DevBuf rows_ws;  // set-up workspace: FP64 inverse diagonal blocks of a level
+  DevBuf rows_ws;  // set-up workspace: FP64 inverse diagonal blocks of a level, then the coarsest inversion's
   DevBuf pl_v, pl_w, pl_t;  // set-up workspace: power iteration
   DevBuf p1_blk, a0_tmp;     // set-up workspace: P1 element blocks, level-0 values before the hierarchy exists
   // the algebraic hierarchy (aggregates and prolongators) is kept across set-ups
@@ -698,7 +698,6 @@ void sipg_solver::setup_amg() {
     const size_t nn = (size_t)cinv_n * cinv_n;
     ensure(cinv64, nn * sizeof(double));
     ensure(cinv32, nn * sizeof(float));
-    ensure(cinv_work, dense_inverse_work(cinv_n) * sizeof(double));
     amg_bct = op->bct_host;
     amg_singular = singular;
     amg_frozen = true;
@@ -720,7 +719,9 @@ void sipg_solver::setup_amg() {
   const size_t nn = (size_t)cinv_n * cinv_n;
   csr_to_dense_device(cinv_n, C.A.ptr.as<int>(), C.A.idx.as<int>(), C.A.v64.as<double>(), cinv64.as<double>(),
                       singular, stream);
-  dense_inverse_device(cinv64.as<double>(), cinv_n, singular, cinv_work.as<double>(), stream);
+  const size_t work = dense_inverse_work(cinv_n) * sizeof(double);
+  if (rows_ws.bytes < work) rows_ws = DevBuf(work);  // the levels' blocks in it have been packed
+  dense_inverse_device(cinv64.as<double>(), cinv_n, singular, rows_ws.as<double>(), stream);
   to_f32(cinv32.as<float>(), cinv64.as<double>(), nn, stream);
   pt.mark("coarsest inverse (device)");
 }
@@ -1301,6 +1302,91 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
 }
 
 namespace sipg {
+// Upper estimate of the device memory a solver of op holds once it has run: the buffers of
+// setup_body, setup_pmg, setup_amg and solve, each rounded up as cudaMalloc does, with the
+// operators of the levels and the traces of every operator applied. The algebraic levels are
+// bounded by what a vertex of a tetrahedral mesh takes (15 matrix entries, prolongators of up to
+// eight, their product lists: 3 KB) and by the largest coarsest level the options allow.
+size_t solver_state_bytes(const sipg_op* op, int kind, const sipg_solver_opts& o) {
+  const sipg_mesh* m = op->mesh;
+  const int dim = m->dim;
+  const size_t K = m->K, nc = op->ncomp, NF = dim + 1, f8 = sizeof(double), f4 = sizeof(float), f2 = sizeof(__half);
+  const size_t n = nc * K * op->Np, page = 2u << 20;
+  size_t b = 4 * page;  // the small buffers
+  auto add = [&](size_t bytes, int count = 1) { b += count * (bytes < page / 2 ? bytes : (bytes + page - 1) / page * page); };
+  auto traces = [&](int p) { return nc * tc_trace_values(dim, p, m->K); };
+  add(n * f8, 7);  // Krylov vectors, host-transfer buffers
+  if (!op->oi) add(traces(op->order) * f8);
+  if (kind == SIPG_SOLVER_JACOBI) add(n * f8);
+  if (kind == SIPG_SOLVER_BLOCK_JACOBI) add(n * op->Np * f8);
+  if (kind != SIPG_SOLVER_PMULTIGRID) return b;
+  const bool f32 = o.precision == SIPG_FP32;
+  const size_t ts = f32 ? f4 : f8;
+  const int nl = std::min(std::max(o.n_levels, 1), 4);
+  const int amo = o.assembled_max_order >= 0 ? o.assembled_max_order : (f32 ? 2 : 1);
+  size_t rows = 0, power = 0;  // workspaces the levels share
+  if (f32) add(n * f4, 2);
+  for (int l = 0; l < nl; ++l) {
+    const int p = l == 0 ? op->order : o.orders[l];
+    if (p < 1 || p > kMaxOrder) break;  // refused by the set-up
+    const size_t np = np_of(dim, p), nb = nc * K, ln = nb * np;
+    const bool own = l > 0 || op->oi, bsr = l > 0 && p <= amo && bsr_supported(dim, p, op->ncomp);
+    add(ln * f8);  // inverse diagonal
+    if (f32) add(ln * f4);
+    add(ln * ts, l == nl - 1 ? 7 : 4);
+    if (own) {
+      add(K * NF * f8);  // tau
+      add(K * NF * f4);
+      add(K * NF * 4 * f8);  // face coefficients
+      add(K * NF * 4 * f4);
+      add(nb * NF * sizeof(uint32_t));  // neighbour records
+      if (op->has_factor || op->oi) {
+        add(K * np * f8, l > 0 ? 2 : 1);
+        add(K * np * f4);
+      }
+      if (op->mm_mode == SIPG_MM_NODAL) {
+        add(K * np * f8, 2);
+        add(K * np * f4);
+      }
+    }
+    if (f32 && !bsr) add(traces(p) * f4);
+    if (own && !(f32 && o.smoother == 1)) add(traces(p) * f8);  // FP64 cycle or eigenvalue bound
+    if (o.smoother == 1) {
+      const bool sym = block_sym_supported((int)np) && nb >= (size_t)kSymMinBlocks;
+      if (f32) add((sym ? block_sym_values<__nv_bfloat16>((int)nb, (int)np) : ln * np) * sizeof(__nv_bfloat16));
+      else add((sym ? block_sym_values<double>((int)nb, (int)np) : ln * np) * f8);
+      rows = std::max(rows, ln * np * f8);
+    }
+    if (bsr) {
+      const size_t nv = (NF + 1) * np * np * K;
+      add(nv * f8);
+      if (f32 && np % 2 == 0) {
+        add(nv * f2);
+        if (o.smoother == 1) {
+          add(nv * f8);
+          add(nv * f2);
+          add(ln * f4, 2);
+        }
+      } else if (f32) {
+        add(nv * f4);
+      }
+    }
+    if (std::max(o.pre_it[l], o.post_it[l]) > 0) power = std::max(power, ln * f8);
+  }
+  add(power, 3);
+  if (o.coarse_kind == 1 && nc == 1) {
+    const size_t cn = std::min<size_t>(std::max(2, o.amg_coarse_max), m->Nv);
+    rows = std::max(rows, dense_inverse_work((int)cn) * f8);
+    add(cn * cn * f8);
+    add(cn * cn * f4);
+    add(K * NF * NF * f8);  // P1 element blocks, their gather, injection into the p = 1 nodes
+    add(K * NF * NF * sizeof(int));
+    add(K * NF * 8 * (f8 + f4 + sizeof(int)), 2);
+    add((size_t)m->Nv * 3000);
+  }
+  add(rows);
+  return b;
+}
 void solver_set_cancel(sipg_solver* s, const std::atomic<int>* flag) { s->cancel = flag; }
 cudaStream_t solver_stream(sipg_solver* s) { return s->stream; }
 }  // namespace sipg

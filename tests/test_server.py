@@ -93,3 +93,64 @@ def test_cancel_and_budget_rejection():
         tiny.submit(op, kind, o, b)
     assert e.value.status == sipg.SIPG_OUT_OF_MEMORY
     tiny.close()
+
+
+def _memory_cases():
+    """name -> (operator, kind, options) on a mesh of n^dim cells; every kind of state."""
+    def case(dim, n, order, ncomp=1, kind=sipg.SOLVER_PMULTIGRID, types=sipg.BC_NEUMANN, **opts):
+        def make(n):
+            mesh = sipg.Mesh.box(dim, n, jitter=0.1, seed=3)
+            op = sipg.Operator(mesh, order, ncomp)
+            op.set_bc_types(np.full((ncomp, mesh.Kb), types, np.int32))
+            op.set_factor(np.ones((mesh.K, op.Np)))
+            o = sipg.default_opts(kind)
+            o.rel_tol, o.abs_tol, o.max_iter, o.nullspace = 1e-6, 0.0, 20, int(types == sipg.BC_NEUMANN)
+            orders = list(range(order, 0, -1))[:3]
+            o.n_levels = len(orders)
+            for l, p in enumerate(orders):
+                o.orders[l] = p
+            for k, v in opts.items():
+                setattr(o, k, v)
+            return op, kind, o
+        return make, n
+    return {
+        "mixed_p3": case(3, 16, 3, precision=sipg.FP32),
+        "fp64_p3": case(3, 14, 3),
+        "mixed_p4": case(3, 10, 4, precision=sipg.FP32),
+        "mixed_p2_small_coarse": case(3, 12, 2, precision=sipg.FP32, amg_coarse_max=100),
+        "fp64_2d": case(2, 60, 3),
+        "point_smoother": case(3, 12, 3, precision=sipg.FP32, smoother=0),
+        "coarse_cg": case(3, 12, 3, precision=sipg.FP32, coarse_kind=0),
+        "jacobi_vector": case(3, 12, 3, ncomp=3, kind=sipg.SOLVER_JACOBI, types=sipg.BC_DIRICHLET),
+        "block_jacobi": case(3, 12, 3, kind=sipg.SOLVER_BLOCK_JACOBI, types=sipg.BC_DIRICHLET),
+    }
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(_memory_cases()))
+def test_resident_bytes_cover_what_a_solver_allocates(name):
+    """The server admits solvers by an estimate of their device memory: it covers what the first
+    request takes from the device and stays within 1.6 times that and 80 MiB (the coarsest inverse
+    of the largest size the options allow, 2,048^2 values in FP64, FP32 and workspace: where
+    aggregation ends is not known beforehand)."""
+    import torch
+    make, n = _memory_cases()[name]
+    srv = sipg.Server(slots=1)
+
+    def request(op, kind, o):
+        b = np.random.default_rng(1).uniform(-1, 1, op.shape())
+        b -= b.mean()
+        x, res = srv.wait(srv.submit(op, kind, o, b))
+        assert res.status in (sipg.SIPG_OK, sipg.SIPG_NOT_CONVERGED), res.error
+
+    warm = make(2)
+    request(*warm)  # kernels and per-order tables
+    base = srv.stats()["resident_bytes"]
+    op, kind, o = make(n)
+    free0 = torch.cuda.mem_get_info()[0]
+    request(op, kind, o)
+    used = free0 - torch.cuda.mem_get_info()[0]
+    estimate = srv.stats()["resident_bytes"] - base
+    srv.close()
+    print(f"{name}: used {used / 2**20:.1f} MiB, estimate {estimate / 2**20:.1f} MiB")
+    assert used <= estimate <= 1.6 * used + (80 << 20)
