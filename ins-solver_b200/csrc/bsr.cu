@@ -215,12 +215,16 @@ __global__ void k_d2f(float* dst, const double* src, size_t n) {
 }
 
 // One thread per (RB consecutive rows, element e), e fastest: block reads are coalesced; a thread
-// gathers its element's and neighbours' x once for its RB rows. With small blocks (Np <= 6) one
-// row per thread keeps enough threads to hide the gather latency; with larger ones the gathers,
-// scattered 8-byte loads that every row repeated, bound the kernel (L1 91 % busy).
-// FP64 p = 3, 24^3 x 6 tets: 343 us with one row per thread, 238 / 210 / 225 / 234 with 2 / 4 / 5 /
-// 10 (16,320 B per element: 97 % of the HBM rate); 8^3 x 6: 22.7, 15.6 / 18.9 / 25.0 / 59.8; p = 4,
-// 16^3 x 6: 279 -> 194 with 5; p = 2, 24^3 x 6: 70.7 -> 57.5 with 2; in 2D one row is best.
+// gathers its element's and neighbours' x once for its RB rows. With one row per thread those
+// gathers, scattered 8-byte loads that every row repeats, bound the kernel on large meshes (L1
+// 91 % busy); on small ones several rows per thread are a longer chain of loads with too few
+// threads to hide it. FP64 p = 3, 24^3 x 6 tets: 343 us with one row per thread, 238 / 210 / 225 /
+// 234 with 2 / 4 / 5 / 10 (16,320 B per element: 97 % of the HBM rate). One row against RB in a
+// CUDA graph (us, FP64 and FP32, K elements): Np = 10, RB = 2: K = 3,072 6.3 / 8.0 and 4.4 / 4.9,
+// 4,374 8.5 / 8.4 and 5.8 / 5.2, 82,944 70.5 / 57.4 and 38.8 / 33.9; Np = 20, RB = 2: 1,296
+// 11.5 / 13.9 and 7.9 / 8.1, 2,058 19.8 / 14.9 and 12.7 / 8.9; Np = 35, RB = 5: 48 13.1 / 38.9 and
+// 8.9 / 30.3, 13,182 163 / 182 and 111 / 151, 16,464 191 / 162 and 134 / 174, 24,576 276 / 196 and
+// 201 / 174. bsr_apply's lines lie between these; smaller blocks and 2D take one row.
 // V4: x rows read as one 16-byte load (FP32, Np = 4, x 16-byte aligned).
 template <typename T, int NP, int NF, int RB = 1, bool V4 = false>
 __global__ void __launch_bounds__(256) k_bsr(int K, const T* __restrict__ v, const int* __restrict__ nbr,
@@ -520,17 +524,21 @@ void bsr_apply(const BsrOp& B, const T* x, T* y, T alpha, T beta, cudaStream_t s
     const int g = (int)std::max<size_t>(1, std::min<size_t>(((size_t)B.K * (B.Np / rb) + 255) / 256, 148 * 32));
     pdl_launch(kern, dim3(g), dim3(256), 0, s, B.K, v, B.nbr, x, y, alpha, beta, c);
   };
+  // threads per SM with rb rows per thread
+  auto per_sm = [&](int rb) { return (long long)B.K * (B.Np / rb) / num_sms(); };
   const bool v4 = std::is_same<T, float>::value && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
   if (B.dim == 3 && B.Np == 4 && v4) run(k_bsr<T, 4, 4, 1, true>, 1);
   else if (B.dim == 3 && B.Np == 4) run(k_bsr<T, 4, 4>, 1);
-  else if (B.dim == 3 && B.Np == 10) run(k_bsr<T, 10, 4, 2>, 2);
+  else if (B.dim == 3 && B.Np == 10 && per_sm(2) >= 128) run(k_bsr<T, 10, 4, 2>, 2);
+  else if (B.dim == 3 && B.Np == 10) run(k_bsr<T, 10, 4>, 1);
   else if (B.dim == 2 && B.Np == 3) run(k_bsr<T, 3, 3>, 1);
   else if (B.dim == 2 && B.Np == 6) run(k_bsr<T, 6, 3>, 1);
   // orders 3 and 4 (the over-integrated operator's blocks)
-  // four rows per thread while that leaves 1024 threads per SM
-  else if (B.dim == 3 && B.Np == 20 && (long long)B.K * 5 >= num_sms() * 1024LL) run(k_bsr<T, 20, 4, 4>, 4);
-  else if (B.dim == 3 && B.Np == 20) run(k_bsr<T, 20, 4, 2>, 2);
-  else if (B.dim == 3 && B.Np == 35) run(k_bsr<T, 35, 4, 5>, 5);
+  else if (B.dim == 3 && B.Np == 20 && per_sm(4) >= 1024) run(k_bsr<T, 20, 4, 4>, 4);
+  else if (B.dim == 3 && B.Np == 20 && per_sm(2) >= 128) run(k_bsr<T, 20, 4, 2>, 2);
+  else if (B.dim == 3 && B.Np == 20) run(k_bsr<T, 20, 4>, 1);
+  else if (B.dim == 3 && B.Np == 35 && per_sm(5) >= (sizeof(T) == 8 ? 768 : 1024)) run(k_bsr<T, 35, 4, 5>, 5);
+  else if (B.dim == 3 && B.Np == 35) run(k_bsr<T, 35, 4>, 1);
   else if (B.dim == 2 && B.Np == 10) run(k_bsr<T, 10, 3>, 1);
   else if (B.dim == 2 && B.Np == 15) run(k_bsr<T, 15, 3>, 1);
   else throw Error(SIPG_INVALID_ARG, "no assembled apply for this element");

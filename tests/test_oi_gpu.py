@@ -13,7 +13,7 @@ import oracle_py as O
 import pmg_oracle as P
 import sipg
 import workloads as W
-from helpers import rel_err
+from helpers import DevArray, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -87,6 +87,25 @@ def test_rows_per_thread_of_the_block_apply_follow_the_mesh(n):
     oi.set_factor_oi(np.ones((gm.K, nq)), np.ones((gm.K, 4, nqs)))
     x = np.random.default_rng(n).uniform(-1.0, 1.0, (1, gm.K, oi.Np))
     assert rel_err(oi.apply_host(x), nodal.apply_host(x)) < 1e-12
+
+
+@pytest.mark.parametrize("p,n", [(2, 8), (2, 9), (3, 6), (3, 7), (4, 13), (4, 14), (4, 15), (4, 16)])
+def test_rows_per_thread_of_the_block_apply_on_both_sides_of_each_line(p, n):
+    """3D: one row per thread below, two (p = 2, 3) and five (p = 4) from 3,789, 1,895 and 16,238
+    (FP64) or 21,651 (FP32) elements on; 6 n^3 elements here. FP32 blocks round the FP64 ones once
+    and sum up to 175 products: 176 * 2^-24 = 1.1e-5 of the products' size."""
+    gm = sipg.Mesh.box(3, n, jitter=0.1, seed=3)
+    oi, nodal = sipg.Operator(gm, p, 1), sipg.Operator(gm, p, 1)
+    for o in (oi, nodal):
+        o.set_bc_types(bct_of(gm.Kb, 2))
+    nq, nqs = oi.oi_sizes()
+    oi.set_factor_oi(np.ones((gm.K, nq)), np.ones((gm.K, 4, nqs)))
+    x = np.random.default_rng(n).uniform(-1.0, 1.0, (1, gm.K, oi.Np))
+    want = nodal.apply_host(x)
+    assert rel_err(oi.apply_host(x), want) < 1e-12
+    xd, yd = DevArray(x.astype(np.float32)), DevArray(np.full(x.shape, 7.0, np.float32))
+    oi.apply_device(sipg.FP32, xd.p, yd.p)
+    assert rel_err(yd.get().astype(np.float64), want) < 1.1e-5
 
 
 def test_operator_is_symmetric_and_pinning_replaces_the_row_and_column():
