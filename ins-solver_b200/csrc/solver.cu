@@ -249,8 +249,9 @@ struct sipg_solver {
   unsigned gver = 0;
   bool graph_broken = false;
   const std::atomic<int>* cancel = nullptr;  // set by a serving loop: non-zero ends the solve
-  // device-resident loop (conditional while-node around one iteration on fixed buffers)
-  cudaGraphExec_t gloop = nullptr;
+  // device-resident loop (conditional while-node around one iteration on fixed buffers), and
+  // the one around several that long Jacobi solves go on with
+  cudaGraphExec_t gloop = nullptr, gloop_long = nullptr;
   unsigned long long gloop_nodes = 0;
   bool gloop_broken = false;
   bool warm = false;  // a solve has run since the last set-up: its kernels are loaded
@@ -263,13 +264,14 @@ struct sipg_solver {
         cudaGraphExecDestroy(g);
         g = nullptr;
       }
-    if (gloop) {
-      cudaGraphExecDestroy(gloop);
-      gloop = nullptr;
-    }
+    for (auto* g : {&gloop, &gloop_long})
+      if (*g) {
+        cudaGraphExecDestroy(*g);
+        *g = nullptr;
+      }
   }
   template <typename F>
-  void capture_loop(F&& body, int group);  // body(while-node handle)
+  bool capture_loop(F&& body, int group, cudaGraphExec_t& exec);  // body(while-node handle)
   ~sipg_solver() {
     drop_graphs();
     if (ev0) cudaEventDestroy(ev0);
@@ -1057,10 +1059,11 @@ void sipg_solver::capture_iteration(int par, F&& body) {
   gnodes[par] = nodes;
 }
 
-// Build gloop: a conditional while-node whose body is `group` iterations, each followed by
-// the stopping test. On any failure the solver falls back to per-iteration graphs.
+// Build gloop or gloop_long: a conditional while-node whose body is `group` iterations, each
+// followed by the stopping test. False (and exec null) on any failure: the solver then goes on
+// with gloop, or without it with per-iteration graphs.
 template <typename F>
-void sipg_solver::capture_loop(F&& body, int group) {
+bool sipg_solver::capture_loop(F&& body, int group, cudaGraphExec_t& exec) {
   std::lock_guard<std::recursive_mutex> capture_lock(g_graph_mu);
   unsigned long long nodes = 0;
   cudaGraph_t g = nullptr;
@@ -1091,16 +1094,16 @@ void sipg_solver::capture_loop(F&& body, int group) {
     cudaGraph_t out = nullptr;
     ok = cudaStreamEndCapture(stream, &out) == cudaSuccess && body_ok;
   }
-  if (ok) ok = cudaGraphInstantiate(&gloop, g, 0) == cudaSuccess;
+  if (ok) ok = cudaGraphInstantiate(&exec, g, 0) == cudaSuccess;
   if (g) cudaGraphDestroy(g);
   if (!ok) {
-    if (gloop) cudaGraphExecDestroy(gloop);
-    gloop = nullptr;
+    if (exec) cudaGraphExecDestroy(exec);
+    exec = nullptr;
     cudaGetLastError();
-    gloop_broken = true;
-    return;
+    return false;
   }
   gloop_nodes = nodes / group;
+  return true;
 }
 
 int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
@@ -1181,14 +1184,19 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
     k_loop_start<<<1, 1, 0, stream>>>(S());
     note_launch();
     const bool jac = !o.nullspace && (kind == SIPG_SOLVER_JACOBI || kind == SIPG_SOLVER_BLOCK_JACOBI);
-    // Iterations per pass of the while-node: a pass costs about 10 us besides its kernels, as
-    // much as a whole Jacobi iteration of a small mesh (three launches). Those kernels do
-    // nothing once the stopping test has ended the loop, so eight share a pass. 2D block-Jacobi
-    // solve of 8,192 triangles, p = 3: 62.1 -> 47.9 ms with eight,
-    // before the kernels themselves got shorter. A plain graph of 8, 16 or 32 iterations,
-    // launched again until the loop has ended, takes what the while-node takes (16.9, 16.5 and
-    // 16.5 against 16.8 us per iteration).
-    const int group = jac && ride ? 8 : 1;
+    // Iterations per pass of the while-node. A pass costs 3.4 us besides its kernels, a third of a
+    // Jacobi iteration of a small mesh (three launches): 13.5 us per iteration of 512 triangles,
+    // p = 3, with one iteration per pass, 10.6 with eight; 8,192 triangles 17.1 and 13.7; 196,608
+    // tets 203 and 199. The kernels do nothing once the stopping test has ended the loop, so
+    // several can share a pass, but the empty iterations at the end (5 to 16 us each) and the
+    // capture (about 20 us per iteration in it) are what a short solve pays: of 2 iterations on 512
+    // triangles, set-up included, 420 us with one per pass, 550 to 590 with eight. Four keep most of
+    // the gain; eight, a second capture (0.2 to 0.3 ms), only where a solve has gone on for long. A
+    // plain graph of 8, 16 or 32 iterations, launched again until the loop has ended, takes what the
+    // while-node takes.
+    const int group = jac && ride ? 4 : 1;
+    int long_group = jac && ride ? 8 : 0;
+    constexpr int kLongSolve = 512;
     // loop: the while-node the iteration is captured into (0: none)
     auto body = [&](cudaGraphConditionalHandle loop) {
       int npap = 0;  // Jacobi: the update sums p . Ap's partials itself (kept apart from its own)
@@ -1245,18 +1253,21 @@ int sipg_solver::solve(const double* b, double* x_user, sipg_solve_info* info) {
     };
     // graphs = 2: the iterations after the first run inside gloop, whose while-node
     // repeats the body until k_loop_check ends it; the host reads the scalars once
-    // per launch of at most kLoopChunk iterations. graphs = 1: one graph launch per
+    // per launch of at most kLoopChunk iterations (Jacobi: gloop_long from kLongSolve
+    // iterations on). graphs = 1: one graph launch per
     // iteration. The first iteration runs eagerly (lazy buffers are allocated there).
     constexpr int kLoopChunk = 64;
     while (status == SIPG_OK && res > tol && iter < o.max_iter) {
-      if (graphs && iter >= 1 && o.graphs >= 2 && !gloop && !gloop_broken) capture_loop(body, group);
+      if (graphs && iter >= 1 && o.graphs >= 2 && !gloop && !gloop_broken) gloop_broken = !capture_loop(body, group, gloop);
+      const bool longer = gloop && long_group > 0 && iter >= kLongSolve;
+      if (longer && !gloop_long && !capture_loop(body, long_group, gloop_long)) long_group = 0;
       if (graphs && iter >= 1 && gloop) {
         hw.h[S_ITER] = (double)iter;
         hw.h[S_STATUS] = 0.0;
         hw.h[S_TOL] = tol;
         hw.h[S_CHUNK] = (double)kLoopChunk;
         SIPG_CUDA(cudaMemcpyAsync(S() + S_ITER, hw.h + S_ITER, 4 * sizeof(double), cudaMemcpyHostToDevice, stream));
-        SIPG_CUDA(cudaGraphLaunch(gloop, stream));
+        SIPG_CUDA(cudaGraphLaunch(longer && gloop_long ? gloop_long : gloop, stream));
         read_scalars();
         const int done = (int)hs.h[S_ITER];
         note_launch((unsigned)((done - iter) * gloop_nodes));

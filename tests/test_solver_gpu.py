@@ -331,3 +331,22 @@ def test_jacobi_loop_ends_within_a_group(kind, max_iter):
     for (xe, ie), (xg, ig) in zip(out[0], out[2]):
         assert ie.iters == ig.iters <= max_iter and ie.status == ig.status
         assert np.array_equal(xe, xg)
+
+
+@pytest.mark.parametrize("max_iter", [67, 68, 69, 511, 513, 517, 520, 521, 577, 585, 640])
+@pytest.mark.parametrize("kind", [sipg.SOLVER_JACOBI, sipg.SOLVER_BLOCK_JACOBI], ids=["jacobi", "block"])
+def test_long_jacobi_solves_end_within_either_group(kind, max_iter):
+    """Four iterations per pass of the loop, eight from 512 on: the iteration limit ends a solve at
+    any place of either with the iterates of kernels launched one by one, also on a second solve
+    that finds both loops captured."""
+    c = W.poisson2d_manufactured(12, order=3)
+    out = {}
+    for graphs in (0, 2):
+        op = make_op(c["mesh"], 3, 1, bct=c["bc_types"])
+        o = sipg.default_opts(kind)
+        o.rel_tol, o.abs_tol, o.max_iter, o.nullspace, o.graphs = 1e-200, 0.0, max_iter, 0, graphs
+        s = sipg.Solver(op, kind, o)
+        out[graphs] = [s.solve_host(c["rhs"]) for _ in range(2)]
+    for (xe, ie), (xg, ig) in zip(out[0], out[2]):
+        assert ie.iters == ig.iters == max_iter and ie.status == ig.status
+        assert np.array_equal(xe, xg)
