@@ -725,7 +725,8 @@ cudaError_t launch_pass(const ApplyArgs<T>& a, const T* blob, TT* trace, int war
   int per_sm = 1;
   cudaError_t err = kernel_setup<K>(warps, bytes, per_sm);
   if (err != cudaSuccess) return err;
-  const int grid = std::min(ntiles, num_sms * per_sm);
+  int grid = std::min(ntiles, num_sms * per_sm);
+  if (ctas) grid = std::min(grid, kRedBlocks);  // a partial sum per CTA, in a buffer of that many
   if (ctas) *ctas = grid;
   if (grid > 0) {
     err = pdl_launch(K, dim3(grid), dim3(warps * 32), bytes, s, a, blob, trace);
@@ -758,10 +759,11 @@ cudaError_t launch_tc_t(const ApplyArgs<T>& a, const T* blob, T* trace, int num_
     // FP32: the tcgen05 kernels (their constants follow the mma.sync blob)
     if (a.tcgen05 && tc5_supported(DIM, P)) return launch_apply_tc5(DIM, P, a, blob + X::NALL, trace, num_sms, s);
   }
-  // the kernels read caller vectors in 16-byte pieces: other alignments take the CUDA-core kernel
+  // the kernels read caller vectors in 16-byte pieces: other alignments take the CUDA-core kernel,
+  // which forms neither a direction step's p nor its dot and applies no batch of components
   if (!aligned16(a.x) || !aligned16(a.y) || !aligned16(trace) || (a.factor && !aligned16(a.factor)) ||
-      (a.beta != T(0) && !aligned16(a.c)))
-    return launch_apply<T>(DIM, P, a, num_sms, s);
+      (a.beta != T(0) && !aligned16(a.c)) || !aligned16(a.pz))
+    return a.pz || a.nvec > 1 ? cudaErrorInvalidValue : launch_apply<T>(DIM, P, a, num_sms, s);
   const int ntiles = (a.K + X::TE - 1) / X::TE * a.nvec;
   constexpr bool two = 2 * (smem1<T, DIM, P>(8) + 1024) <= (size_t)kSmemBudget + 1024;
   constexpr int W = two ? 8 : 12, B = two ? 2 : 1;
