@@ -1,5 +1,5 @@
-"""Edges of the eight-element tiles of the momentum kernels (meshes below one tile, whole tiles,
-a remainder) and device arrays on 8-byte but not 16-byte boundaries, at every order: the device
+"""Edges of the eight-element tiles of the momentum and projection kernels (meshes below one tile,
+whole tiles, a remainder) and device arrays on 8-byte but not 16-byte boundaries, at every order: the device
 entries on shifted arrays against the host entries, which the oracle tests cover."""
 import ctypes as C
 
@@ -58,3 +58,37 @@ def test_pressure_rhs_on_shifted_arrays(dim, n, order, off):
     sipg.check(sipg.lib().sipg_pressure_rhs(mesh.h, order, C.c_double(1e-2), C.c_double(2.0), C.c_double(-1.0), d[0].p,
                                             d[1].p, d[2].p, d[3].p, C.c_void_p(0)))
     assert np.array_equal(d[3].get(), rhs) and np.array_equal(d[2].get(), dold)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("n", [1, 2, 3])
+@pytest.mark.parametrize("kind", ["grad", "pressure", "two_phase"])
+def test_projection_on_shifted_arrays(n, order, kind):
+    """Every array shifted alone, and all together: one misaligned pointer takes the unpaired loads."""
+    dt = 1e-2
+    mesh = sipg.Mesh.box(3, n, jitter=0.1, seed=3)
+    Np = sipg.ref_sizes(3, order)[0]
+    rng = np.random.default_rng(order)
+    v = rng.uniform(-1, 1, (3, mesh.K, Np))
+    if kind == "grad":
+        ins = [rng.uniform(-1, 1, (3, mesh.K, Np)), v]
+        want, st = sipg.project_velocity(mesh, order, dt, *ins)
+    else:
+        ins = [rng.uniform(-1, 1, (mesh.K, Np)), v]
+        rho = rng.uniform(1.0, 1000.0, (mesh.K, Np)) if kind == "two_phase" else None
+        want, st = sipg.pressure_projection(mesh, order, dt, *ins, rho=rho)
+        if rho is not None:
+            ins.insert(1, rho)
+    na = len(ins) + 1
+    for mask in [0] + [1 << i for i in range(na)] + [(1 << na) - 1]:
+        d = [Shifted(x, mask >> i & 1) for i, x in enumerate(ins + [np.zeros_like(v)])]
+        dst = sipg.DeviceVector(np.full(2, 12345, np.uint64))
+        if kind == "grad":
+            sipg.check(sipg.lib().sipg_project_velocity(mesh.h, order, C.c_double(dt), C.c_double(dt), d[0].p, d[1].p,
+                                                        d[2].p, C.c_void_p(dst.ptr), C.c_void_p(0)))
+        else:
+            r = d[1].p if kind == "two_phase" else C.c_void_p(0)
+            sipg.check(sipg.lib().sipg_pressure_projection(mesh.h, order, C.c_double(dt), C.c_double(dt), d[0].p, r,
+                                                           d[-2].p, d[-1].p, C.c_void_p(dst.ptr), C.c_void_p(0)))
+        assert np.array_equal(d[-1].get(), want), mask
+        assert dst.get().tolist() == [int(st[1]), int(st[2])], mask
