@@ -249,8 +249,8 @@ def run_viscous(steps=3):
     on the x and z walls and no-slip on the y walls, right-hand side from the
     fused viscous right-hand side kernel (mp_ins_3d_vis_0 + mass) of seeded
     U(-1, 1) velocities, ViscousSolver3D's Jacobi-preconditioned CG to 1e-8
-    relative. FP64 applies on the tensor cores (three scalar applies and the slip
-    coupling terms) and on the CUDA cores, and the solve."""
+    relative. FP64 applies on the tensor cores (all components and their slip faces
+    in one pair of launches) and on the CUDA cores, and the solve."""
     import torch
     n, order, dt, Re, g0 = PROJ_N, 3, 1e-3, 100.0, 1.5
     mesh = sipg.Mesh.box(3, n, jitter=0.1, seed=20261203)
@@ -1081,7 +1081,7 @@ def run_profile(args):
     """Small fixed workloads for ncu captures (no timing is reported from them).
 
     apply: the headline operator at --n (order --order, precision --precision),
-           3 applies after set-up; with -k regex:"sipg_(trace|apply_tc)" -s 2 -c 2
+           3 applies after set-up; with -k regex:"sipg_(volume|face)" -s 2 -c 2
            ncu captures the second apply's two kernels.
     projection: the velocity projection workload at --n (3 launches of k_proj_tc).
     pressure: the pressure step kernels at --n: sipg_pressure_rhs and

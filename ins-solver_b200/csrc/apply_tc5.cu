@@ -67,7 +67,8 @@ struct T5 {
   static constexpr int OFF_F = rup5(3 * NP, 8);
   static constexpr int OFF_MM = OFF_F + NF * KFACE;
   static constexpr int K2 = rup5(OFF_MM + NP, 8);
-  // trace records: the mma.sync kernels' layout (u at [0, NFP), g at [TRP, TRP + NFP))
+  // trace records, written and read by these kernels alone: u at [0, NFP), g at [TRP, TRP + NFP), of
+  // the size of the mma.sync kernels' records (which hold (u, q) pairs), whose scratch they use
   static constexpr int TRP = rup5(NFP, 2), TR = rup5(2 * TRP, 4), TRV = TR / 4;
   // constant blob (floats, MMA layout): B1 (N1 x K1), B2 (N2 x K2)
   static constexpr int CB1 = 0, CB2 = N1 * K1, CALL = CB2 + N2 * K2;

@@ -1,8 +1,9 @@
-// Tensor-core SIPG apply (scalar operator): FP32 data on TF32 tensor cores or
-// FP64 data on the FP64 tensor cores, in two passes over the elements.
+// Tensor-core SIPG apply: FP32 data on TF32 tensor cores or FP64 data on the FP64
+// tensor cores, in two passes over the elements; a scalar operator, or a component
+// or all components of an unpinned vector one.
 //
 // Same operator as sipg_apply.cu (FactorViscousMatrix3D::mult,
-// src/solvers/3d/slip_matrix/factor_viscous_matrix.cpp:96-310, one component).
+// src/solvers/3d/slip_matrix/factor_viscous_matrix.cpp:96-310).
 // The reference exchanges face data through 12 face buffers per component
 // (mesh->jump / mesh->avg into K x Nf*Nfp op_dats); here each element publishes
 // one trace record per face and every matrix product is batched over elements.
@@ -41,8 +42,8 @@
 // and fewer instructions than with every input staged. A boundary face is a code in its
 // neighbour record, so pass 2 has no branch between a tile's loads.
 // Measured per apply, with the earlier form (derivatives at the face nodes in pass 1, all
-// inputs staged) and now: FP64 p = 4 Helmholtz at 48^3 x 6 tets 2.24 -> 0.99 ms (30 of the
-// 37 TFLOP/s the FP64 pipe has, counting issued MMAs), FP64 p = 3 two-phase at 24^3 x 6
+// inputs staged) and now: FP64 p = 4 Helmholtz at 48^3 x 6 tets 2.24 -> 0.99 ms (635 MMAs
+// per 8 elements: 27.4 of the 37 TFLOP/s the FP64 pipe has), FP64 p = 3 two-phase at 24^3 x 6
 // 97 -> 65 us, FP32 there 42.8 -> 32.4 us (L1 transactions of the gathers and latency).
 #include <cuda_runtime.h>
 

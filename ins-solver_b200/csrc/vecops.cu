@@ -227,6 +227,9 @@ __global__ void __launch_bounds__(kRedThreads) k_finish_z_dot(double* z, const f
 // an iteration of 8,192 triangles, p = 3, takes 16.8 us instead of 19.7, of 512 triangles 11.4
 // instead of 14.6. BLK: the first NB entries of a block row are loaded with the rows, not after
 // alpha (15.5 and 10.6 us); NB = 10 is a whole row at 2D p = 3 and 3D p = 2 and leaves no spill.
+// Longer rows, read in part after alpha, gain too; per iteration with NB = 1 and 10: 15 values (8,192
+// triangles) 22.2 and 19.3 us, 20 (24,576 tets) 86.4 and 68.4, (196,608) 373 and 371, 35 (24,576)
+// 218 and 177.
 template <bool BLK, int NB = 10>
 __global__ void __launch_bounds__(kRedThreads) k_cg_update_precond(double* x, double* r, const double* p,
                                                                    const double* Ap, double* z, const double* B,
